@@ -94,7 +94,10 @@ typedef struct {
     int32_t graph_mode;       /* 0 = plain launches, 1 = replayed window graph,
                                  2 = one graph with a device-driven while loop (default) */
     int32_t device;           /* CUDA device ordinal */
-    int32_t max_blocks;       /* schedule tuning: blocks per matrix-pass launch, 0 = one resident wave */
+    int32_t max_blocks;       /* schedule tuning: blocks per matrix-pass launch, 0 = one resident wave
+                                 (an LP that one thread-block cluster can hold then runs a whole
+                                 window of attempts in one launch; a value given here keeps the
+                                 launched passes: the same results bit for bit) */
     int32_t batch_group;      /* batched solver: lanes per column (1, 2, 4, 8, 16, 32), 0 = autotune */
     int32_t escalate;         /* adaptive FP32 stall handling.  A solve stalls when its best
                                  relative KKT error has not halved for max(2048, k/2) attempts
@@ -178,7 +181,8 @@ int sps_solve(sps_handle *h, sps_result *res);
 int sps_get_solution(sps_handle *h, double *x, double *y);
 
 /* Benchmark support (no reference counterpart): after a sps_solve, launch
- * `reps` iterations' kernels one by one on the handle's stream and time each
+ * `reps` iterations' kernels (the launched passes, also on an LP whose solve runs
+ * its attempts in one resident launch per window) one by one on the handle's stream and time each
  * launch with CUDA events.  out[0] = mean ms of the row-pass kernel (CSR SpMV
  * fused with the dual update), out[1] = mean ms of the column-pass kernel (CSC
  * SpMV fused with the primal update), out[2] = fraction of step attempts whose

@@ -17,6 +17,7 @@
 
 #include "host_pool.cuh"
 #include "mem_pool.cuh"
+#include "resident.cuh"
 #include "setup.cuh"
 
 namespace sps {
@@ -84,6 +85,8 @@ struct EngineBase {
     } while (0)
 
 constexpr int kSms = 152;
+constexpr int kResEntries64 = 2304;                // FP64: entries per block above which a larger cluster is taken
+constexpr size_t kResSmem = 226 * 1024;     // dynamic shared memory of a resident block (227 KB with its static part)
 
 template <class V>
 struct Engine : EngineBase {
@@ -115,6 +118,8 @@ struct Engine : EngineBase {
     Args<V> args{};
     cudaMemPool_t pool = nullptr;       // device memory (engine_pool; null: the default pool)
     cudaGraphExec_t win_exec = nullptr, loop_exec = nullptr;
+    void* res_tasks = nullptr;              // resident window kernel: its tasks (null: the passes are launched)
+    size_t res_bytes = 0;                   // its dynamic shared memory
     int64_t launches = 0;
     double setup_ms = 0.0;
     std::vector<double> x_sol, y_sol;
@@ -126,6 +131,7 @@ struct Engine : EngineBase {
         if (win_exec) cudaGraphExecDestroy(win_exec);
         if (loop_exec) cudaGraphExecDestroy(loop_exec);
         if (arena) cudaFreeAsync(arena, st);
+        if (res_tasks) cudaFreeAsync(res_tasks, st);
         if (st) cudaStreamSynchronize(st);
         if (h_ctl) cudaFreeHost(h_ctl);
         if (h_abort) cudaFreeHost(h_abort);
@@ -955,6 +961,7 @@ struct Engine : EngineBase {
         a.abort_flag = d_abort;
         a.has_cond = 0;
         a.check_interval = opt.check_interval > 0 ? opt.check_interval : (adaptive ? 64 : 50);
+        if (int rc = choose_resident(rp, cp)) return rc;
         layout_rows = rp.bt;
         layout_cols = cp.bt;
         padded_nnz_rows = rp.total;
@@ -969,8 +976,177 @@ struct Engine : EngineBase {
         return SPS_OK;
     }
 
+    using WindowKernel = void (*)(const Args<V>);
+    WindowKernel resident_kernel(bool multi) const {
+        if (mode == SPS_MODE_ADAPTIVE) return multi ? ad_resident<V, true> : ad_resident<V, false>;
+        return multi ? rf_resident<V, true> : rf_resident<V, false>;
+    }
+    cudaLaunchConfig_t resident_config(cudaLaunchAttribute* at) const {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)args.res.blocks);
+        cfg.blockDim = dim3((unsigned)(32 * (args.res.warps + (mode == SPS_MODE_ADAPTIVE ? 1 : 0))));
+        cfg.dynamicSmemBytes = res_bytes;
+        cfg.stream = st;
+        at->id = cudaLaunchAttributeClusterDimension;
+        at->val.clusterDim.x = (unsigned)args.res.blocks;
+        at->val.clusterDim.y = at->val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = args.res.blocks > 1 ? 1 : 0;
+        return cfg;
+    }
+
+    // The warps' tasks of one orientation (every warp of the launched pass that has
+    // work); false when a schedule has no resident form: SEGMENT rows, a bin
+    // whose warps take more than one step.
+    static bool resident_tasks(const Plan& P, std::vector<ResTask>& out) {
+        for (int i = 0; i < P.bt.nbins; ++i) {
+            const Bin& b = P.bt.bin[i];
+            if (b.mode == BM_SEGMENT) return false;
+            const int stride = b.nblocks * kWarps, per = b.mode == BM_SLAB ? 1 : 2;
+            if ((int64_t)stride * per < b.units) return false;
+            for (int w0 = 0; w0 < stride && w0 < b.units; ++w0) {
+                ResTask t{};
+                t.mode = b.mode;
+                t.kind = b.kind;
+                t.rend = b.end;
+                t.part = b.block_begin * kWarps + w0;
+                t.u[1].steps = -1;
+                for (int h = 0; h < per && w0 + h * stride < b.units; ++h) {
+                    const int u = w0 + h * stride;
+                    ResTask::Unit& q = t.u[h];
+                    if (b.mode == BM_SLICED) {
+                        q.r0 = b.begin + 32 * u;
+                        q.src = b.part0 > 0 ? b.slice0 + u * 32 * b.part0 : P.soff[b.aux + u];
+                        q.steps = b.part0 > 0 ? b.part0 : (P.soff[b.aux + u + 1] - q.src) / 32;
+                        q.cnt = 32 * q.steps;
+                    } else if (b.mode == BM_WARP) {
+                        q.r0 = b.begin + u;
+                        q.src = P.fptr[q.r0];
+                        q.cnt = P.fptr[q.r0 + 1] - q.src;
+                        q.steps = (q.cnt + 31) / 32;
+                    } else {
+                        const int32_t* d = &P.unit[8 * (size_t)(b.aux + u)];   // {offset, length, slice, unit}
+                        q.r0 = b.begin + 32 * d[2];
+                        q.src = d[0] + 32 * kSlabSteps * d[3];
+                        q.steps = std::min(d[1] - kSlabSteps * d[3], kSlabSteps);
+                        q.cnt = 32 * q.steps;
+                        t.slab_c = d[3];
+                        t.slab_n = (d[1] + kSlabSteps - 1) / kSlabSteps;
+                        t.part = P.bt.total_blocks * kWarps + b.slot0 + d[2];
+                    }
+                }
+                out.push_back(t);
+            }
+        }
+        return true;
+    }
+    static int task_entries(const ResTask& t) { return 32 * (std::max(t.u[0].steps, 0) + std::max(t.u[1].steps, 0)); }
+
+    // The tasks dealt to C blocks of `warps` warps, each (with the units of its SLAB
+    // slice) to the block with the fewest entries that has room; false when they
+    // do not fit.
+    static bool deal_tasks(const std::vector<ResTask>& in, int C, int warps, std::vector<ResTask>& out,
+                           std::vector<int>& ent, std::vector<int>& slab) {
+        ResTask none{};
+        none.mode = -1;
+        none.u[0].steps = none.u[1].steps = -1;
+        out.assign((size_t)C * warps, none);
+        std::vector<int> used(C, 0);
+        for (size_t i = 0; i < in.size();) {
+            const size_t cnt = in[i].mode == BM_SLAB ? (size_t)in[i].slab_n : 1;   // a slice's units are consecutive
+            int best = -1;
+            for (int q = 0; q < C; ++q)
+                if (used[q] + (int)cnt <= warps && (best < 0 || ent[q] < ent[best])) best = q;
+            if (best < 0) return false;
+            for (size_t k = 0; k < cnt; ++k, ++i) {
+                ResTask t = in[i];
+                t.ent = ent[best];
+                ent[best] += task_entries(t);
+                if (cnt > 1) t.slab = slab[best]++;
+                out[(size_t)best * warps + used[best]++] = t;
+            }
+        }
+        return true;
+    }
+
+    // Whether the window's attempts run as one resident launch (resident.cuh), and its
+    // shape.  The line is capacity: wherever every warp's task, the matrix and the
+    // vectors fit one cluster the resident launch won (us per attempt, checks
+    // included, launched -> resident: 40 x 100 17.2 -> 5.7 FP32, 22.2 -> 7.9 FP64;
+    // 200 x 500 19.4 -> 6.3, 26.9 -> 9.7; 2000 x 5000 22.3 -> 9.7, 30.2 -> 13.9;
+    // 100 x 200 transportation 15.3 -> 12.5 FP32; reference mode 200 x 500 FP64 19.2
+    // -> 6.8).  The smallest cluster that fits is taken in FP32: more blocks only
+    // add to the barriers (200 x 500: 6.3 us on one block, 7.5-8.5 on 2-16).  In FP64
+    // a block's products pass a pipe of two per cycle, so up to eight blocks share
+    // them while one holds over kResEntries64 entries (37 x 53 transportation: 12.5
+    // us on 4 blocks, 11.0 on 8; 40 x 100, 1.3k entries: 7.9 on 1, 8.8 on 2).  A
+    // caller who gives the passes' blocks (max_blocks) gets the launched passes.
+    int choose_resident(const Plan& rp, const Plan& cp) {
+        args.res = ResShape{};
+        if (opt.max_blocks > 0) return SPS_OK;
+        std::vector<ResTask> rows, cols, dr, dc;
+        if (rp.bt.total_blocks + cp.bt.total_blocks > 160) return SPS_OK;    // over twice what a cluster can hold
+        if (!resident_tasks(rp, rows) || !resident_tasks(cp, cols)) return SPS_OK;
+        const int extra = mode == SPS_MODE_ADAPTIVE ? 1 : 0;       // the deciding warp
+        const int most = res_max_threads<V>() / 32 - extra;
+        for (int C = 1; C <= kResMaxCluster; C *= 2) {
+            ResShape S{};
+            S.blocks = C;
+            const int need = (int)std::max(rows.size(), cols.size());
+            std::vector<int> ent, slab;
+            bool ok = false;
+            for (S.warps = (need + C - 1) / C; S.warps <= most && !ok; ++S.warps) {   // SLAB slices may need a little room
+                ent.assign(C, 0);
+                slab.assign(C, 0);
+                ok = deal_tasks(rows, C, S.warps, dr, ent, slab) && deal_tasks(cols, C, S.warps, dc, ent, slab);
+                if (ok) break;
+            }
+            if (!ok) continue;
+            S.entries = *std::max_element(ent.begin(), ent.end());
+            S.slab_rows = *std::max_element(slab.begin(), slab.end());
+            S.row_warps = rp.bt.total_blocks * kWarps;
+            S.row_parts = S.row_warps + rp.nslots;
+            S.col_parts = cp.bt.total_blocks * kWarps;
+            const size_t bytes = res_smem_bytes<V>(S, n, m);
+            if (bytes > kResSmem) continue;
+            if (sizeof(V) == 8 && C < kResMaxCluster / 2 && S.entries > kResEntries64) continue;
+            WindowKernel k = resident_kernel(C > 1);
+            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem) != cudaSuccess ||
+                (C > 8 && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
+                cudaGetLastError();
+                continue;
+            }
+            res_bytes = bytes;
+            args.res = S;
+            if (C > 1) {
+                cudaLaunchAttribute at[1];
+                const cudaLaunchConfig_t cfg = resident_config(at);
+                int clusters = 0;
+                const bool fits = cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) == cudaSuccess && clusters > 0;
+                cudaGetLastError();
+                if (!fits) {
+                    args.res = ResShape{};
+                    continue;
+                }
+            }
+            ResTask* d = nullptr;
+            const size_t cnt = dr.size();
+            SPS_CK(dalloc(&d, 2 * cnt * sizeof(ResTask)));
+            res_tasks = d;
+            SPS_CK(cudaMemcpyAsync(d, dr.data(), cnt * sizeof(ResTask), cudaMemcpyHostToDevice, st));
+            SPS_CK(cudaMemcpyAsync(d + cnt, dc.data(), cnt * sizeof(ResTask), cudaMemcpyHostToDevice, st));
+            SPS_CK(cudaStreamSynchronize(st));
+            args.res_rows = d;
+            args.res_cols = d + cnt;
+            return SPS_OK;
+        }
+        return SPS_OK;
+    }
+
     // ---------------------------------------------------------------- solve
-    int nodes_per_window() const { return 2 * args.check_interval + (mode == SPS_MODE_ADAPTIVE ? 4 : 3); }
+    int nodes_per_window() const {
+        return (args.res.blocks ? 1 : 2 * args.check_interval) + (mode == SPS_MODE_ADAPTIVE ? 4 : 3);
+    }
 
     // column check in the error form the options ask for (the PDLP form's kernel adds
     // the Lagrangian form's partials of the same points)
@@ -1002,8 +1178,14 @@ struct Engine : EngineBase {
     void launch_window(const Args<V>& a) {
         const int W = a.check_interval;
         const int gr = a.rows.total_blocks, gc = a.cols.total_blocks;
+        if (a.res.blocks) {
+            cudaLaunchAttribute at[1];
+            const cudaLaunchConfig_t cfg = resident_config(at);
+            const cudaError_t e = cudaLaunchKernelEx(&cfg, resident_kernel(a.res.blocks > 1), a);
+            if (e != cudaSuccess && launch_err == cudaSuccess) launch_err = e;
+        }
         if (mode == SPS_MODE_ADAPTIVE) {
-            for (int w = 0; w < W; ++w) {
+            for (int w = 0; w < W && !a.res.blocks; ++w) {
                 if (a.pdl) {
                     launch_pass(ad_row_step<V, true>, gr, a);
                     launch_pass(ad_col_step<V, true>, gc + a.col_tail_blocks, a);
@@ -1017,7 +1199,7 @@ struct Engine : EngineBase {
             launch_col_check(a);
             ad_apply<V><<<a.apply_blocks, kBlock, 0, st>>>(a);
         } else {
-            for (int w = 0; w < W; ++w) {
+            for (int w = 0; w < W && !a.res.blocks; ++w) {
                 rf_col_step<V><<<gc, kBlock, 0, st>>>(a);
                 rf_row_step<V><<<gr, kBlock, 0, st>>>(a);
             }

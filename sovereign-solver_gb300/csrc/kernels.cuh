@@ -25,6 +25,15 @@
 
 namespace sps {
 
+struct ResTask;               // resident.cuh
+struct ResShape {             // shapes of a resident launch (blocks 0: the passes are launched)
+    int32_t blocks, warps;    // cluster size, working warps per block (in adaptive mode one more decides)
+    int32_t entries;          // shared matrix entries per block (the largest block's)
+    int32_t row_parts, col_parts;   // partial sums of a pass (row pass: warps, then SLAB slices)
+    int32_t row_warps;        // ... of which warps of the launched row pass
+    int32_t slab_rows;        // rows of lane partials per block (SLAB slices of several units)
+};
+
 template <class V>
 struct Args {
     int32_t n, m;
@@ -55,6 +64,8 @@ struct Args {
     int32_t pdl;               // launch the step kernels' programmatic-dependent instantiations
     int32_t check_interval;
     int64_t max_windows;
+    ResShape res;
+    const ResTask *res_rows, *res_cols;   // res.warps tasks per block
 };
 
 
@@ -62,6 +73,11 @@ struct Args {
 // check kernels (FP64 accumulators, once per window) get the default budget
 #define SPS_PASS_KERNEL __global__ void __launch_bounds__(kBlock, kPassMinBlocks)
 #define SPS_CHECK_KERNEL __global__ void __launch_bounds__(kBlock)
+
+// a b + c with one rounding, written out where two kernels must round alike (the
+// compiler's own contraction of a * b + c depends on the code around it)
+__device__ __forceinline__ float mad(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double mad(double a, double b, double c) { return __fma_rn(a, b, c); }
 
 // --- precision helpers -------------------------------------------------------
 __device__ __forceinline__ float rn_add(float a, float b) { return __fadd_rn(a, b); }
@@ -104,11 +120,19 @@ struct GatherOne {
 // Adaptive mode
 // ============================================================================
 
-template <class V>
+// What a step's epilogue does with its new vector entry besides storing it (the
+// resident kernels copy it to the shared memory their next pass gathers from).
+struct NoSink {
+    template <class V>
+    __device__ __forceinline__ void operator()(int, V) const {}
+};
+
+template <class V, class Sink = NoSink>
 struct AdRowStepEpi {
     const V *b, *axo, *yo;
     V *axn, *yn;
     V sigma;
+    Sink sink = Sink{};
     V dy2 = V(0), inter = V(0);          // per-thread partials; FP64 from the block sum on
     struct Pre { V ao, yv, br; };
     static constexpr int NP = 2;
@@ -119,12 +143,13 @@ struct AdRowStepEpi {
     __device__ __forceinline__ void operator()(int r, int kind, const V (&acc)[1], const Pre& p) {
         const V ax = acc[0];
         axn[r] = ax;
-        V y2 = p.yv + sigma * (p.br - (ax + ax - p.ao));
+        V y2 = mad(sigma, p.br - (ax + ax - p.ao), p.yv);
         if (kind) y2 = fmin(y2, V(0));
         yn[r] = y2;
+        sink(r, y2);
         const V dy = y2 - p.yv;
-        dy2 += dy * dy;
-        inter += dy * (ax - p.ao);
+        dy2 = mad(dy, dy, dy2);
+        inter = mad(dy, ax - p.ao, inter);
     }
 };
 
@@ -169,7 +194,7 @@ SPS_PASS_KERNEL ad_row_step(Args<V> a) {
     decide_step(*ctl, double(t[0]), double(t[1]));
 }
 
-template <class V>
+template <class V, class Sink = NoSink>
 struct AdColStepEpi {
     const Args<V>* a;
     const V *xc, *cc, *atyo;
@@ -177,6 +202,7 @@ struct AdColStepEpi {
     V *aty, *xn, *xs;
     V tau, wgt;
     bool accepted;
+    Sink sink = Sink{};
     V dx2 = V(0);
     struct Pre { V xj, cj, lo, hi, s, l; };
     static constexpr int NP = 1;
@@ -194,11 +220,12 @@ struct AdColStepEpi {
         return p;
     }
     __device__ __forceinline__ void finish(int j, V atyj, const Pre& p) {
-        if (accepted) { aty[j] = atyj; xs[j] = p.s + wgt * (p.xj - p.l); }
-        const V x2 = clampv(p.xj - tau * (p.cj - atyj), p.lo, p.hi);
+        if (accepted) { aty[j] = atyj; xs[j] = mad(wgt, p.xj - p.l, p.s); }
+        const V x2 = clampv(mad(-tau, p.cj - atyj, p.xj), p.lo, p.hi);
         xn[j] = x2;
+        sink(j, x2);
         const V d = x2 - p.xj;
-        dx2 += d * d;
+        dx2 = mad(d, d, dx2);
     }
     __device__ __forceinline__ void operator()(int j, int, const V (&acc)[1], const Pre& p) { finish(j, acc[0], p); }
 };
@@ -238,7 +265,7 @@ SPS_PASS_KERNEL ad_col_step(Args<V> a) {
         // as a second wave after the columns; it adds nothing to the step partials)
         const V* yc = a.Y[cur];
         for (int i = blockIdx.x * kBlock + threadIdx.x; i < a.m; i += colblocks * kBlock)
-            a.ys[i] += wgt * (yc[i] - a.yl[i]);
+            a.ys[i] = mad(wgt, yc[i] - a.yl[i], a.ys[i]);
     } else {
         for (int j = blockIdx.x * kBlock + threadIdx.x; j < a.n; j += colblocks * kBlock)
             e.finish(j, e.atyo[j], e.pre(j));
@@ -570,17 +597,20 @@ SPS_CHECK_KERNEL spmv_cols(Args<V> a, const V* y, V* out) {
 // reference's own order of operations.
 // ============================================================================
 
-template <class V>
+template <class V, class Sink = NoSink>
 struct RfColStepEpi {
     const V *tau, *c;
     V *x, *xbar, *xs;
+    Sink sink = Sink{};
     struct Pre { V xv, t, cj, s; };
     static constexpr int NP = 0;
     __device__ __forceinline__ Pre pre(int j) const { return Pre{x[j], tau[j], c[j], xs[j]}; }
     __device__ __forceinline__ void operator()(int j, int, const V (&acc)[1], const Pre& p) {
         V x2 = rn_sub(p.xv, rn_mul(p.t, rn_sub(p.cj, acc[0])));
         x2 = fmax(x2, V(0));
-        xbar[j] = rn_sub(rn_mul(V(2), x2), p.xv);
+        const V xb = rn_sub(rn_mul(V(2), x2), p.xv);
+        xbar[j] = xb;
+        sink(j, xb);
         x[j] = x2;
         xs[j] = rn_add(p.s, x2);
     }
@@ -594,16 +624,18 @@ SPS_PASS_KERNEL rf_col_step(Args<V> a) {
     visit_bins<1, V>(a.cols, blockIdx.x, a.csc, GatherOne<V>{a.Y[0]}, e);
 }
 
-template <class V>
+template <class V, class Sink = NoSink>
 struct RfRowStepEpi {
     const V *sigma, *b;
     V *y, *ys;
+    Sink sink = Sink{};
     struct Pre { V yv, s, br, acc_s; };
     static constexpr int NP = 0;
     __device__ __forceinline__ Pre pre(int r) const { return Pre{y[r], sigma[r], b[r], ys[r]}; }
     __device__ __forceinline__ void operator()(int r, int, const V (&acc)[1], const Pre& p) {
         const V y2 = rn_add(p.yv, rn_mul(p.s, rn_sub(p.br, acc[0])));
         y[r] = y2;
+        sink(r, y2);
         ys[r] = rn_add(p.acc_s, y2);
     }
 };

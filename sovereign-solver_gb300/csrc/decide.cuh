@@ -39,7 +39,7 @@ constexpr int kLagPartials = 4;
 // Returns false (and marks the state done) when the movement is not finite.
 __device__ __forceinline__ bool decide_step(Ctl& c, double dy2, double inter_signed) {
     const double w = c.omega, eta = c.eta, dx2 = c.dx2, inter = fabs(inter_signed);
-    const double move = w * dx2 + dy2 / w;
+    const double move = __fma_rn(w, dx2, dy2 / w);
     const int64_t k = c.iters + 1;
     if (!isfinite(move) || !isfinite(inter)) {
         c.done = 1;

@@ -978,13 +978,19 @@ struct Engine : EngineBase {
 
     using WindowKernel = void (*)(const Args<V>);
     WindowKernel resident_kernel(bool multi) const {
-        if (mode == SPS_MODE_ADAPTIVE) return multi ? ad_resident<V, true> : ad_resident<V, false>;
-        return multi ? rf_resident<V, true> : rf_resident<V, false>;
+        constexpr int most = res_max_threads<V>();
+        const bool few = resident_threads() <= kResThreads;
+        if (mode == SPS_MODE_ADAPTIVE)
+            return few ? (multi ? ad_resident<V, true, kResThreads> : ad_resident<V, false, kResThreads>)
+                       : (multi ? ad_resident<V, true, most> : ad_resident<V, false, most>);
+        return few ? (multi ? rf_resident<V, true, kResThreads> : rf_resident<V, false, kResThreads>)
+                   : (multi ? rf_resident<V, true, most> : rf_resident<V, false, most>);
     }
+    int resident_threads() const { return 32 * (args.res.warps + (mode == SPS_MODE_ADAPTIVE ? 1 : 0)); }
     cudaLaunchConfig_t resident_config(cudaLaunchAttribute* at) const {
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)args.res.blocks);
-        cfg.blockDim = dim3((unsigned)(32 * (args.res.warps + (mode == SPS_MODE_ADAPTIVE ? 1 : 0))));
+        cfg.blockDim = dim3((unsigned)resident_threads());
         cfg.dynamicSmemBytes = res_bytes;
         cfg.stream = st;
         at->id = cudaLaunchAttributeClusterDimension;
@@ -1035,6 +1041,9 @@ struct Engine : EngineBase {
                         t.part = P.bt.total_blocks * kWarps + b.slot0 + d[2];
                     }
                 }
+                if (std::max(t.u[0].steps, t.u[1].steps) >= 4)      // res_dots takes four steps at a time
+                    for (auto& q : t.u)
+                        if (q.steps >= 0) q.steps = (q.steps + 3) & ~3;
                 out.push_back(t);
             }
         }
@@ -1072,11 +1081,12 @@ struct Engine : EngineBase {
     // Whether the window's attempts run as one resident launch (resident.cuh), and its
     // shape.  The line is capacity: wherever every warp's task, the matrix and the
     // vectors fit one cluster the resident launch won (us per attempt, checks
-    // included, launched -> resident: 40 x 100 17.2 -> 5.7 FP32, 22.2 -> 7.9 FP64;
-    // 200 x 500 19.4 -> 6.3, 26.9 -> 9.7; 2000 x 5000 22.3 -> 9.7, 30.2 -> 13.9;
-    // 100 x 200 transportation 15.3 -> 12.5 FP32; reference mode 200 x 500 FP64 19.2
-    // -> 6.8).  The smallest cluster that fits is taken in FP32: more blocks only
-    // add to the barriers (200 x 500: 6.3 us on one block, 7.5-8.5 on 2-16).  In FP64
+    // included, launched -> resident: 40 x 100 15.4 -> 3.7 FP32, 21.9 -> 6.8 FP64;
+    // 200 x 500 18.0 -> 4.3, 25.2 -> 9.1; 2000 x 5000 20.0 -> 7.2, 29.8 -> 13.3;
+    // 100 x 200 transportation 15.2 -> 11.4 FP32; reference mode 200 x 500 FP64 18.8
+    // -> 7.0).  The smallest cluster that fits is taken in FP32: more blocks only
+    // add to the barriers (200 x 500, an earlier form: 6.3 us on one block, 7.5-8.5
+    // on 2-16).  In FP64
     // a block's products pass a pipe of two per cycle, so up to eight blocks share
     // them while one holds over kResEntries64 entries (37 x 53 transportation: 12.5
     // us on 4 blocks, 11.0 on 8; 40 x 100, 1.3k entries: 7.9 on 1, 8.8 on 2).  A
@@ -1105,19 +1115,20 @@ struct Engine : EngineBase {
             S.entries = *std::max_element(ent.begin(), ent.end());
             S.slab_rows = *std::max_element(slab.begin(), slab.end());
             S.row_warps = rp.bt.total_blocks * kWarps;
-            S.row_parts = S.row_warps + rp.nslots;
+            S.row_parts = (S.row_warps + rp.nslots + 3) & ~3;
             S.col_parts = cp.bt.total_blocks * kWarps;
             const size_t bytes = res_smem_bytes<V>(S, n, m);
             if (bytes > kResSmem) continue;
             if (sizeof(V) == 8 && C < kResMaxCluster / 2 && S.entries > kResEntries64) continue;
+            res_bytes = bytes;
+            args.res = S;
             WindowKernel k = resident_kernel(C > 1);
             if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem) != cudaSuccess ||
                 (C > 8 && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
                 cudaGetLastError();
+                args.res = ResShape{};
                 continue;
             }
-            res_bytes = bytes;
-            args.res = S;
             if (C > 1) {
                 cudaLaunchAttribute at[1];
                 const cudaLaunchConfig_t cfg = resident_config(at);

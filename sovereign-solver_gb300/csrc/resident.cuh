@@ -31,9 +31,10 @@
 namespace sps {
 
 constexpr int kResMaxCluster = 16;
-// Threads of a resident block: registers for 32 warps in FP32, 16 in FP64.
+// Threads of a resident block: 512 (128 registers each), or in FP32 1024 where an LP needs them.
+constexpr int kResThreads = 512;
 template <class V>
-constexpr int res_max_threads() { return sizeof(V) == 4 ? 1024 : 512; }
+constexpr int res_max_threads() { return sizeof(V) == 4 ? 1024 : kResThreads; }
 
 // One warp's share of a pass.  SLICED and SLAB units: lane t owns row r0 + t
 // and its entries lie 32 apart; WARP units: one row, its entries dealt to the
@@ -143,32 +144,54 @@ struct ResLane {
     }
 };
 
-// The lane's dot products of the task's two units with the vector g.
+// The lane's dot products of the task's two units with the vector g, four steps
+// of each at a time (steps are padded to that unless both units have fewer; the
+// padding adds zeros).
 template <class V>
 __device__ __forceinline__ void res_dots(const ResEntries<V>& E, const ResLane& t, const V* g, V (&acc)[2]) {
     V a0 = V(0), a1 = V(0);
     const int s0 = t.s0, s1 = t.s1;
     int p = t.ent + (threadIdx.x & 31), q = p + 32 * s0;
-    const int both = min(s0, s1);
     int k = 0;
-#pragma unroll 4
-    for (; k < both; ++k, p += 32, q += 32) {
-        int j0, j1;
-        V v0, v1;
-        E.get(p, j0, v0);
-        E.get(q, j1, v1);
-        a0 = mad(v0, g[j0], a0);
-        a1 = mad(v1, g[j1], a1);
+    if (max(s0, s1) < 4) {     // the columns of assignment and transportation LPs
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+            int j;
+            V v;
+            if (u < s0) {
+                E.get(p + 32 * u, j, v);
+                a0 = mad(v, g[j], a0);
+            }
+            if (u < s1) {
+                E.get(q + 32 * u, j, v);
+                a1 = mad(v, g[j], a1);
+            }
+        }
+        k = 4;
     }
-    const int left = max(s0, s1) - max(both, 0);
+    for (; k < min(s0, s1); k += 4, p += 128, q += 128) {
+        int j[8];
+        V v[8];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            E.get(p + 32 * u, j[u], v[u]);
+            E.get(q + 32 * u, j[4 + u], v[4 + u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            a0 = mad(v[u], g[j[u]], a0);
+            a1 = mad(v[4 + u], g[j[4 + u]], a1);
+        }
+    }
     V rest = s0 > s1 ? a0 : a1;
     int r = s0 > s1 ? p : q;
-#pragma unroll 4
-    for (k = 0; k < left; ++k, r += 32) {
-        int j;
-        V v;
-        E.get(r, j, v);
-        rest = mad(v, g[j], rest);
+    for (const int s = max(s0, s1); k < s; k += 4, r += 128) {
+        int j[4];
+        V v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) E.get(r + 32 * u, j[u], v[u]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) rest = mad(v[u], g[j[u]], rest);
     }
     if (s0 > s1) a0 = rest;
     else a1 = rest;
@@ -202,6 +225,17 @@ __device__ __forceinline__ void res_slab(const ResSlab& t, bool first, V* slab, 
 template <int NP, class V, class Get>
 __device__ __forceinline__ void res_tree(V (&tot)[NP], int count, const Get& get) {
     const int lane = threadIdx.x & 31;
+    if (count <= 32) {         // the other warps add zeros, and lanes past the values too: those steps are left out
+#pragma unroll
+        for (int p = 0; p < NP; ++p) tot[p] = V(0);
+        if (lane < count) get(lane, tot);
+        int o = 16;
+        while (o >= count) o >>= 1;
+        for (; o > 0; o >>= 1)
+#pragma unroll
+            for (int p = 0; p < NP; ++p) tot[p] += __shfl_xor_sync(0xffffffffu, tot[p], o);
+        return;                // lane 0 holds the sum
+    }
 #pragma unroll
     for (int p = 0; p < NP; ++p) tot[p] = V(0);
     for (int g = 0; g * 32 < count && g < kWarps; ++g) {
@@ -219,15 +253,18 @@ __device__ __forceinline__ void res_tree(V (&tot)[NP], int count, const Get& get
 template <int NP, class V>
 __device__ __forceinline__ void res_total(V (&tot)[NP], const V* wp, int warps, int slots) {
     res_tree<NP>(tot, warps / kWarps, [&](int b, V (&v)[NP]) {
-        V s[NP];
+        constexpr int N = kWarps * NP, per = 16 / sizeof(V);      // 16-byte reads
+        V a[N];
+        const int4* src = reinterpret_cast<const int4*>(wp + b * N);
 #pragma unroll
-        for (int p = 0; p < NP; ++p) s[p] = V(0);
+        for (int i = 0; i < N / per; ++i) reinterpret_cast<int4*>(a)[i] = src[i];
 #pragma unroll
-        for (int q = 0; q < kWarps; ++q)
+        for (int p = 0; p < NP; ++p) {
+            V s = V(0);
 #pragma unroll
-            for (int p = 0; p < NP; ++p) s[p] += wp[(b * kWarps + q) * NP + p];
-#pragma unroll
-        for (int p = 0; p < NP; ++p) v[p] += s[p];
+            for (int q = 0; q < kWarps; ++q) s += a[q * NP + p];
+            v[p] += s;
+        }
     });
     if (slots == 0) return;
     V st[NP];
@@ -239,25 +276,128 @@ __device__ __forceinline__ void res_total(V (&tot)[NP], const V* wp, int warps, 
     for (int p = 0; p < NP; ++p) tot[p] += st[p];
 }
 
+// ---- the step decision ------------------------------------------------------
+// decide_step divides three times in a row and compares in FP64: about 3 800
+// cycles of one thread (every dependent FP64 operation is 62 cycles on this GPU),
+// while every warp waits.  Here it is a chain of ten such operations with the
+// same values: what depends on the attempt number alone is formed during the
+// row pass, a quotient is a product with a reciprocal corrected once by its
+// remainder, and whether it is the rounded quotient is checked off the chain,
+// by the exact remainder; positive values are compared as integers.  Operands
+// outside the ranges this needs, and the quotients the check leaves open, take
+// decide_step itself.
+__device__ __forceinline__ int64_t res_bits(double v) { return __double_as_longlong(v); }
+__device__ __forceinline__ bool res_mid(double v) {       // 2^-300 <= |v| < 2^300
+    return ((unsigned)(__double2hiint(v) >> 20) & 0x7ffu) - 723u < 600u;
+}
+// q is a / b rounded to nearest (q > 0 near it, r = a - q b exactly): the remainder is below half
+// a unit in the last place of q times b.  A power of two has a finer grid below it: left open.
+__device__ __forceinline__ bool res_rounded(double q, double r, double b) {
+    const int h = __double2hiint(q);
+    const double half = __hiloint2double(((h >> 20) - 53) << 20, 0);
+    return res_mid(q) && ((h & 0xfffff) | __double2loint(q)) != 0 && res_bits(fabs(r)) < res_bits(half * b);
+}
+// V(a / b) from y = 1 / b rounded to nearest.  In FP32: a y is within two units in the last place
+// (of FP64) of the quotient, so it rounds as the quotient does unless it lies that
+// near to the middle between two floats.  ok: the value is certain.
+__device__ __forceinline__ void res_quot(double a, double, double y, float* out, bool* ok) {
+    const double q = a * y;
+    const unsigned low = (unsigned)__double2loint(q) & 0x1fffffffu;
+    *ok = ((unsigned)(__double2hiint(q) >> 20) & 0x7ffu) - 903u < 240u && low - 0x0ffffffcu > 8u;   // a normal float
+    *out = float(q);
+}
+__device__ __forceinline__ void res_quot(double a, double b, double y, double* out, bool* ok) {
+    double q = a * y;
+    q = __fma_rn(__fma_rn(-q, b, a), y, q);
+    *ok = res_rounded(q, __fma_rn(-q, b, a), b);
+    *out = q;
+}
+__device__ __forceinline__ void res_twice(float v, double* b, float* bf) { *bf = 2.f * fabsf(v); *b = double(*bf); }
+__device__ __forceinline__ void res_twice(double v, double* b, float* bf) { *b = 2.0 * fabs(v); *bf = float(*b); }
+
+template <class V>
+struct ResDecide {
+    double omega_inv, shrink, grow;                // 1 / omega; 1 - (k+1)^-0.3; (1 + (k+1)^-0.6) eta
+    double next;
+    int acc, usual;
+    __device__ __forceinline__ void window(const Ctl& c) { omega_inv = 1.0 / c.omega; }
+    __device__ __forceinline__ void ready(const Ctl& c) {
+        const float kk = float(c.iters + 2);
+        shrink = 1.0 - double(powf(kk, -0.3f));
+        grow = (1.0 + double(powf(kk, -0.6f))) * c.eta;
+        usual = res_mid(c.omega) && res_mid(c.eta) && res_mid(c.dx2) && res_mid(grow);
+    }
+    __device__ __forceinline__ void operator()(Ctl& c, V dy2v, V interv, V* tau, V* wgt) {
+        const double w = c.omega, eta = c.eta, wi = omega_inv;
+        const double dy2 = double(dy2v);
+        double b;
+        float bf;
+        res_twice(interv, &b, &bf);
+        if (usual && res_mid(dy2) && (__float_as_uint(bf) >> 23) - 27u < 200u) {      // 2^-100 <= bf < 2^100
+            const double y0 = double(__frcp_rn(bf));
+            const double y = __fma_rn(y0, __fma_rn(-b, y0, 1.0), y0);         // 1 / b to about 2^-46
+            double d = dy2 * wi;
+            d = __fma_rn(__fma_rn(-d, w, dy2), wi, d);
+            const double move = __fma_rn(w, c.dx2, d);
+            double q = move * y;
+            q = __fma_rn(__fma_rn(-q, b, move), y, q);
+            const double a0 = shrink * q;
+            const double nx = res_bits(a0) < res_bits(grow) ? a0 : grow;
+            bool sure;
+            res_quot(nx, w, wi, tau, &sure);
+            if (sure && res_mid(nx) && res_rounded(d, __fma_rn(-d, w, dy2), w) &&
+                res_rounded(q, __fma_rn(-q, b, move), b)) {
+                next = nx;
+                acc = res_bits(eta) <= res_bits(q);
+                *wgt = V(acc ? eta : c.eta_used);
+                return;
+            }
+        }
+        usual = 0;
+        decide_step(c, dy2, double(interv));
+        next = c.eta;
+        acc = c.accepted;
+        *tau = V(c.eta / w);
+        *wgt = V(c.eta_used);
+    }
+    // the rest of decide_step, after the other warps have their step sizes
+    __device__ __forceinline__ void record(Ctl& c) const {
+        if (usual) {
+            c.iters += 1;
+            c.window += 1;
+            c.accepted = acc;
+            if (acc) {
+                c.cur = 1 - c.cur;
+                c.eta_used = c.eta;
+                c.w_sum += c.eta;
+                c.accepted_total += 1;
+            }
+            c.eta = next;
+        }
+        c.apply = 0;
+    }
+};
+
 // The attempts of one window (check_interval of them, fewer when the solve ends).
-template <class V, bool Multi>
-__global__ void __launch_bounds__(res_max_threads<V>(), 1) ad_resident(const __grid_constant__ Args<V> a) {
+template <class V, bool Multi, int Threads>
+__global__ void __launch_bounds__(Threads, 1) ad_resident(const __grid_constant__ Args<V> a) {
     extern __shared__ __align__(16) unsigned char res_buf[];
     __shared__ Ctl c;
     __shared__ V s_sigma, s_tau, s_wgt;
     __shared__ int s_acc, s_done;
+    __shared__ ResDecide<V> decide;                // the deciding thread's
     const ResShape& S = a.res;
     const int blocks = Multi ? S.blocks : 1, rank = Multi ? (int)blockIdx.x : 0;
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool control = wid == S.warps;
     ResEntries<V> E(res_buf, S.entries);
-    V* xb = reinterpret_cast<V*>(res_buf + (sizeof(V) + 4) * (size_t)S.entries);   // x and the candidate
-    V* sy = xb + 2 * (size_t)a.n;
-    V* wr = sy + a.m;                              // row pass: dy2, inter per warp, then per SLAB slice
+    V* wr = reinterpret_cast<V*>(res_buf + (sizeof(V) + 4) * (size_t)S.entries);   // row pass: dy2, inter per warp, then per SLAB slice
     V* wc = wr + 2 * S.row_parts;                  // column pass: dx2 per warp
     V* wj = wc + S.col_parts;                      // rejected attempt: dx2 per warp
-    V* slab = wj + S.col_parts;
-    const int row_slots = S.row_parts - S.row_warps;
+    V* xb = wj + S.col_parts;                      // x and the candidate
+    V* sy = xb + 2 * (size_t)a.n;
+    V* slab = sy + a.m;
+    const int row_slots = a.csr.nsegrows;
     if (threadIdx.x == 0) {
         c = *a.ctl;
         s_sigma = V(c.eta * c.omega);
@@ -304,6 +444,7 @@ __global__ void __launch_bounds__(res_max_threads<V>(), 1) ad_resident(const __g
             aty[h] = a.ATY[cur][j];
         }
     }
+    if (control && lane == 0) decide.window(c);
     res_barrier<Multi>();
     bool rejected = false;                         // the last column pass took the rejected branch
     int w = 0;
@@ -316,6 +457,7 @@ __global__ void __launch_bounds__(res_max_threads<V>(), 1) ad_resident(const __g
                 res_total<1>(d, rejected ? wj : wc, S.col_parts, 0);
                 if (lane == 0) c.dx2 = double(d[0]);
             }
+            if (lane == 0) decide.ready(c);
             if (S.slab_rows) __syncthreads();
         } else {
             if (rt.any()) res_dots(E, rt, xb + (size_t)(1 - cur) * a.n, axn);
@@ -348,13 +490,12 @@ __global__ void __launch_bounds__(res_max_threads<V>(), 1) ad_resident(const __g
             V t[2];
             res_total<2>(t, wr, S.row_warps, row_slots);
             if (lane == 0) {
-                decide_step(c, double(t[0]), double(t[1]));
-                s_acc = c.accepted;
+                V tau, wgt;
+                decide(c, t[0], t[1], &tau, &wgt);
+                s_acc = decide.acc;
                 s_done = c.done;
-                s_tau = V(c.eta / c.omega);
-                s_wgt = V(c.eta_used);
-                s_sigma = V(c.eta * c.omega);
-                c.apply = 0;
+                s_tau = tau;
+                s_wgt = wgt;
             }
         } else if (ct.any()) {
             res_dots(E, ct, sy, g);
@@ -363,6 +504,10 @@ __global__ void __launch_bounds__(res_max_threads<V>(), 1) ad_resident(const __g
         if (s_done) break;
         const V tau = s_tau, wgt = s_wgt;
         rejected = !s_acc;
+        if (control && lane == 0) {
+            decide.record(c);
+            s_sigma = V(c.eta * c.omega);
+        }
         if (s_acc) {
             cur ^= 1;
 #pragma unroll
@@ -439,16 +584,16 @@ __global__ void __launch_bounds__(res_max_threads<V>(), 1) ad_resident(const __g
 
 // Reference mode: the iterations of one window (RfColStepEpi, RfRowStepEpi; no
 // sums, so every warp works).
-template <class V, bool Multi>
-__global__ void __launch_bounds__(res_max_threads<V>(), 1) rf_resident(const __grid_constant__ Args<V> a) {
+template <class V, bool Multi, int Threads>
+__global__ void __launch_bounds__(Threads, 1) rf_resident(const __grid_constant__ Args<V> a) {
     extern __shared__ __align__(16) unsigned char res_buf[];
     const ResShape& S = a.res;
     const int blocks = Multi ? S.blocks : 1, rank = Multi ? (int)blockIdx.x : 0;
     const int wid = threadIdx.x >> 5;
     ResEntries<V> E(res_buf, S.entries);
     V* sx = reinterpret_cast<V*>(res_buf + (sizeof(V) + 4) * (size_t)S.entries);
-    V* sy = sx + 2 * (size_t)a.n;
-    V* slab = sy + a.m + 2 * S.row_parts + 2 * S.col_parts;
+    V* sy = sx + a.n;
+    V* slab = sy + a.m;
     Ctl* ctl = a.ctl;
     const int64_t iters = ctl->iters, left = ctl->max_iters - iters;
     if (ctl->done || left <= 0) return;                    // every block reads the same

@@ -154,30 +154,96 @@ __device__ __forceinline__ T group_sum(T v) {
     return v;
 }
 
+// NP sums over the warp at once: at each butterfly step a lane keeps half of its
+// values and hands the others to its partner, so the warp makes about NP
+// additions in all where NP butterflies make 5 NP (each costs an FP64 warp 16
+// cycles of the pipe).  Every value is added in the butterfly's own tree, so the
+// sums have the same bits.  On return the lane holds the sum of value *which
+// (< NP rounded up to a power of two; lanes that share it hold the same).
+template <int N, int O, class T>
+__device__ __forceinline__ T warp_sums_step(T (&v)[N], int& which) {
+    if constexpr (N == 1) {
+#pragma unroll
+        for (int o = O; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        return v[0];
+    } else {
+        constexpr int H = N / 2;
+        const bool up = threadIdx.x & O;
+        T keep[H];
+#pragma unroll
+        for (int i = 0; i < H; ++i) {
+            const T give = up ? v[i] : v[H + i];
+            keep[i] = (up ? v[H + i] : v[i]) + __shfl_xor_sync(0xffffffffu, give, O);
+        }
+        if (up) which += H;
+        return warp_sums_step<H, O / 2>(keep, which);
+    }
+}
+__host__ __device__ constexpr int pow2_ceil(int n) { return n <= 1 ? 1 : 2 * pow2_ceil((n + 1) / 2); }
+template <int NP, class T>
+__device__ __forceinline__ T warp_sums(T (&v)[NP], int* which) {
+    constexpr int N = pow2_ceil(NP);
+    static_assert(N <= 32, "a warp holds 32 sums");
+    T p[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) p[i] = i < NP ? v[i < NP ? i : 0] : T(0);
+    *which = 0;
+    return warp_sums_step<N, 16>(p, *which);
+}
+
 // Sum NP values over the block; result valid in thread 0.  Fixed order.  T is
 // float in the FP32 engine's iteration kernels: this GPU issues FP64 at 1/64 of
 // the FP32 rate (2 thread operations per SM cycle), so a 256-thread FP64 shuffle
 // tree per block and per attempt costs more than the block's own FP32 work.
+// In FP64 the values of a warp are summed together, a warp that has none (its
+// units are done elsewhere) writes its zeros at once, and a thread per value
+// adds the warps: the tail of a check (four of these sums of 11 to 18 values
+// by one block, 62 cycles per dependent addition) took 24 of the 60 us of a
+// 40 x 100 LP's column check and a third of a transportation LP's.
 template <int NP, class T>
 __device__ __forceinline__ void block_sum(T (&v)[NP], T* smem /* kWarps*NP */) {
-#pragma unroll
-    for (int p = 0; p < NP; ++p) v[p] = group_sum<32>(v[p]);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    __syncthreads();
-    if (l == 0) {
+    if constexpr (sizeof(T) == 8 && NP >= 2) {
+        unsigned bits = 0u;
 #pragma unroll
-        for (int p = 0; p < NP; ++p) smem[w * NP + p] = v[p];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
+        for (int p = 0; p < NP; ++p) bits |= (unsigned)__double2hiint(v[p]) | (unsigned)__double2loint(v[p]);
+        constexpr int same = 32 / pow2_ceil(NP);          // lanes that end with one value's sum
+        int which = (l / same < NP) ? l / same : NP;      // any lane's value will do for zeros
+        T mine = T(0);
+        if (__any_sync(0xffffffffu, bits != 0u)) mine = warp_sums<NP>(v, &which);
+        __syncthreads();
+        if (which < NP) smem[w * NP + which] = mine;
+        __syncthreads();
+        if (threadIdx.x < NP) {
             T s = T(0);
-            for (int q = 0; q < kWarps; ++q) s += smem[q * NP + p];
-            v[p] = s;
+#pragma unroll
+            for (int q = 0; q < kWarps; ++q) s += smem[q * NP + threadIdx.x];
+            smem[threadIdx.x] = s;                        // its own column's first entry
         }
+        __syncthreads();
+        if (threadIdx.x == 0)
+#pragma unroll
+            for (int p = 0; p < NP; ++p) v[p] = smem[p];
+        __syncthreads();
+    } else {
+#pragma unroll
+        for (int p = 0; p < NP; ++p) v[p] = group_sum<32>(v[p]);
+        __syncthreads();
+        if (l == 0) {
+#pragma unroll
+            for (int p = 0; p < NP; ++p) smem[w * NP + p] = v[p];
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                T s = T(0);
+                for (int q = 0; q < kWarps; ++q) s += smem[q * NP + p];
+                v[p] = s;
+            }
+        }
+        __syncthreads();
     }
-    __syncthreads();
 }
 
 // Ticket counters (a kernel's blocks, a SLAB slice's units, a SEGMENT row's

@@ -922,6 +922,10 @@ struct Engine : EngineBase {
                 SPS_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nr, rf_row_check<V>, kBlock, 0));
                 SPS_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nc, rf_col_check<V>, kBlock, 0));
             }
+            // the blocks' shares are part of the sums' order: at most the counts that order
+            // was set with, whatever registers a later compilation needs
+            nr = std::min(nr, sizeof(V) == 4 ? 3 : 2);
+            nc = std::min(nc, adaptive || sizeof(V) == 8 ? 2 : 3);
             a.rows_chk = rp.bt;
             a.cols_chk = cp.bt;
             share_blocks(a.rows_chk, rp.bin_store, std::min(block_cap, kSms * std::max(nr, 1)));

@@ -23,8 +23,9 @@
 // by every GPU that loads the library until the process exits:
 //   [0, 3 kMaxCols)                        three digit accumulators per column
 //   [kPartBase, + 2 kMaxBlocks kParts)     per-block partial sums of the two passes
-//   kMaxSlot                               largest |a_ij y_i| (bits), cleared each call
-//   kTicketSlot                            ticket of the column pass, cleared each call
+//   [kMaxBase, + kMaxBlocks)               per-block largest |a_ij y_i| (bits)
+//   kTicketSlot                            ticket of the column pass
+// (all written by the call's first pass before they are read: no clearing launches)
 // Limits: n <= kMaxCols (262144) columns; any number of rows.
 // Every call shares the array: two calls that overlap on the GPU (different
 // streams, or different host threads without ordering) race and return
@@ -52,8 +53,8 @@ constexpr int kParts = 4;
 constexpr int kMaxCols = 1 << 18;
 constexpr int kDigits = 3;
 constexpr int kPartBase = kDigits * kMaxCols;
-constexpr int kMaxSlot = kPartBase + 2 * kMaxBlocks * kParts;
-constexpr int kTicketSlot = kMaxSlot + 1;
+constexpr int kMaxBase = kPartBase + 2 * kMaxBlocks * kParts;
+constexpr int kTicketSlot = kMaxBase + kMaxBlocks;
 constexpr int kScratchWords = kTicketSlot + 31;
 
 static __device__ __align__(256) double g_noalloc_scratch[kScratchWords];
@@ -129,19 +130,40 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// Block sum of kParts values into part[blockIdx.x * kParts + q] (fixed order).
-__device__ __forceinline__ void store_block_partials(double (&v)[kParts], double* part) {
-    __shared__ double sm[kThreads / 32][kParts];
-    for (int q = 0; q < kParts; ++q) v[q] = warp_sum(v[q]);
+// Sums of N values over the block in a fixed order, into out[0, N) (a thread per
+// value adds the warps; FP64 additions are 62 cycles each on this GPU).  Ends
+// with a barrier.
+template <int N>
+__device__ __forceinline__ void block_total(double (&v)[N], double* out) {
+    __shared__ double sm[kThreads / 32][N];
+    long long any = 0;             // a warp without values writes its zeros at once
+#pragma unroll
+    for (int q = 0; q < N; ++q) any |= __double_as_longlong(v[q]);
+    if (__any_sync(0xffffffffu, any != 0))
+#pragma unroll
+        for (int q = 0; q < N; ++q) v[q] = warp_sum(v[q]);
     if ((threadIdx.x & 31) == 0)
-        for (int q = 0; q < kParts; ++q) sm[threadIdx.x >> 5][q] = v[q];
+#pragma unroll
+        for (int q = 0; q < N; ++q) sm[threadIdx.x >> 5][q] = v[q];
     __syncthreads();
-    if (threadIdx.x == 0)
-        for (int q = 0; q < kParts; ++q) {
-            double s = 0.0;
-            for (int w = 0; w < kThreads / 32; ++w) s += sm[w][q];
-            part[blockIdx.x * kParts + q] = s;
-        }
+    if (threadIdx.x < N) {
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < kThreads / 32; ++w) s += sm[w][threadIdx.x];
+        out[threadIdx.x] = s;
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ unsigned long long block_max(unsigned long long v) {
+    __shared__ unsigned long long sm[kThreads / 32];
+    for (int o = 16; o > 0; o >>= 1) v = max(v, (unsigned long long)__shfl_xor_sync(0xffffffffu, v, o));
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = sm[0];
+#pragma unroll
+    for (int w = 1; w < kThreads / 32; ++w) v = max(v, sm[w]);
+    return v;
 }
 
 // Grid of the digits: e0 = exponent with max|a_ij y_i| < 2^e0, b bits per digit.
@@ -150,10 +172,14 @@ struct Grid {
     bool finite;
 };
 
-__device__ __forceinline__ Grid grid_of(const sps_device_lp& lp, const double* s) {
+// All threads of the block; row_blocks: the blocks of the first pass.
+__device__ __forceinline__ Grid grid_of(const sps_device_lp& lp, const double* s, int row_blocks) {
     const int m = lp.m_ub + lp.m_eq;
     const long long nnz = m > 0 ? (long long)max(lp.indptr[m], 0) : 0ll;
-    const unsigned long long bits = *reinterpret_cast<const unsigned long long*>(s + kMaxSlot);
+    unsigned long long bits = 0ull;
+    for (int b = threadIdx.x; b < row_blocks; b += kThreads)
+        bits = max(bits, __ldcg(reinterpret_cast<const unsigned long long*>(s + kMaxBase) + b));
+    bits = block_max(bits);
     Grid g;
     g.finite = bits < 0x7FF0000000000000ull;
     const int ex = (int)(bits >> 52);                 // biased exponent of the largest |product|
@@ -164,57 +190,125 @@ __device__ __forceinline__ Grid grid_of(const sps_device_lp& lp, const double* s
     return g;
 }
 
-// Pass 1, one warp per row: largest |a_ij y_i| (as bits: non-negative doubles
-// order like their bit patterns, so an integer max is order-independent).
+// Rows of a warp: four at a time, eight lanes each (most rows hold a few dozen
+// nonzeros: a warp per row left its lanes idle and its next row's offsets one
+// round trip away), rows of over kLongRow nonzeros by the whole warp after
+// them.  visit(i, k, lanes) runs the lane's share of row i: nonzeros k, k +
+// lanes, ...; done(i, lanes) ends it, in all of the row's lanes.
+constexpr int kRowLanes = 8;
+constexpr int kLongRow = 256;
+template <class Visit, class Done>
+__device__ __forceinline__ void rows_of_warp(const int32_t* __restrict__ ptr, int m, const Visit& visit, const Done& done) {
+    constexpr int per = 32 / kRowLanes;
+    const int lane = threadIdx.x & 31;
+    const int warps = (gridDim.x * kThreads) >> 5;
+    for (int i0 = ((blockIdx.x * kThreads + threadIdx.x) >> 5) * per; i0 < m; i0 += warps * per) {
+        const int i = i0 + lane / kRowLanes;
+        const int b = i < m ? ptr[i] : 0, e = i < m ? ptr[i + 1] : 0;
+        const bool lng = e - b > kLongRow;
+        if (!lng) visit(i, b + (lane & (kRowLanes - 1)), e, kRowLanes);
+        unsigned todo = __ballot_sync(0xffffffffu, lng && (lane & (kRowLanes - 1)) == 0);
+        done(i, i < m && !lng, kRowLanes);
+        while (todo) {                              // warp-uniform
+            const int src = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const int il = __shfl_sync(0xffffffffu, i, src);
+            const int bl = __shfl_sync(0xffffffffu, b, src), el = __shfl_sync(0xffffffffu, e, src);
+            visit(il, bl + lane, el, 32);
+            done(il, true, 32);
+        }
+    }
+}
+
+// Pass 1: largest |a_ij y_i| (as bits: non-negative doubles order like their bit
+// patterns, so an integer max is order-independent), one per block; clears the
+// columns' accumulators for pass 2 and the ticket of pass 3.
 __global__ void __launch_bounds__(kThreads) na_max(sps_device_lp lp, const double* __restrict__ y,
                                                      double* __restrict__ s) {
     const int m = lp.m_ub + lp.m_eq;
-    const int lane = threadIdx.x & 31;
+    for (int j = blockIdx.x * kThreads + threadIdx.x; j < lp.n; j += gridDim.x * kThreads)
+#pragma unroll
+        for (int d = 0; d < kDigits; ++d) s[(size_t)d * kMaxCols + j] = 0.0;
     unsigned long long mx = 0ull;
-    for (int i = (blockIdx.x * kThreads + threadIdx.x) >> 5; i < m; i += (gridDim.x * kThreads) >> 5) {
-        const double yi = y[i];
-        for (int k = lp.indptr[i] + lane; k < lp.indptr[i + 1]; k += 32) {
-            const double p = fabs(lp.values[k] * yi);
-            const unsigned long long pb = isnan(p) ? 0x7FF8000000000000ull : __double_as_longlong(p);
-            mx = max(mx, pb);
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, (unsigned long long)__shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0 && mx) atomicMax(reinterpret_cast<unsigned long long*>(s + kMaxSlot), mx);
+    const double* __restrict__ val = lp.values;
+    rows_of_warp(lp.indptr, m,
+        [&](int i, int k, int e, int lanes) {
+            if (k >= e) return;
+            const double yi = y[i];
+#pragma unroll 4
+            for (; k < e; k += lanes) {
+                const double p = fabs(val[k] * yi);
+                const unsigned long long pb = isnan(p) ? 0x7FF8000000000000ull : __double_as_longlong(p);
+                mx = max(mx, pb);
+            }
+        },
+        [](int, bool, int) {});
+    mx = block_max(mx);
+    if (threadIdx.x != 0) return;
+    reinterpret_cast<unsigned long long*>(s + kMaxBase)[blockIdx.x] = mx;
+    if (blockIdx.x == 0) *reinterpret_cast<unsigned int*>(s + kTicketSlot) = 0u;
 }
 
-// Pass 2, one warp per row: residual of K x against the rhs (<= rows count
-// only violations), rhs^T y, ||rhs||^2, sign violations of y on <= rows, and
-// the digits of every product a_ij y_i added into column j's accumulators.
+// Pass 2: residual of K x against the rhs (<= rows count only violations),
+// rhs^T y, ||rhs||^2, sign violations of y on <= rows, and the digits of every
+// product a_ij y_i added into column j's accumulators.  The digits are cut from
+// the product's mantissa with integer shifts (as magnitudes, with the
+// product's sign): cut with FP64 scalings and conversions, about twenty
+// operations of the FP64 pipe per nonzero, this pass took 217 us on 1.5M
+// nonzeros; with two left, 49 us (the 64-bit atomics, up to three per nonzero,
+// are what is left).  The whole call: 60k x 150k, 1.5M nonzeros 578 -> 105 us,
+// 5k x 12k 183 -> 35 us, 300 x 700 48 -> 31 us.
 __global__ void __launch_bounds__(kThreads) na_rows(sps_device_lp lp, const double* __restrict__ x,
                                                      const double* __restrict__ y, double* __restrict__ s) {
     double v[kParts] = {0.0, 0.0, 0.0, 0.0};
     const int m = lp.m_ub + lp.m_eq;
     const int lane = threadIdx.x & 31;
-    const Grid g = grid_of(lp, s);
+    const Grid g = grid_of(lp, s, gridDim.x);
     unsigned long long* acc = reinterpret_cast<unsigned long long*>(s);
-    for (int i = (blockIdx.x * kThreads + threadIdx.x) >> 5; i < m; i += (gridDim.x * kThreads) >> 5) {
-        const double yi = y[i];
-        double sum = 0.0;
-        for (int k = lp.indptr[i] + lane; k < lp.indptr[i + 1]; k += 32) {
-            const double a = lp.values[k];
-            const int j = lp.indices[k];
-            sum += a * x[j];
-            if (!g.finite) continue;
-            // digits of p on the grids 2^(e0-b), 2^(e0-2b), 2^(e0-3b): each scaling by a
-            // power of two and each remainder is exact, so only the last digit rounds
-            double r = a * yi;
-            for (int d = 0; d < kDigits; ++d) {
-                const int e = g.e0 - (d + 1) * g.b;
-                const long long q = __double2ll_rn(scalbn(r, -e));
-                if (q) atomicAdd(acc + (size_t)d * kMaxCols + j, (unsigned long long)q);
-                r -= scalbn((double)q, e);
+    const int unit = g.e0 - kDigits * g.b;                 // the finest grid's exponent
+    const unsigned long long mask = (1ull << g.b) - 1ull;
+    const double* __restrict__ val = lp.values;
+    const int32_t* __restrict__ idx = lp.indices;
+    double sum = 0.0;
+    rows_of_warp(lp.indptr, m,
+        [&](int i, int k, int e, int lanes) {
+            if (k >= e) return;
+            const double yi = y[i];
+#pragma unroll 2
+            for (; k < e; k += lanes) {
+                const double a = val[k];
+                const int j = idx[k];
+                sum += a * x[j];
+                if (!g.finite) continue;
+                const unsigned long long bits = __double_as_longlong(a * yi);
+                const int ex = (int)(bits >> 52) & 0x7ff;
+                unsigned long long mant = bits & 0xfffffffffffffull;
+                if (ex) mant |= 1ull << 52;
+                int sh = (ex ? ex - 1075 : -1074) - unit;  // the product is mant 2^sh finest units
+                if (sh < 0) {                              // only the last digit rounds (to nearest)
+                    mant = sh < -53 ? 0ull : ((mant >> (-sh - 1)) + 1ull) >> 1;
+                    sh = 0;
+                }
+                const bool neg = (long long)bits < 0;
+#pragma unroll
+                for (int d = 0; d < kDigits; ++d) {
+                    const int r = (kDigits - 1 - d) * g.b - sh;   // the digit's place in mant
+                    const unsigned long long q = (r > 63 ? 0ull : r >= 0 ? mant >> r : -r > 63 ? 0ull : mant << -r) &
+                                                 (d == 0 ? ~0ull : mask);
+                    if (q) atomicAdd(acc + (size_t)d * kMaxCols + j, neg ? 0ull - q : q);
+                }
             }
-        }
-        sum = warp_sum(sum);
-        if (lane == 0) {
-            const double b = lp.rhs[i];
-            double res = sum - b;
+        },
+        [&](int i, bool row, int lanes) {
+            double t = sum;
+            sum = 0.0;
+            if (lanes == 32)
+                for (int o = 16; o >= kRowLanes; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+#pragma unroll
+            for (int o = kRowLanes / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            if (!row || (lane & (lanes - 1)) != 0) return;
+            const double b = lp.rhs[i], yi = y[i];
+            double res = t - b;
             double sign = 0.0;
             if (i < lp.m_ub) {
                 res = fmax(res, 0.0);
@@ -224,9 +318,13 @@ __global__ void __launch_bounds__(kThreads) na_rows(sps_device_lp lp, const doub
             v[1] += b * yi;
             v[2] += b * b;
             v[3] += sign * sign;
-        }
-    }
-    store_block_partials(v, s + kPartBase);
+        });
+    block_total(v, s + kPartBase + blockIdx.x * kParts);
+}
+
+// 2^e as a factor; scalbn where that is no normal number.
+__device__ __forceinline__ double scaled(double v, int e) {
+    return e >= -1022 && e <= 1023 ? v * __hiloint2double((e + 1023) << 20, 0) : scalbn(v, e);
 }
 
 // Pass 3, one thread per column, and the final reduction in the last block.
@@ -235,13 +333,13 @@ __global__ void __launch_bounds__(kThreads) na_cols(sps_device_lp lp, const doub
                                                      double* __restrict__ s, int row_blocks,
                                                      double* __restrict__ out) {
     double v[kParts] = {0.0, 0.0, 0.0, 0.0};
-    const Grid g = grid_of(lp, s);
+    const Grid g = grid_of(lp, s, row_blocks);
     const long long* acc = reinterpret_cast<const long long*>(s);
     for (int j = blockIdx.x * kThreads + threadIdx.x; j < lp.n; j += gridDim.x * kThreads) {
         const double cj = lp.c[j], lo = lp.lb[j], hi = lp.ub[j];
         const bool hl = isfinite(lo), hh = isfinite(hi);
         double aty = 0.0;      // coarse digit first: two roundings in a fixed order
-        for (int d = 0; d < kDigits; ++d) aty += scalbn((double)acc[(size_t)d * kMaxCols + j], g.e0 - (d + 1) * g.b);
+        for (int d = 0; d < kDigits; ++d) aty += scaled((double)acc[(size_t)d * kMaxCols + j], g.e0 - (d + 1) * g.b);
         if (!g.finite) aty = NAN;
         const double r = cj - aty;
         const double lam = (hl && hh) ? r : hl ? fmax(r, 0.0) : hh ? fmin(r, 0.0) : 0.0;
@@ -251,21 +349,28 @@ __global__ void __launch_bounds__(kThreads) na_cols(sps_device_lp lp, const doub
         v[2] += (hl ? lo * fmax(lam, 0.0) : 0.0) + (hh ? hi * fmin(lam, 0.0) : 0.0);
         v[3] += cj * cj;
     }
-    store_block_partials(v, s + kPartBase + kMaxBlocks * kParts);
+    block_total(v, s + kPartBase + (kMaxBlocks + blockIdx.x) * kParts);
     __shared__ bool last;
     if (threadIdx.x == 0) {
         __threadfence();
         unsigned int* ticket = reinterpret_cast<unsigned int*>(s + kTicketSlot);
         last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        __threadfence();
     }
     __syncthreads();
-    if (!last || threadIdx.x != 0) return;
-    __threadfence();
-    double R[kParts] = {0, 0, 0, 0}, Cc[kParts] = {0, 0, 0, 0};
-    for (int b = 0; b < row_blocks; ++b)
-        for (int q = 0; q < kParts; ++q) R[q] += __ldcg(s + kPartBase + b * kParts + q);
-    for (int b = 0; b < (int)gridDim.x; ++b)
-        for (int q = 0; q < kParts; ++q) Cc[q] += __ldcg(s + kPartBase + kMaxBlocks * kParts + b * kParts + q);
+    if (!last) return;
+    // both passes' block partials: thread t adds blocks t, t + 256, ... of each, then the
+    // block's fixed tree (one thread took them one by one, an L2 round trip each:
+    // 0.4 of the 0.58 ms of a call on 1.5M nonzeros)
+    double w[2 * kParts] = {};
+    for (int b = threadIdx.x; b < row_blocks; b += kThreads)
+        for (int q = 0; q < kParts; ++q) w[q] += __ldcg(s + kPartBase + b * kParts + q);
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += kThreads)
+        for (int q = 0; q < kParts; ++q) w[kParts + q] += __ldcg(s + kPartBase + kMaxBlocks * kParts + b * kParts + q);
+    __shared__ double fin[2 * kParts];
+    block_total(w, fin);
+    if (threadIdx.x != 0) return;
+    const double *R = fin, *Cc = fin + kParts;
     const double rp = sqrt(R[0]) / (1.0 + sqrt(R[2]));
     const double rd = sqrt(Cc[0] + R[3]) / (1.0 + sqrt(Cc[3]));
     const double po = Cc[1], dob = R[1] + Cc[2];
@@ -276,7 +381,6 @@ __global__ void __launch_bounds__(kThreads) na_cols(sps_device_lp lp, const doub
     out[3] = gap;
     out[4] = po;
     out[5] = dob;
-    *reinterpret_cast<unsigned int*>(s + kTicketSlot) = 0u;
 }
 
 }  // namespace
@@ -306,19 +410,13 @@ extern "C" int sps_kkt_noalloc(const sps_device_lp* lp, const double* x, const d
     double* s = nullptr;
     if (int rc = scratch_address(&s)) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // clear what must start at zero: the digit accumulators, the max and the ticket
-    cudaError_t e = cudaSuccess;
-    for (int d = 0; d < kDigits && e == cudaSuccess && lp->n > 0; ++d)
-        e = cudaMemsetAsync(s + (size_t)d * kMaxCols, 0, sizeof(double) * (size_t)lp->n, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(s + kMaxSlot, 0, 2 * sizeof(double), st);
-    const int row_blocks = (int)std::min<int64_t>(kMaxBlocks, std::max<int64_t>(1, ((int64_t)m * 32 + kThreads - 1) / kThreads));
+    // a warp takes 32 / kRowLanes rows at a time
+    const int row_blocks = (int)std::min<int64_t>(kMaxBlocks, std::max<int64_t>(1, ((int64_t)m * kRowLanes + kThreads - 1) / kThreads));
     const int col_blocks = (int)std::min<int64_t>(kMaxBlocks, std::max<int64_t>(1, ((int64_t)lp->n + kThreads - 1) / kThreads));
-    if (e == cudaSuccess) {
-        na_max<<<row_blocks, kThreads, 0, st>>>(*lp, y, s);
-        na_rows<<<row_blocks, kThreads, 0, st>>>(*lp, x, y, s);
-        na_cols<<<col_blocks, kThreads, 0, st>>>(*lp, x, s, row_blocks, out);
-        e = cudaGetLastError();
-    }
+    na_max<<<row_blocks, kThreads, 0, st>>>(*lp, y, s);
+    na_rows<<<row_blocks, kThreads, 0, st>>>(*lp, x, y, s);
+    na_cols<<<col_blocks, kThreads, 0, st>>>(*lp, x, s, row_blocks, out);
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         sps::set_create_error(std::string("sps_kkt_noalloc: ") + cudaGetErrorString(e));
         return SPS_ERR_CUDA;

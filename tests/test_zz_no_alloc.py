@@ -113,3 +113,44 @@ def test_noalloc_rejects_null_arrays(missing):
     rc = lib.sps_kkt_noalloc(C.byref(lp), 8, 8, 8, None)
     assert rc == -1
     assert b"null device array" in lib.sps_last_error(None)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lengths,spread", [
+    ([1, 7, 8, 9, 31, 32, 33, 255, 256, 257, 700, 0, 2], 0),     # around the lanes of a row and the long-row limit
+    ([5] * 130, 0), ([0] * 40 + [1], 0), ([257] * 9, 0),         # (an LP without entries has null arrays: refused)
+    ([12] * 70, 30),                                             # products over 60 decades: every digit, and below the last
+])
+def test_noalloc_kkt_row_schedules(lengths, spread):
+    """Rows around the schedule's edges and products of very different sizes against FP64 sums
+    (2 ** -50 of the sum of magnitudes: FP64 sums of at most 1500 terms in another order)."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    rng = np.random.default_rng(5)
+    m, n = len(lengths), 900
+    idx = np.concatenate([np.sort(rng.choice(n, k, replace=False)) for k in lengths]).astype(np.int32)
+    val = rng.standard_normal(idx.size) * 10.0 ** rng.uniform(-spread, spread, idx.size)
+    A = sp.csr_matrix((val, idx, np.concatenate([[0], np.cumsum(lengths)])), shape=(m, n))
+    k = m // 3
+    p = sps.Problem(c=rng.standard_normal(n), A_ub=A[:k], b_ub=rng.standard_normal(k), A_eq=A[k:],
+                    b_eq=rng.standard_normal(m - k), lb=np.zeros(n), ub=np.full(n, 3.0), integer_mask=np.zeros(n, bool))
+    x, y = rng.random(n), rng.standard_normal(m)
+    lib, (lp, keep) = N.load(), _device_lp(torch, p)
+    xd, yd = (torch.tensor(v, dtype=torch.float64, device="cuda") for v in (x, y))
+    outs = []
+    for _ in range(2):
+        out = torch.full((6,), float("nan"), dtype=torch.float64, device="cuda")
+        assert lib.sps_kkt_noalloc(C.byref(lp), xd.data_ptr(), yd.data_ptr(), out.data_ptr(), None) == 0
+        torch.cuda.synchronize()
+        outs.append(out.cpu().numpy())
+    assert np.array_equal(outs[0], outs[1])
+    rhs = np.concatenate([p.b_ub, p.b_eq])
+    res = A @ x - rhs
+    res[:k] = np.maximum(res[:k], 0)
+    rc = p.c - A.T @ y
+    po, do = p.c @ x, rhs @ y + 3.0 * np.minimum(rc, 0).sum()
+    eps = 2.0 ** -50
+    assert abs(outs[0][1] - np.linalg.norm(res) / (1 + np.linalg.norm(rhs))) <= eps * (1 + np.linalg.norm(abs(A) @ x))
+    assert abs(outs[0][4] - po) <= eps * (abs(p.c) @ x)
+    assert abs(outs[0][5] - do) <= eps * (abs(rhs) @ abs(y) + 3.0 * (abs(p.c) + abs(A).T @ abs(y)).sum())

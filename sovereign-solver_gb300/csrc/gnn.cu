@@ -266,6 +266,14 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
                  : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
 }  // namespace tc
 
 __global__ void __launch_bounds__(kT, 2) k_update_tc(const float* __restrict__ h, const float* __restrict__ a,
@@ -382,6 +390,415 @@ __global__ void __launch_bounds__(kT, 2) k_update_tc(const float* __restrict__ h
     __syncthreads();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tc::kTmemCols) : "memory");
+}
+
+// ---- the variable side's node update on the tensor cores (H = 64) --------------------
+// relu(U h + M a + b) with a_j = sum_i a_ij hc_i is relu(U h + sum_i a_ij (M hc_i) + b):
+// M is applied to the constraint nodes (a few thousand) instead of to every
+// variable node's aggregate, so the aggregate is neither written nor read and
+// the large contraction has K = 64 instead of 128.  What is left is a stream: h
+// in, out (512 bytes a node), the rows of M hc from L2.  On 1.28M nodes (16
+// instances of the 200 x 400 family) a layer's aggregation and update took 180 +
+// 300 us; now 229 us (0.66 GB, 96 us at the measured HBM rate: the chain staging ->
+// MMA -> edges -> read-back of each tile, two blocks an SM, is what is left).
+//
+// FP32 activations as three BF16 parts (8 bits of mantissa each, all 24), the
+// weights exact in BF16: three products per step, accumulated in FP32, agree
+// with FP32 arithmetic.  A tile is 128 nodes: a part is 128 rows of 128 bytes
+// (128-byte swizzle: 16-byte piece q of row r at piece q ^ (r & 7)), staged by all
+// threads from registers that were loaded while the last tile was computed.
+// Every wait is bounded; a block that gives up sets *err and stops.
+namespace bf {
+constexpr int kPart = 128 * 128;              // one BF16 part of a 128-node tile (16 KB)
+constexpr int kW = 64 * 128;                  // a 64 x 64 weight matrix (8 KB)
+// instruction descriptor: D F32, A and B BF16
+__host__ __device__ constexpr uint32_t idesc(int M, int N, bool transA, bool transB) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((transA ? 1u : 0u) << 15) | ((transB ? 1u : 0u) << 16) |
+           ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+template <uint32_t Idesc>
+__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(d), "l"(a), "l"(b), "n"(Idesc), "r"(accumulate) : "memory");
+}
+// four floats as three parts of four BF16 values, cut by truncation (masks and exact
+// subtractions: the three parts of 8 bits add up to the float itself)
+__device__ __forceinline__ uint32_t upper(float a, float b) {
+    return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+}
+__device__ __forceinline__ float cut(float v) { return __uint_as_float(__float_as_uint(v) & 0xffff0000u); }
+__device__ __forceinline__ void split(const float4& x, uint2 (&p)[3]) {
+    float4 r = x;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        p[q] = make_uint2(upper(r.x, r.y), upper(r.z, r.w));
+        if (q < 2) r = make_float4(r.x - cut(r.x), r.y - cut(r.y), r.z - cut(r.z), r.w - cut(r.w));
+    }
+}
+// piece f (four floats) of row r of a tile's parts
+__device__ __forceinline__ void put(unsigned char* parts, int r, int f, const float4& x) {
+    uint2 p[3];
+    split(x, p);
+    const int off = r * 128 + (((f >> 1) ^ (r & 7)) << 4) + ((f & 1) << 3);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(parts + q * kPart + off) = p[q];
+}
+// W (64 x 64 BF16, row-major, any 2-byte alignment) as rows of 128 bytes; Trans: its transpose
+template <bool Trans>
+__device__ __forceinline__ void put_weights(unsigned char* dst, const __nv_bfloat16* __restrict__ W) {
+    for (int t = threadIdx.x; t < 64 * 64; t += blockDim.x) {
+        const int o = t >> 6, k = t & 63, r = Trans ? k : o, c = Trans ? o : k;
+        *reinterpret_cast<__nv_bfloat16*>(dst + r * 128 + (((c >> 3) ^ (r & 7)) << 4) + ((c & 7) << 1)) = W[t];
+    }
+}
+}  // namespace bf
+
+// Input layer of a node with four features, outputs 4 f .. 4 f + 3 (as k_input).
+struct InW {
+    float4 w[4];
+    float4 b;
+    __device__ __forceinline__ void load(const __nv_bfloat16* __restrict__ W, const float* __restrict__ bias, int f) {
+        float wf[4][4], bf4[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            bf4[c] = bias[4 * f + c];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) wf[c][q] = __bfloat162float(W[(4 * f + c) * 4 + q]);
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) w[c] = make_float4(wf[c][0], wf[c][1], wf[c][2], wf[c][3]);
+        b = make_float4(bf4[0], bf4[1], bf4[2], bf4[3]);
+    }
+    static __device__ __forceinline__ float one(const float4& w, float b, const float4& f) {
+        return relu(fmaf(w.w, f.w, fmaf(w.z, f.z, fmaf(w.y, f.y, fmaf(w.x, f.x, b)))));
+    }
+    __device__ __forceinline__ float4 operator()(const float4& f) const {
+        return make_float4(one(w[0], b.x, f), one(w[1], b.y, f), one(w[2], b.z, f), one(w[3], b.w, f));
+    }
+};
+
+struct Node64 {
+    const float* h;                           // nodes x 64, or with First the features (nodes x 4)
+    const __nv_bfloat16* Win; const float* bin;   // First: the input layer
+    const __nv_bfloat16* U;                   // 64 x 64
+    const float* P;                           // rows added along the edges (null: none)
+    const int32_t *ptr, *idx; const float* val;   // edges of a node; rows of instance s at P + s * rows * 64
+    int n, rows;                              // nodes and rows of an instance
+    const float* bias;                        // null: neither bias nor ReLU
+    float* out;                               // null: not stored
+    int64_t nodes;
+    const __nv_bfloat16* wx; const float* bx; float* x0;   // Heads: out . wx + bx
+    float* pool;                              // Heads: column sums, [tile][instance of the tile][64]
+    int32_t* err;
+};
+
+constexpr int kNode64Smem = bf::kW + 3 * bf::kPart + 1024;   // + alignment
+// 512 threads, two blocks an SM: 16 threads a row of 256 contiguous bytes, four
+// rows a thread.  The node's edges are a chain of three dependent loads; with
+// 256 threads (eight rows each, half the warps to overlap) a layer of 1.28M
+// nodes took 230 us.
+constexpr int kN64T = 512;
+
+template <bool First, bool Heads>
+__global__ void __launch_bounds__(kN64T, 2) k_node64(const Node64 a) {
+    extern __shared__ __align__(16) unsigned char n64_smem[];
+    unsigned char* base = n64_smem + ((1024 - (tc::smem_u32(n64_smem) & 1023)) & 1023);
+    unsigned char* Ws = base;
+    unsigned char* As = base + bf::kW;
+    __shared__ uint64_t bar;
+    __shared__ uint32_t tmem_slot;
+    __shared__ float4 cs[2][kN64T / 32][16];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    bf::put_weights<false>(Ws, a.U);
+    if (threadIdx.x == 0) {
+        tc::mbar_init(tc::smem_u32(&bar), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(tc::smem_u32(&tmem_slot)), "r"(64u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t tmem = tmem_slot;
+    const int col0 = 16 * (warp >> 2);                          // the warp's accumulator columns
+    const uint32_t tq = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)col0;
+    const int f = threadIdx.x & 15, r0 = threadIdx.x >> 4;      // the thread's piece of rows r0 + 32 i
+    const int nodes = (int)a.nodes;
+    InW in;
+    if (First) in.load(a.Win, a.bin, f);
+    const int tiles = (nodes + 127) / 128;
+    uint32_t parity = 0u;
+    bool ok = true;
+    float4 x[4];
+    int e[4], end[4];
+    int next_inst = 0;                                          // first instance of the fetched tile
+    auto fetch = [&](int tile) {
+        const int s0 = next_inst = (int)((unsigned)tile * 128u / (unsigned)a.n);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int v = tile * 128 + r0 + 32 * i;
+            const bool live = v < nodes;
+            x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (live)
+                x[i] = First ? __ldg(reinterpret_cast<const float4*>(a.h) + v)
+                             : __ldg(reinterpret_cast<const float4*>(a.h) + (int64_t)v * 16 + f);
+            if (a.P) {
+                int r = v - s0 * a.n;
+                while (r >= a.n) r -= a.n;
+                e[i] = live ? __ldg(a.ptr + r) : 0;
+                end[i] = live ? __ldg(a.ptr + r + 1) : 0;
+            }
+        }
+    };
+    if (blockIdx.x < tiles) fetch(blockIdx.x);
+    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) bf::put(As, r0 + 32 * i, f, First ? in(x[i]) : x[i]);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        tc::fence_before();
+        __syncthreads();
+        tc::fence_after();
+        if (threadIdx.x == 0) {
+            const uint32_t as = tc::smem_u32(As), ws = tc::smem_u32(Ws);
+#pragma unroll
+            for (int q = 2; q >= 0; --q)                       // the small parts first
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+                    bf::mma<bf::idesc(128, 64, false, false)>(tmem, tc::desc_sw128(as + q * bf::kPart + 32 * kk),
+                                                             tc::desc_sw128(ws + 32 * kk), (q == 2 && kk == 0) ? 0u : 1u);
+            tc::mma_commit(tc::smem_u32(&bar));
+        }
+        // the edges' rows, while the MMAs run
+        float4 y[4];
+        const int v0 = tile * 128 + r0;
+        const int s0 = next_inst;                                 // the tile's first instance
+#pragma unroll
+        for (int i = 0; i < 4; ++i) y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (a.P) {
+            int most = 0;
+            const float4* src[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                int at = s0 * a.rows;                             // the instance's first row
+                for (int r = v0 + 32 * i - s0 * a.n; r >= a.n; r -= a.n) at += a.rows;
+                most = max(most, end[i] - e[i]);
+                src[i] = reinterpret_cast<const float4*>(a.P) + (int64_t)at * 16 + f;
+            }
+            for (int k = 0; k < most; ++k) {
+                float w[4];
+                float4 p[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const bool on = e[i] + k < end[i];
+                    w[i] = on ? __ldg(a.val + e[i] + k) : 0.f;
+                    p[i] = on ? __ldg(src[i] + (int64_t)__ldg(a.idx + e[i] + k) * 16) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    y[i].x = fmaf(w[i], p[i].x, y[i].x);
+                    y[i].y = fmaf(w[i], p[i].y, y[i].y);
+                    y[i].z = fmaf(w[i], p[i].z, y[i].z);
+                    y[i].w = fmaf(w[i], p[i].w, y[i].w);
+                }
+            }
+        }
+        if (tile + (int)gridDim.x < tiles) fetch(tile + gridDim.x);
+        if (!tc::mbar_wait(tc::smem_u32(&bar), parity)) ok = false;
+        parity ^= 1u;
+        tc::fence_after();
+        {
+            // the accumulators (a lane per node) through the operands' shared memory to
+            // the staging layout: 16-byte piece c of row r at piece c ^ (r & 15)
+            uint32_t d[16];
+            tc::tmem_ld16(tq, d);
+            const int row = 32 * (warp & 3) + lane;
+            float4* D = reinterpret_cast<float4*>(As) + row * 16;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                D[(col0 / 4 + j) ^ (row & 15)] = make_float4(__uint_as_float(d[4 * j]), __uint_as_float(d[4 * j + 1]),
+                                                             __uint_as_float(d[4 * j + 2]), __uint_as_float(d[4 * j + 3]));
+        }
+        __syncthreads();
+        float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (a.bias) bias = make_float4(a.bias[4 * f], a.bias[4 * f + 1], a.bias[4 * f + 2], a.bias[4 * f + 3]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = r0 + 32 * i;
+            const float4 d = reinterpret_cast<const float4*>(As)[row * 16 + (f ^ (row & 15))];
+            float4 t = make_float4(d.x + y[i].x + bias.x, d.y + y[i].y + bias.y, d.z + y[i].z + bias.z,
+                                   d.w + y[i].w + bias.w);
+            if (a.bias) t = make_float4(relu(t.x), relu(t.y), relu(t.z), relu(t.w));
+            y[i] = t;
+            if (a.out && v0 + 32 * i < nodes && ok) reinterpret_cast<float4*>(a.out)[(int64_t)(v0 + 32 * i) * 16 + f] = t;
+        }
+        if constexpr (Heads) {
+            float wx[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) wx[c] = __bfloat162float(a.wx[4 * f + c]);
+            const float bx = a.bx[0];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float t = y[i].x * wx[0] + y[i].y * wx[1] + y[i].z * wx[2] + y[i].w * wx[3];
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+                if (f == 0 && v0 + 32 * i < nodes) a.x0[v0 + 32 * i] = t + bx;
+            }
+            // column sums of the tile's one or two instances (n >= 128): rows, then the warp's two row groups
+            const int split = (s0 + 1) * a.n;
+            const int sets = min(tile * 128 + 128, nodes) > split ? 2 : 1;
+#pragma unroll
+            for (int set = 0; set < 2; ++set) {
+                float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int v = v0 + 32 * i;
+                    if (v < nodes && (v >= split) == (set == 1)) {
+                        t.x += y[i].x;
+                        t.y += y[i].y;
+                        t.z += y[i].z;
+                        t.w += y[i].w;
+                    }
+                }
+                t.x += __shfl_xor_sync(0xffffffffu, t.x, 16);
+                t.y += __shfl_xor_sync(0xffffffffu, t.y, 16);
+                t.z += __shfl_xor_sync(0xffffffffu, t.z, 16);
+                t.w += __shfl_xor_sync(0xffffffffu, t.w, 16);
+                if (lane < 16) cs[set][warp][f] = t;
+            }
+            __syncthreads();
+            if (threadIdx.x < 128) {
+                const int set = threadIdx.x >> 6, c = threadIdx.x & 63;
+                if (set < sets) {
+                    float t = 0.f;
+#pragma unroll
+                    for (int w = 0; w < kN64T / 32; ++w) t += reinterpret_cast<const float*>(&cs[set][w][0])[c];
+                    a.pool[((int64_t)tile * 2 + set) * 64 + c] = t;
+                }
+            }
+        }
+        tc::fence_before();
+        ok = __syncthreads_and(ok) != 0;                       // shared and tensor memory free for the next tile
+        tc::fence_after();
+    }
+    if (!ok && threadIdx.x == 0) atomicExch(a.err, 1);
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(64u) : "memory");
+}
+
+// Aggregation over long rows (H = 64): a block per destination row of one instance,
+// each warp a stretch of its edges (lane l: features 2 l, 2 l + 1; eight rows in
+// flight), the warps' sums added in order.  A warp per row left 4 800 warps with
+// up to 400 dependent steps each on the constraint rows of the 200 x 400 family
+// (62 us for 164 MB).  First: the source is the input layer of the nodes' four
+// features, recomputed per edge (16 bytes instead of 256).
+template <bool First>
+__global__ void __launch_bounds__(kT) k_agg_rows(const int32_t* __restrict__ ptr, const int32_t* __restrict__ idx,
+                                                 const float* __restrict__ val, const float* __restrict__ in,
+                                                 const __nv_bfloat16* __restrict__ Win, const float* __restrict__ bin,
+                                                 float* __restrict__ out, int n_dst, int n_src, int accumulate) {
+    __shared__ float2 part[kT / 32][32];
+    const int s = blockIdx.x / n_dst, r = blockIdx.x % n_dst;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int b = ptr[r], len = ptr[r + 1] - b;
+    const int e0 = b + int((int64_t)len * warp / (kT / 32)), e1 = b + int((int64_t)len * (warp + 1) / (kT / 32));
+    float4 w0, w1;
+    float b0 = 0.f, b1 = 0.f;
+    if (First) {
+        const __nv_bfloat16* w = Win + 8 * lane;
+        w0 = make_float4(__bfloat162float(w[0]), __bfloat162float(w[1]), __bfloat162float(w[2]), __bfloat162float(w[3]));
+        w1 = make_float4(__bfloat162float(w[4]), __bfloat162float(w[5]), __bfloat162float(w[6]), __bfloat162float(w[7]));
+        b0 = bin[2 * lane];
+        b1 = bin[2 * lane + 1];
+    }
+    const float* src = in + (int64_t)s * n_src * (First ? 4 : 64);
+    float2 acc = make_float2(0.f, 0.f);
+    float an[8];                               // the next group's edges load with this group's rows
+    int jn[8];
+    auto edges = [&](int e) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const bool ok = e + u < e1;
+            an[u] = ok ? __ldg(val + e + u) : 0.f;
+            jn[u] = ok ? __ldg(idx + e + u) : 0;
+        }
+    };
+    edges(e0);
+    for (int e = e0; e < e1; e += 8) {
+        float a[8];
+        float4 ff[8];
+        float2 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            a[u] = an[u];
+            if (First) ff[u] = __ldg(reinterpret_cast<const float4*>(src) + jn[u]);
+            else v[u] = __ldg(reinterpret_cast<const float2*>(src + (int64_t)jn[u] * 64) + lane);
+        }
+        if (e + 8 < e1) edges(e + 8);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            if (First) v[u] = make_float2(InW::one(w0, b0, ff[u]), InW::one(w1, b1, ff[u]));
+            acc.x = fmaf(a[u], v[u].x, acc.x);
+            acc.y = fmaf(a[u], v[u].y, acc.y);
+        }
+    }
+    part[warp][lane] = acc;
+    __syncthreads();
+    if (warp) return;
+    float2 t = part[0][lane];
+#pragma unroll
+    for (int w = 1; w < kT / 32; ++w) {
+        t.x += part[w][lane].x;
+        t.y += part[w][lane].y;
+    }
+    float2* o = reinterpret_cast<float2*>(out + (int64_t)blockIdx.x * 64) + lane;
+    if (accumulate) {
+        const float2 p = *o;
+        t.x += p.x;
+        t.y += p.y;
+    }
+    *o = t;
+}
+
+// The pooled head from k_node64's column sums of the variables (per tile, in order) and k_colsum_part's of the constraints.
+__global__ void __launch_bounds__(1024) k_pool_finish64(const float* __restrict__ pc, int nbc,
+                                                        const float* __restrict__ pv, int m, int n, int64_t nodes,
+                                                        const __nv_bfloat16* __restrict__ wo,
+                                                        const float* __restrict__ bo, float* __restrict__ pool,
+                                                        float* __restrict__ lw) {
+    __shared__ float sub[16][64];
+    __shared__ float red[128];
+    const int s = blockIdx.x, f = threadIdx.x & 63, g = threadIdx.x >> 6;
+    const int64_t t0 = (int64_t)s * n / 128, t1 = ((int64_t)(s + 1) * n - 1) / 128;
+    float acc = 0.f;
+#pragma unroll 4
+    for (int64_t t = t0 + g; t <= t1; t += 16)                    // a tile that starts in the instance before: its second set
+        acc += pv[(t * 2 + (t * 128 < (int64_t)s * n ? 1 : 0)) * 64 + f];
+    sub[g][f] = acc;
+    __syncthreads();
+    if (threadIdx.x < 128) {
+        float t = 0.f;
+        if (threadIdx.x < 64) {
+            for (int b = 0; b < nbc; ++b) t += pc[((int64_t)s * nbc + b) * 64 + f];
+            t /= float(m);
+        } else {
+            for (int q = 0; q < 16; ++q) t += sub[q][f];
+            t /= float(n);
+        }
+        pool[s * 128 + threadIdx.x] = t;
+        red[threadIdx.x] = t * __bfloat162float(wo[threadIdx.x]);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float t = 0.f;
+        for (int q = 0; q < 128; ++q) t += red[q];
+        lw[s] = t + bo[0];
+    }
 }
 
 // ---- heads: out[v] = w . h[v] + b (warp per node) ----------------------------------
@@ -759,6 +1176,7 @@ struct sps_gnn {
     int32_t* d_err = nullptr;    // set by a tensor-core update that gave up waiting (internal error)
     float *part;              // weight-gradient block partials
     double* lpart;            // loss partials
+    float* MH = nullptr;      // H = 64: M hc of the layer being computed
     float *pcp, *pvp;         // pooling partials
     int nb_dense = 0, nb_pool_c = 0, nb_pool_v = 0, nb_loss = 0;
     int64_t part_floats = 0;
@@ -807,6 +1225,9 @@ int set_smem_attrs() {
     if (H == 64 &&
         cudaFuncSetAttribute(k_update_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmemBytes) != cudaSuccess)
         return -2;
+    if (H == 64)
+        for (auto k : {k_node64<false, false>, k_node64<false, true>, k_node64<true, false>, k_node64<true, true>})
+            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kNode64Smem) != cudaSuccess) return -2;
     if (cudaFuncSetAttribute(k_update_back<H>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)update_back_smem<H>()) != cudaSuccess)
         return -2;
@@ -840,9 +1261,98 @@ int device_error(sps_gnn* g) {
     return e ? g->fail(-2, "internal error: a tensor-core node update stopped waiting for its MMAs") : 0;
 }
 
+// Whether a graph's constraint rows are long enough for a block each.
+bool long_rows(const sps_gnn* g) { return g->nnz >= 64 * (int64_t)g->m; }
+
+// The aggregation onto the constraints (H = 64) of the variable nodes `in`, or of
+// the input layer of their features (first).
+void agg_rows64(sps_gnn* g, const float* val, const float* in, bool first, float* out, int batch, int accumulate) {
+    const __nv_bfloat16* W = g->PB + g->oWv;
+    const float* b = g->P + g->obv;
+    if (first)
+        k_agg_rows<true><<<g->m * batch, kT, 0, g->st>>>(g->cptr, g->cidx, val, in, W, b, out, g->m, g->n, accumulate);
+    else if (long_rows(g))
+        k_agg_rows<false><<<g->m * batch, kT, 0, g->st>>>(g->cptr, g->cidx, val, in, W, b, out, g->m, g->n, accumulate);
+    else
+        k_agg<64><<<grid_for((int64_t)g->m * batch * 32, kT), kT, 0, g->st>>>(g->cptr, g->cidx, val, in, out, g->m,
+                                                                             g->n, batch, accumulate);
+}
+
+template <bool First, bool Heads>
+void node64(sps_gnn* g, const Node64& a) {
+    const int64_t tiles = (a.nodes + 127) / 128;
+    k_node64<First, Heads><<<(int)std::min<int64_t>(tiles, 2 * 152), kN64T, kNode64Smem, g->st>>>(a);
+}
+
+// Forward pass, H = 64: M on the constraint side (k_node64).  keep: the variables'
+// last activations are stored too (the backward pass reads them).
+int forward64(sps_gnn* g, int batch, bool keep) {
+    const int n = g->n, m = g->m, L = g->L;
+    const int64_t NV = (int64_t)n * batch, NC = (int64_t)m * batch;
+    const __nv_bfloat16* W = g->PB;
+    const float* P = g->P;
+    cudaStream_t st = g->st;
+    // the input layer of four features is recomputed where it is read (16 bytes a node instead of 256)
+    const bool in4 = g->Fv == 4;
+    if (!in4) k_input<64><<<grid_for(NV * 64, kT), kT, 0, st>>>(g->fv, NV, g->Fv, W + g->oWv, P + g->obv, g->HV[0]);
+    k_input<64><<<grid_for(NC * 64, kT), kT, 0, st>>>(g->fc, NC, g->Fc, W + g->oWc, P + g->obc, g->HC[0]);
+    const bool heads = n >= 128;                  // a tile of 128 nodes then has at most two instances
+    for (int l = 0; l < L; ++l) {
+        const int64_t o = g->layer_off(l);
+        const int64_t oUc = o, oMc = o + 4096, obc = o + 8192;
+        const int64_t oUv = obc + 64, oMv = oUv + 4096, obv = oMv + 4096;
+        const bool first = l == 0 && in4, last = l == L - 1;
+        agg_rows64(g, g->ac_c, first ? g->fv : g->HV[l], first, g->AC[l], batch, 0);
+        dense_update<64>(g, g->HC[l], g->AC[l], W + oUc, W + oMc, P + obc, g->HC[l + 1], NC);
+        Node64 p{};
+        p.h = g->HC[l + 1];
+        p.U = W + oMv;
+        p.out = g->MH;
+        p.nodes = NC;
+        p.err = g->d_err;
+        node64<false, false>(g, p);
+        Node64 a{};
+        a.h = first ? g->fv : g->HV[l];
+        a.Win = W + g->oWv;
+        a.bin = P + g->obv;
+        a.U = W + oUv;
+        a.P = g->MH;
+        a.ptr = g->vptr;
+        a.idx = g->vidx;
+        a.val = g->av_v;
+        a.n = n;
+        a.rows = m;
+        a.bias = P + obv;
+        a.out = last && heads && !keep ? nullptr : g->HV[l + 1];
+        a.nodes = NV;
+        a.wx = W + g->oWx;
+        a.bx = P + g->obx;
+        a.x0 = g->x0;
+        a.pool = g->pvp;
+        a.err = g->d_err;
+        if (last && heads) { if (first) node64<true, true>(g, a); else node64<false, true>(g, a); }
+        else { if (first) node64<true, false>(g, a); else node64<false, false>(g, a); }
+    }
+    k_head<64><<<grid_for(NC * 32, kT), kT, 0, st>>>(g->HC[L], W + g->oWy, P + g->oby, g->y0, NC);
+    k_colsum_part<64><<<dim3(g->nb_pool_c, batch), kT, 0, st>>>(g->HC[L], m, g->pcp);
+    if (heads) {
+        k_pool_finish64<<<batch, 1024, 0, st>>>(g->pcp, g->nb_pool_c, g->pvp, m, n, NV, W + g->oWo, P + g->obo, g->pool,
+                                               g->lw);
+    } else {
+        k_head<64><<<grid_for(NV * 32, kT), kT, 0, st>>>(g->HV[L], W + g->oWx, P + g->obx, g->x0, NV);
+        k_colsum_part<64><<<dim3(g->nb_pool_v, batch), kT, 0, st>>>(g->HV[L], n, g->pvp);
+        k_pool_finish<64><<<batch, 128, 0, st>>>(g->pcp, g->nb_pool_c, g->pvp, g->nb_pool_v, m, n, W + g->oWo,
+                                                 P + g->obo, g->pool, g->lw);
+    }
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? 0 : g->fail(-2, std::string("forward: ") + cudaGetErrorString(e));
+}
+
 // Forward pass over `batch` instances whose features are already on the device.
 template <int H>
-int forward(sps_gnn* g, int batch) {
+int forward(sps_gnn* g, int batch, bool keep) {
+    if constexpr (H == 64)
+        if (!keep) return forward64(g, batch, keep);
     const int n = g->n, m = g->m, L = g->L;
     const int64_t NV = (int64_t)n * batch, NC = (int64_t)m * batch;
     const __nv_bfloat16* W = g->PB;
@@ -987,7 +1497,7 @@ void init_params(std::vector<float>& p, const sps_gnn* g) {
 
 template <int H>
 int run_loss_grad(sps_gnn* g, int batch, double* loss) {
-    if (int rc = forward<H>(g, batch)) return rc;
+    if (int rc = forward<H>(g, batch, true)) return rc;
     return backward<H>(g, batch, loss);
 }
 
@@ -1021,7 +1531,7 @@ int forward_in_place(sps_gnn* g, int batch) {
     k_lp_var_features<<<grid_for((int64_t)g->n * batch, kT), kT, 0, g->st>>>(g->vptr, g->vidx, g->kind, g->craw,
                                                                           g->cmin, g->n, g->m, batch, g->fv);
     if (cudaGetLastError() != cudaSuccess) return g->fail(-2, "feature kernels failed to launch");
-    return g->H == 64 ? forward<64>(g, batch) : forward<32>(g, batch);
+    return g->H == 64 ? forward<64>(g, batch, false) : forward<32>(g, batch, false);
 }
 
 }  // namespace gnn
@@ -1164,7 +1674,8 @@ int sps_gnn_create(const sps_gnn_graph* gr, const sps_gnn_options* opt_in, sps_g
             GNN_CK(g->alloc(&g->part, g->part_floats));
             GNN_CK(g->alloc(&g->lpart, 2 * g->nb_loss + 1));
             GNN_CK(g->alloc(&g->pcp, (int64_t)g->nb_pool_c * H * B));
-            GNN_CK(g->alloc(&g->pvp, (int64_t)g->nb_pool_v * H * B));
+            GNN_CK(g->alloc(&g->pvp, std::max<int64_t>((int64_t)g->nb_pool_v * H * B, (NV + 127) / 128 * 128)));
+            if (H == 64) GNN_CK(g->alloc(&g->MH, NC * H));
             std::vector<float> p(g->np);
             init_params(p, g);
             GNN_CK(up(g->P, p.data(), sizeof(float) * g->np));
@@ -1192,7 +1703,7 @@ int sps_gnn_predict(sps_gnn* g, int32_t batch, const float* vf, const float* cf,
     if (int rc = check_batch(g, batch, vf, cf)) return rc;
     GNN_CK(cudaSetDevice(g->opt.device));
     if (int rc = upload_inputs(g, batch, vf, cf, nullptr, nullptr, nullptr)) return rc;
-    const int rc = g->H == 64 ? forward<64>(g, batch) : forward<32>(g, batch);
+    const int rc = g->H == 64 ? forward<64>(g, batch, false) : forward<32>(g, batch, false);
     if (rc) return rc;
     const size_t nv = (size_t)g->n * batch, nc = (size_t)g->m * batch;
     if (x0) GNN_CK(cudaMemcpyAsync(x0, g->x0, sizeof(float) * nv, cudaMemcpyDeviceToHost, g->st));

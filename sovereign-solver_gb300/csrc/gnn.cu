@@ -4,12 +4,12 @@
 // Activations are kept per instance and node, row-major with the hidden width
 // innermost ([instance][node][H], FP32), so every per-node kernel runs over the
 // flattened node list of the whole batch and the weight gradients are sums
-// over it.  Aggregations are CSR SpMMs (warp per destination row, float2 per
-// lane); the dense node update is a register-tiled FP32 contraction of
-// 128-node tiles with both weight matrices staged in shared memory (BF16
-// weights widened to FP32), its backward a 32-node-tile kernel.  Every
+// over it.  With H = 64 the variable side's dense updates, forward and backward, run
+// on the tensor cores (k_node64, k_back64: tcgen05, FP32 as three BF16 parts) and
+// the constraint side's M products are made there (k_con_update, k_agg_rows);
+// H = 32 keeps register-tiled FP32 contractions and CSR SpMM aggregations.  Every
 // reduction (weight gradients, losses, pooling) writes per-block partials that
-// a second kernel sums in block order: training is bitwise reproducible.
+// are summed in block order: training is bitwise reproducible.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -186,39 +186,10 @@ __global__ void __launch_bounds__(kT, 2) k_update(const float* __restrict__ h, c
     }
 }
 
-// ---- dense node update on the tensor cores (H = 64) -------------------------------
-// The same update as k_update, out = relu([h | a] W^T + b) with W = [U | M]
-// (64 x 128), as tcgen05 MMAs: M = 128 nodes per tile (one TMEM lane each), N =
-// 64 outputs (64 TMEM columns of FP32 accumulators), K = 128 in four 32-float
-// chunks of 128-byte rows (K-major, 128-byte swizzle: 16-byte piece q of row r
-// sits at piece q ^ (r & 7) of the row; 8-row groups 1024 bytes apart), eight
-// K = 8 steps per chunk.  The activations are split as x = big + small, both
-// TF32 (round to nearest), and both parts are multiplied (the BF16 weights are
-// exact in TF32): the products are exact and the sum is accumulated in FP32,
-// so the result agrees with the FP32 update to FP32 rounding, not TF32's.
-// All 256 threads stage a chunk (global -> split -> swizzled shared memory,
-// two buffers); thread 0 issues the chunk's MMAs and commits them to the
-// buffer's mbarrier, which the stagers wait on before they overwrite it; the
-// eight warps read the accumulators back (tcgen05.ld, warp w: lanes of quarter
-// w % 4, columns 32 (w / 4) ..) for the bias and ReLU.  Every wait is bounded;
-// a block that gives up sets *err, stops, and still frees its TMEM.
+// ---- tensor-core helpers ---------------------------------------------------------------
 namespace tc {
-constexpr int kRows = 128;                    // nodes per tile: the MMA's M and the TMEM lanes
-constexpr int kABytes = kRows * 128;          // one 32-float chunk of the activations (16 KB)
-constexpr int kBBytes = 64 * 128;             // one 32-float chunk of the weights (8 KB)
-constexpr uint32_t kTmemCols = 64;
-constexpr int kSmemBytes = 4 * kBBytes + 4 * kABytes + 64 + 1024;   // + barriers, TMEM slot, alignment
 constexpr int kWaitPolls = 1 << 20;
-// instruction descriptor: D F32, A and B TF32, both K-major, N = 64, M = 128
-constexpr uint32_t kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
-
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ float tf32_rna(float x) {
-    uint32_t u;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(x));
-    return __uint_as_float(u);
-}
 
 // K-major operand, 128-byte swizzle, 8-row groups 1024 bytes apart
 __device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {
@@ -244,28 +215,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-__device__ __forceinline__ void mma_tf32(uint32_t d, uint64_t a, uint64_t b, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(d), "l"(a), "l"(b), "r"(kIdesc), "r"(accumulate) : "memory");
-}
-
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                   "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-                   "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
-                   "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-                   "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                 : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
                  "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
@@ -275,122 +228,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 }  // namespace tc
-
-__global__ void __launch_bounds__(kT, 2) k_update_tc(const float* __restrict__ h, const float* __restrict__ a,
-                                                     const __nv_bfloat16* __restrict__ U,
-                                                     const __nv_bfloat16* __restrict__ M,
-                                                     const float* __restrict__ bias, float* __restrict__ out,
-                                                     int64_t nodes, int32_t* __restrict__ err) {
-    constexpr int H = 64;
-    extern __shared__ __align__(16) unsigned char tc_smem[];
-    unsigned char* base = tc_smem + ((1024 - (tc::smem_u32(tc_smem) & 1023)) & 1023);
-    unsigned char* Bs = base;                              // 4 chunks of W, 64 rows of 128 bytes
-    unsigned char* As = base + 4 * tc::kBBytes;            // buffer b: big at As + 2 b kABytes, small after it
-    uint64_t* bars = reinterpret_cast<uint64_t*>(As + 4 * tc::kABytes);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-
-    // the weights, K-major: row o of chunk c holds W[o][32 c .. 32 c + 31]
-    for (int t = threadIdx.x; t < 4 * H * 8; t += kT) {
-        const int c = t / (H * 8), o = (t / 8) % H, q = t % 8;
-        float w[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int k = 32 * c + 4 * q + e;
-            w[e] = __bfloat162float(k < H ? U[o * H + k] : M[o * H + (k - H)]);
-        }
-        *reinterpret_cast<float4*>(Bs + c * tc::kBBytes + o * 128 + ((q ^ (o & 7)) << 4)) =
-            make_float4(w[0], w[1], w[2], w[3]);
-    }
-    if (threadIdx.x == 0) {
-        tc::mbar_init(tc::smem_u32(&bars[0]), 1);
-        tc::mbar_init(tc::smem_u32(&bars[1]), 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(tc::smem_u32(tmem_slot)), "r"(tc::kTmemCols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // W, written by threads, read by the MMA
-    tc::fence_before();
-    __syncthreads();
-    tc::fence_after();
-    const uint32_t tmem = *tmem_slot;
-    const int col0 = 32 * (warp >> 2);                     // this warp's accumulator columns
-    const uint32_t tq = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)col0;
-    uint32_t parity[2] = {0u, 0u};
-    bool ok = true;
-    const int64_t tiles = (nodes + tc::kRows - 1) / tc::kRows;
-    for (int64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        const int64_t base_node = tile * tc::kRows;
-        for (int c = 0; c < 4; ++c) {
-            const int buf = c & 1;
-            if (c >= 2) {                                  // the MMAs that read this buffer (chunk c - 2)
-                if (!tc::mbar_wait(tc::smem_u32(&bars[buf]), parity[buf])) ok = false;
-                parity[buf] ^= 1u;
-            }
-            unsigned char* big = As + 2 * buf * tc::kABytes;
-            unsigned char* small = big + tc::kABytes;
-            const float* src = c < 2 ? h + 32 * c : a + 32 * (c - 2);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int pc = threadIdx.x + kT * i, row = pc >> 3, q = pc & 7;
-                const int64_t v = base_node + row;
-                float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (v < nodes) x = __ldg(reinterpret_cast<const float4*>(src + v * H + 4 * q));
-                const float4 hi = make_float4(tc::tf32_rna(x.x), tc::tf32_rna(x.y), tc::tf32_rna(x.z), tc::tf32_rna(x.w));
-                const float4 lo = make_float4(tc::tf32_rna(x.x - hi.x), tc::tf32_rna(x.y - hi.y),
-                                              tc::tf32_rna(x.z - hi.z), tc::tf32_rna(x.w - hi.w));
-                const int off = row * 128 + ((q ^ (row & 7)) << 4);
-                *reinterpret_cast<float4*>(big + off) = hi;
-                *reinterpret_cast<float4*>(small + off) = lo;
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            tc::fence_before();
-            __syncthreads();
-            tc::fence_after();
-            if (threadIdx.x == 0) {
-                const uint32_t ab = tc::smem_u32(big), as = tc::smem_u32(small);
-                const uint32_t bb = tc::smem_u32(Bs + c * tc::kBBytes);
-#pragma unroll
-                for (int kk = 0; kk < 4; ++kk) {
-                    const uint64_t bd = tc::desc_sw128(bb + 32 * kk);
-                    tc::mma_tf32(tmem, tc::desc_sw128(ab + 32 * kk), bd, (c | kk) != 0 ? 1u : 0u);
-                    tc::mma_tf32(tmem, tc::desc_sw128(as + 32 * kk), bd, 1u);
-                }
-                tc::mma_commit(tc::smem_u32(&bars[buf]));
-            }
-        }
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {                      // chunks 2 and 3: the tile's last MMAs
-            if (!tc::mbar_wait(tc::smem_u32(&bars[b]), parity[b])) ok = false;
-            parity[b] ^= 1u;
-        }
-        tc::fence_after();
-        uint32_t r[32];
-        tc::tmem_ld32(tq, r);
-        const int64_t v = base_node + 32 * (warp & 3) + lane;
-        if (v < nodes && ok) {
-            float* o = out + v * H + col0;
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-                const float4 y = make_float4(relu(__uint_as_float(r[j]) + bias[col0 + j]),
-                                             relu(__uint_as_float(r[j + 1]) + bias[col0 + j + 1]),
-                                             relu(__uint_as_float(r[j + 2]) + bias[col0 + j + 2]),
-                                             relu(__uint_as_float(r[j + 3]) + bias[col0 + j + 3]));
-                *reinterpret_cast<float4*>(o + j) = y;
-            }
-        }
-        tc::fence_before();
-        ok = __syncthreads_and(ok) != 0;                    // TMEM read before the next tile's MMAs
-        tc::fence_after();
-    }
-    if (!ok && threadIdx.x == 0) atomicExch(err, 1);
-    __syncthreads();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tc::kTmemCols) : "memory");
-}
 
 // ---- the variable side's node update on the tensor cores (H = 64) --------------------
 // relu(U h + M a + b) with a_j = sum_i a_ij hc_i is relu(U h + sum_i a_ij (M hc_i) + b):
@@ -691,11 +528,416 @@ __global__ void __launch_bounds__(kN64T, 2) k_node64(const Node64 a) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(64u) : "memory");
 }
 
+// ---- backward of a 64 x 64 node map on the tensor cores -------------------------------
+// z = dout where the map's output is positive; dh = z W, and this block's share of
+// dW = sum_v z_v h_v^T and db = sum_v z_v.  dout is read, or formed from the heads'
+// gradients; rows of the constraint side's gradient are added along the edges.
+// (With M on the constraint side, da and the M gradient need only sum_j a_ij z_j:
+// z is stored for that aggregation, half of what da and its scatter moved.)
+// On CUDA cores, one shared-memory word per FMA, this took 1453 us for 640k nodes
+// of K = 128; now 200-260 us (the stream, five arrays of 164 MB, takes 120 us at
+// the measured HBM rate; each tile's chain of loads, MMAs and read-backs with two
+// blocks an SM is what is left).
+//
+// FP32 as three BF16 parts.  Both products read the same shared-memory image of a
+// 128-node tile, rows of 128 bytes with the 128-byte swizzle: as the K-major A of
+// dh (M = nodes, K = 64 features, 16 per step), and as MN-major operands of dW
+// (K = nodes, 16 per step): A = [z1; z2] (M = 128: two parts one above the other), B =
+// [h1 | h2 | h3] (N = 192), and A = [z2; z3], B = h1 for z3 h1, whose accumulators take the
+// place of dh's once that is read.  z2 h2 and smaller products are below FP32.
+// The tensor core adds FP32 accumulators without rounding to nearest, so dW is
+// moved to registers and added there after every tile.
+namespace bk {
+constexpr int kThreads = 512;
+constexpr int kSmem = bf::kW + 6 * bf::kPart + 1024;
+constexpr uint32_t kTmem = 256;               // columns: dW parts 0..191, dh then z3 h1 192..255
+constexpr int kOut = 64 * 64 + 64;            // a block's partial: dW, db
+constexpr int kHeadOut = 65;                  // dw, db of a head
+// MN-major operand, 128-byte swizzle: 64-element blocks `block` bytes apart, 8-row groups 1024
+__device__ __forceinline__ uint64_t desc_mn(uint32_t addr, uint32_t block) {
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(block >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+           ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+}  // namespace bk
+
+struct Back64 {
+    const float* dout;                        // nodes x 64 (null: from the head)
+    const float* dhead; const __nv_bfloat16* whead;       // head: dhead[v] whead + dlw[instance] wpool / n
+    const float* dlw; const __nv_bfloat16* wpool;
+    const float* Q; const int32_t *ptr, *idx; const float* val; int rows;   // rows added along the edges (null: none)
+    const float* out;                         // the map's output (null: no mask)
+    const float* h;                           // the map's input, or with First the features (nodes x 4)
+    const __nv_bfloat16* Win; const float* bin;
+    const __nv_bfloat16* W;                   // 64 x 64
+    float* z;                                 // null: not stored
+    float* dh; int accumulate;                // dh += instead of =
+    float* part;                              // kOut per block
+    float* hpart;                             // kHeadOut per block (head only)
+    int n;                                    // nodes of an instance
+    int64_t nodes;
+    int32_t* err;
+};
+
+template <bool First>
+__global__ void __launch_bounds__(bk::kThreads, 2) k_back64(const Back64 a) {
+    extern __shared__ __align__(16) unsigned char bk_smem[];
+    unsigned char* base = bk_smem + ((1024 - (tc::smem_u32(bk_smem) & 1023)) & 1023);
+    unsigned char* Ws = base;
+    unsigned char* Zs = base + bf::kW;
+    unsigned char* Hs = Zs + 3 * bf::kPart;
+    __shared__ uint64_t bars[3];
+    __shared__ uint32_t tmem_slot;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    bf::put_weights<true>(Ws, a.W);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) tc::mbar_init(tc::smem_u32(&bars[q]), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(tc::smem_u32(&tmem_slot)), "r"(bk::kTmem) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t tmem = tmem_slot;
+    const int c0 = 16 * (warp >> 2);                            // the warp's columns of each 64
+    const uint32_t tq = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)c0;
+    const int trow = 32 * (warp & 3) + lane;
+    const int f = threadIdx.x & 15, r0 = threadIdx.x >> 4;
+    const int nodes = (int)a.nodes, tiles = (nodes + 127) / 128;
+    float acc[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) acc[j] = 0.f;
+    float4 zsum = make_float4(0.f, 0.f, 0.f, 0.f), hw = zsum;
+    float hb = 0.f;
+    uint32_t parity = 0u;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+        const int v0 = tile * 128 + r0;
+        // z
+        float4 z[4];
+        if (a.dout) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                z[i] = v0 + 32 * i < nodes ? __ldg(reinterpret_cast<const float4*>(a.dout) + (int64_t)(v0 + 32 * i) * 16 + f)
+                                           : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if (a.Q || !a.dout) {
+            const int s0 = (int)((unsigned)tile * 128u / (unsigned)a.n);
+            if (a.Q) {
+                int e[4], end[4], most = 0;
+                const float4* src[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const bool live = v0 + 32 * i < nodes;
+                    int at = s0 * a.rows, r = v0 + 32 * i - s0 * a.n;
+                    while (r >= a.n) { r -= a.n; at += a.rows; }
+                    e[i] = live ? __ldg(a.ptr + r) : 0;
+                    end[i] = live ? __ldg(a.ptr + r + 1) : 0;
+                    most = max(most, end[i] - e[i]);
+                    src[i] = reinterpret_cast<const float4*>(a.Q) + (int64_t)at * 16 + f;
+                }
+                for (int k = 0; k < most; ++k) {
+                    float w[4];
+                    float4 p[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const bool on = e[i] + k < end[i];
+                        w[i] = on ? __ldg(a.val + e[i] + k) : 0.f;
+                        p[i] = on ? __ldg(src[i] + (int64_t)__ldg(a.idx + e[i] + k) * 16) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        z[i].x = fmaf(w[i], p[i].x, z[i].x);
+                        z[i].y = fmaf(w[i], p[i].y, z[i].y);
+                        z[i].z = fmaf(w[i], p[i].z, z[i].z);
+                        z[i].w = fmaf(w[i], p[i].w, z[i].w);
+                    }
+                }
+            } else {
+                const float inv = 1.f / float(a.n);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const bool live = v0 + 32 * i < nodes;
+                    int s = s0;
+                    for (int r = v0 + 32 * i - s0 * a.n; r >= a.n; r -= a.n) ++s;
+                    const float d = live ? __ldg(a.dhead + v0 + 32 * i) : 0.f, g = live ? __ldg(a.dlw + s) * inv : 0.f;
+                    const __nv_bfloat16 *w = a.whead + 4 * f, *q = a.wpool + 4 * f;
+                    z[i] = make_float4(fmaf(d, __bfloat162float(w[0]), g * __bfloat162float(q[0])),
+                                       fmaf(d, __bfloat162float(w[1]), g * __bfloat162float(q[1])),
+                                       fmaf(d, __bfloat162float(w[2]), g * __bfloat162float(q[2])),
+                                       fmaf(d, __bfloat162float(w[3]), g * __bfloat162float(q[3])));
+                }
+            }
+        }
+        if (a.out) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int v = v0 + 32 * i;
+                float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (v < nodes) o = __ldg(reinterpret_cast<const float4*>(a.out) + (int64_t)v * 16 + f);
+                if (a.hpart && v < nodes) {
+                    const float d = __ldg(a.dhead + v);
+                    hw.x = fmaf(d, o.x, hw.x);
+                    hw.y = fmaf(d, o.y, hw.y);
+                    hw.z = fmaf(d, o.z, hw.z);
+                    hw.w = fmaf(d, o.w, hw.w);
+                    hb += d;
+                }
+                z[i] = make_float4(o.x > 0.f ? z[i].x : 0.f, o.y > 0.f ? z[i].y : 0.f, o.z > 0.f ? z[i].z : 0.f,
+                                   o.w > 0.f ? z[i].w : 0.f);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int v = v0 + 32 * i;
+            if (a.z && v < nodes) reinterpret_cast<float4*>(a.z)[(int64_t)v * 16 + f] = z[i];
+            zsum.x += z[i].x;
+            zsum.y += z[i].y;
+            zsum.z += z[i].z;
+            zsum.w += z[i].w;
+            bf::put(Zs, r0 + 32 * i, f, z[i]);
+        }
+        // h
+        if constexpr (First) {
+            InW in;
+            in.load(a.Win, a.bin, f);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int v = v0 + 32 * i;
+                bf::put(Hs, r0 + 32 * i, f, v < nodes ? in(__ldg(reinterpret_cast<const float4*>(a.h) + v))
+                                                     : make_float4(0.f, 0.f, 0.f, 0.f));
+            }
+        } else {
+            float4 x[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                x[i] = v0 + 32 * i < nodes ? __ldg(reinterpret_cast<const float4*>(a.h) + (int64_t)(v0 + 32 * i) * 16 + f)
+                                           : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) bf::put(Hs, r0 + 32 * i, f, x[i]);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        tc::fence_before();
+        __syncthreads();
+        tc::fence_after();
+        const uint32_t zs = tc::smem_u32(Zs), hs = tc::smem_u32(Hs), ws = tc::smem_u32(Ws);
+        if (threadIdx.x == 0) {
+#pragma unroll
+            for (int q = 2; q >= 0; --q)
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+                    bf::mma<bf::idesc(128, 64, false, false)>(tmem + 192, tc::desc_sw128(zs + q * bf::kPart + 32 * kk),
+                                                             tc::desc_sw128(ws + 32 * kk), (q == 2 && kk == 0) ? 0u : 1u);
+            tc::mma_commit(tc::smem_u32(&bars[0]));
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)
+                bf::mma<bf::idesc(128, 192, true, true)>(tmem, bk::desc_mn(zs + 2048 * kk, bf::kPart),
+                                                        bk::desc_mn(hs + 2048 * kk, bf::kPart), kk ? 1u : 0u);
+            tc::mma_commit(tc::smem_u32(&bars[1]));
+        }
+        if (!tc::mbar_wait(tc::smem_u32(&bars[0]), parity)) ok = false;
+        tc::fence_after();
+        uint32_t dh[16];
+        tc::tmem_ld16(tq + 192, dh);
+        tc::fence_before();
+        ok = __syncthreads_and(ok) != 0;                        // dh read: its columns take z3 h1
+        tc::fence_after();
+        if (threadIdx.x == 0 && ok) {
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)
+                bf::mma<bf::idesc(128, 64, true, true)>(tmem + 192, bk::desc_mn(zs + bf::kPart + 2048 * kk, bf::kPart),
+                                                       bk::desc_mn(hs + 2048 * kk, bf::kPart), kk ? 1u : 0u);
+            tc::mma_commit(tc::smem_u32(&bars[2]));
+        }
+        if (!ok) break;
+        if (!tc::mbar_wait(tc::smem_u32(&bars[1]), parity)) ok = false;
+        tc::fence_after();
+        uint32_t q[16];
+#pragma unroll
+        for (int p = 2; p >= 0; --p) {                          // z1 h3 + z2 h3 (rows apart), ... h2, ... h1
+            tc::tmem_ld16(tq + 64 * p, q);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) acc[j] += __uint_as_float(q[j]);
+        }
+        if (!tc::mbar_wait(tc::smem_u32(&bars[2]), parity)) ok = false;
+        parity ^= 1u;
+        tc::fence_after();
+        tc::tmem_ld16(tq + 192, q);
+        if (trow >= 64)
+#pragma unroll
+            for (int j = 0; j < 16; ++j) acc[j] += __uint_as_float(q[j]);
+        // dh through shared memory to the staging layout (the operands are done with)
+        float4* D = reinterpret_cast<float4*>(Zs) + trow * 16;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            D[(c0 / 4 + j) ^ (trow & 15)] = make_float4(__uint_as_float(dh[4 * j]), __uint_as_float(dh[4 * j + 1]),
+                                                        __uint_as_float(dh[4 * j + 2]), __uint_as_float(dh[4 * j + 3]));
+        tc::fence_before();
+        ok = __syncthreads_and(ok) != 0;
+        tc::fence_after();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = r0 + 32 * i, v = v0 + 32 * i;
+            float4 d = reinterpret_cast<const float4*>(Zs)[row * 16 + (f ^ (row & 15))];
+            if (v >= nodes || !ok) continue;
+            float4* o = reinterpret_cast<float4*>(a.dh) + (int64_t)v * 16 + f;
+            if (a.accumulate) {
+                const float4 p = *o;
+                d = make_float4(d.x + p.x, d.y + p.y, d.z + p.z, d.w + p.w);
+            }
+            *o = d;
+        }
+        __syncthreads();                                        // Zs read before the next tile's staging
+    }
+    if (!ok && threadIdx.x == 0) atomicExch(a.err, 1);
+    // the block's partials: rows r and r + 64 of dW, then the sums over the row groups, in order
+    __syncthreads();
+    float* S = reinterpret_cast<float*>(Zs);
+    float* P = a.part + (int64_t)blockIdx.x * bk::kOut;
+    if (trow >= 64)
+#pragma unroll
+        for (int j = 0; j < 16; ++j) S[(trow - 64) * 65 + c0 + j] = acc[j];
+    __syncthreads();
+    if (trow < 64)
+#pragma unroll
+        for (int j = 0; j < 16; ++j) P[trow * 64 + c0 + j] = acc[j] + S[trow * 65 + c0 + j];
+    __syncthreads();
+    float* R = S;                                               // [32 row groups][64]
+    reinterpret_cast<float4*>(R)[r0 * 16 + f] = zsum;
+    __syncthreads();
+    if (threadIdx.x < 64) {
+        float t = 0.f;
+        for (int g = 0; g < 32; ++g) t += R[g * 64 + threadIdx.x];
+        P[4096 + threadIdx.x] = t;
+    }
+    if (a.hpart) {
+        __syncthreads();
+        reinterpret_cast<float4*>(R)[r0 * 16 + f] = hw;
+        if (f == 0) R[2048 + r0] = hb;
+        __syncthreads();
+        float* Hp = a.hpart + (int64_t)blockIdx.x * bk::kHeadOut;
+        if (threadIdx.x < 64) {
+            float t = 0.f;
+            for (int g = 0; g < 32; ++g) t += R[g * 64 + threadIdx.x];
+            Hp[threadIdx.x] = t;
+        } else if (threadIdx.x == 64) {
+            float t = 0.f;
+            for (int g = 0; g < 32; ++g) t += R[2048 + g];
+            Hp[64] = t;
+        }
+    }
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(bk::kTmem) : "memory");
+}
+
+// Input layer backward for four features (H = 64): z = (dout + rows along the edges)
+// where the recomputed layer is positive; partials of dW (64 x 4) and db.
+constexpr int kInOut = 64 * 4 + 64;
+__global__ void __launch_bounds__(bk::kThreads, 2) k_in_back64(const Back64 a) {
+    const int f = threadIdx.x & 15, r0 = threadIdx.x >> 4;
+    const int nodes = (int)a.nodes;
+    InW in;
+    in.load(a.Win, a.bin, f);
+    float g[4][4], gb[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        gb[c] = 0.f;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) g[c][q] = 0.f;
+    }
+    for (int v = blockIdx.x * 32 + r0; v < nodes; v += gridDim.x * 32) {
+        float4 z = __ldg(reinterpret_cast<const float4*>(a.dout) + (int64_t)v * 16 + f);
+        const float4 x = __ldg(reinterpret_cast<const float4*>(a.h) + v);
+        if (a.Q) {
+            const int s = (int)((unsigned)v / (unsigned)a.n), r = v - s * a.n;
+            const float4* src = reinterpret_cast<const float4*>(a.Q) + (int64_t)s * a.rows * 16 + f;
+            for (int e = __ldg(a.ptr + r), end = __ldg(a.ptr + r + 1); e < end; ++e) {
+                const float w = __ldg(a.val + e);
+                const float4 p = __ldg(src + (int64_t)__ldg(a.idx + e) * 16);
+                z = make_float4(fmaf(w, p.x, z.x), fmaf(w, p.y, z.y), fmaf(w, p.z, z.z), fmaf(w, p.w, z.w));
+            }
+        }
+        const float4 o = in(x);
+        const float zz[4] = {o.x > 0.f ? z.x : 0.f, o.y > 0.f ? z.y : 0.f, o.z > 0.f ? z.z : 0.f, o.w > 0.f ? z.w : 0.f};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            g[c][0] = fmaf(zz[c], x.x, g[c][0]);
+            g[c][1] = fmaf(zz[c], x.y, g[c][1]);
+            g[c][2] = fmaf(zz[c], x.z, g[c][2]);
+            g[c][3] = fmaf(zz[c], x.w, g[c][3]);
+            gb[c] += zz[c];
+        }
+    }
+    // sums over the 32 row groups in order: [group][output][4 features, bias]
+    __shared__ float R[32][64 * 5 / 2];                          // two halves of the outputs, one after the other
+    float* P = a.part + (int64_t)blockIdx.x * kInOut;
+    for (int half = 0; half < 2; ++half) {
+        __syncthreads();
+        if (f / 8 == half)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                float* d = &R[r0][((f & 7) * 4 + c) * 5];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) d[q] = g[c][q];
+                d[4] = gb[c];
+            }
+        __syncthreads();
+        for (int t = threadIdx.x; t < 160; t += bk::kThreads) {
+            float sum = 0.f;
+            for (int q = 0; q < 32; ++q) sum += R[q][t];
+            const int o = 32 * half + t / 5, k = t % 5;
+            if (k < 4) P[o * 4 + k] = sum;
+            else P[256 + o] = sum;
+        }
+    }
+}
+
+// grad[p] += the sum over a job's blocks, in order, for every job (one launch for
+// all weight gradients; eight loads in flight where one per block was 62 us each).
+struct SumJob {
+    const float* part;
+    float* grad;
+    int32_t blocks, stride, width;
+};
+constexpr int kMaxJobs = 80;                  // 8 layers x 7 + inputs and heads
+struct SumJobs {
+    SumJob job[kMaxJobs];
+};
+__global__ void __launch_bounds__(kT) k_sum_jobs(const __grid_constant__ SumJobs J) {
+    const SumJob j = J.job[blockIdx.y];
+    for (int p = blockIdx.x * kT + threadIdx.x; p < j.width; p += gridDim.x * kT) {
+        float s = 0.f;
+        for (int b = 0; b < j.blocks; b += 8) {
+            float v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = b + u < j.blocks ? __ldg(j.part + (int64_t)(b + u) * j.stride + p) : 0.f;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s += v[u];
+        }
+        j.grad[p] += s;
+    }
+}
+
+// hi + lo += p with the sum's rounding kept in lo (Knuth's two-sum): long sums are
+// made of short ones (eight products) added this way.
+__device__ __forceinline__ void add2(float p, float& hi, float& lo) {
+    const float t = __fadd_rn(hi, p), b = __fsub_rn(t, hi);
+    lo += __fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(p, b));
+    hi = t;
+}
+
 // Aggregation over long rows (H = 64): a block per destination row of one instance,
 // each warp a stretch of its edges (lane l: features 2 l, 2 l + 1; eight rows in
 // flight), the warps' sums added in order.  A warp per row left 4 800 warps with
 // up to 400 dependent steps each on the constraint rows of the 200 x 400 family
-// (62 us for 164 MB).  First: the source is the input layer of the nodes' four
+// (62 us for 164 MB; now 39).  Sums of hundreds of terms, compensated.  First: the
+// source is the input layer of the nodes' four
 // features, recomputed per edge (16 bytes instead of 256).
 template <bool First>
 __global__ void __launch_bounds__(kT) k_agg_rows(const int32_t* __restrict__ ptr, const int32_t* __restrict__ idx,
@@ -717,7 +959,7 @@ __global__ void __launch_bounds__(kT) k_agg_rows(const int32_t* __restrict__ ptr
         b1 = bin[2 * lane + 1];
     }
     const float* src = in + (int64_t)s * n_src * (First ? 4 : 64);
-    float2 acc = make_float2(0.f, 0.f);
+    float2 acc = make_float2(0.f, 0.f), low = acc;
     float an[8];                               // the next group's edges load with this group's rows
     int jn[8];
     auto edges = [&](int e) {
@@ -740,13 +982,18 @@ __global__ void __launch_bounds__(kT) k_agg_rows(const int32_t* __restrict__ ptr
             else v[u] = __ldg(reinterpret_cast<const float2*>(src + (int64_t)jn[u] * 64) + lane);
         }
         if (e + 8 < e1) edges(e + 8);
+        float2 t = make_float2(0.f, 0.f);
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             if (First) v[u] = make_float2(InW::one(w0, b0, ff[u]), InW::one(w1, b1, ff[u]));
-            acc.x = fmaf(a[u], v[u].x, acc.x);
-            acc.y = fmaf(a[u], v[u].y, acc.y);
+            t.x = fmaf(a[u], v[u].x, t.x);
+            t.y = fmaf(a[u], v[u].y, t.y);
         }
+        add2(t.x, acc.x, low.x);
+        add2(t.y, acc.y, low.y);
     }
+    acc.x += low.x;
+    acc.y += low.y;
     part[warp][lane] = acc;
     __syncthreads();
     if (warp) return;
@@ -763,6 +1010,56 @@ __global__ void __launch_bounds__(kT) k_agg_rows(const int32_t* __restrict__ ptr
         t.y += p.y;
     }
     *o = t;
+}
+
+// The constraint nodes' update (H = 64): relu(U h + M a + b) in compensated FP32, 16
+// nodes a block, a thread one output of four.  There are few constraint nodes
+// and each stands for hundreds of variables: a ReLU that takes the other side of
+// zero than exact arithmetic changes the gradient by parts in 10^5, so this sum and
+// the aggregation's are made more exactly than the tensor cores' FP32 sums (the
+// gradient's error against FP64 on the 200 x 400 family: 2.4e-6 before).
+constexpr int kConNodes = 16;
+__global__ void __launch_bounds__(kT) k_con_update(const float* __restrict__ h, const float* __restrict__ a,
+                                                   const __nv_bfloat16* __restrict__ U,
+                                                   const __nv_bfloat16* __restrict__ M,
+                                                   const float* __restrict__ bias, float* __restrict__ out,
+                                                   int64_t nodes) {
+    __shared__ float Wt[128 * 64];             // [k][o]
+    __shared__ float4 X[kConNodes][32];
+    for (int t = threadIdx.x; t < 128 * 64; t += kT) {
+        const int o = t & 63, k = t >> 6;
+        Wt[t] = __bfloat162float(k < 64 ? U[o * 64 + k] : M[o * 64 + k - 64]);
+    }
+    const int64_t v0 = (int64_t)blockIdx.x * kConNodes;
+    for (int t = threadIdx.x; t < kConNodes * 32; t += kT) {
+        const int nd = t >> 5, q = t & 31;
+        const int64_t v = v0 + nd;
+        X[nd][q] = v >= nodes ? make_float4(0.f, 0.f, 0.f, 0.f)
+                   : q < 16 ? reinterpret_cast<const float4*>(h)[v * 16 + q] : reinterpret_cast<const float4*>(a)[v * 16 + q - 16];
+    }
+    __syncthreads();
+    const int o = threadIdx.x & 63, g = threadIdx.x >> 6;
+    float hi[4], lo[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        hi[i] = bias[o];
+        lo[i] = 0.f;
+    }
+    for (int q = 0; q < 32; q += 2) {
+        float w[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) w[c] = Wt[(4 * q + c) * 64 + o];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 x = X[g + 4 * i][q], y = X[g + 4 * i][q + 1];
+            const float t = fmaf(w[3], x.w, fmaf(w[2], x.z, fmaf(w[1], x.y, w[0] * x.x)));
+            const float u = fmaf(w[7], y.w, fmaf(w[6], y.z, fmaf(w[5], y.y, w[4] * y.x)));
+            add2(t + u, hi[i], lo[i]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (v0 + g + 4 * i < nodes) out[(v0 + g + 4 * i) * 64 + o] = relu(hi[i] + lo[i]);
 }
 
 // The pooled head from k_node64's column sums of the variables (per tile, in order) and k_colsum_part's of the constraints.
@@ -1173,10 +1470,10 @@ struct sps_gnn {
     std::vector<float*> HV, HC, AV, AC;
     float *dHV, *dHC, *dHV2, *dHC2, *dA;
     float *x0, *y0, *lw, *pool, *dx0, *dy0, *dlw;
-    int32_t* d_err = nullptr;    // set by a tensor-core update that gave up waiting (internal error)
+    int32_t* d_err = nullptr;    // set by a tensor-core kernel that gave up waiting (internal error)
     float *part;              // weight-gradient block partials
     double* lpart;            // loss partials
-    float* MH = nullptr;      // H = 64: M hc of the layer being computed
+    float *MH = nullptr, *AG = nullptr;   // H = 64: M hc of the layer being computed; sum_j a_ij z_j
     float *pcp, *pvp;         // pooling partials
     int nb_dense = 0, nb_pool_c = 0, nb_pool_v = 0, nb_loss = 0;
     int64_t part_floats = 0;
@@ -1219,35 +1516,25 @@ size_t update_back_smem() { return sizeof(float) * (2 * H * H + 3 * kTile * (H +
 
 template <int H>
 int set_smem_attrs() {
-    if (cudaFuncSetAttribute(k_update<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)update_smem<H>()) !=
-        cudaSuccess)
-        return -2;
-    if (H == 64 &&
-        cudaFuncSetAttribute(k_update_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmemBytes) != cudaSuccess)
-        return -2;
-    if (H == 64)
+    if constexpr (H == 64) {
         for (auto k : {k_node64<false, false>, k_node64<false, true>, k_node64<true, false>, k_node64<true, true>})
             if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kNode64Smem) != cudaSuccess) return -2;
-    if (cudaFuncSetAttribute(k_update_back<H>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)update_back_smem<H>()) != cudaSuccess)
-        return -2;
-    return 0;
+        for (auto k : {k_back64<false>, k_back64<true>})
+            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bk::kSmem) != cudaSuccess) return -2;
+        return 0;
+    } else {
+        if (cudaFuncSetAttribute(k_update<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)update_smem<H>()) !=
+                cudaSuccess ||
+            cudaFuncSetAttribute(k_update_back<H>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)update_back_smem<H>()) != cudaSuccess)
+            return -2;
+        return 0;
+    }
 }
 
 int grid_for(int64_t work, int per_block) {
     const int64_t b = (work + per_block - 1) / per_block;
     return (int)std::max<int64_t>(1, std::min<int64_t>(b, 152 * 8));
-}
-
-// The dense node update: on the tensor cores for H = 64, the register-tiled
-// FP32 kernel for H = 32.
-template <int H>
-void dense_update(sps_gnn* g, const float* h, const float* a, const __nv_bfloat16* U, const __nv_bfloat16* M,
-                  const float* b, float* out, int64_t nodes) {
-    if constexpr (H == 64)
-        k_update_tc<<<g->nb_dense, kT, tc::kSmemBytes, g->st>>>(h, a, U, M, b, out, nodes, g->d_err);
-    else
-        k_update<H><<<g->nb_dense, kT, update_smem<H>(), g->st>>>(h, a, U, M, b, out, nodes);
 }
 
 // After the stream is synchronised: a tensor-core update that gave up waiting
@@ -1258,7 +1545,7 @@ int device_error(sps_gnn* g) {
     if (cudaMemcpyAsync(&e, g->d_err, sizeof(e), cudaMemcpyDeviceToHost, g->st) != cudaSuccess ||
         cudaStreamSynchronize(g->st) != cudaSuccess)
         return g->fail(-2, "reading the network's error flag failed");
-    return e ? g->fail(-2, "internal error: a tensor-core node update stopped waiting for its MMAs") : 0;
+    return e ? g->fail(-2, "internal error: a tensor-core kernel stopped waiting for its MMAs") : 0;
 }
 
 // Whether a graph's constraint rows are long enough for a block each.
@@ -1303,7 +1590,8 @@ int forward64(sps_gnn* g, int batch, bool keep) {
         const int64_t oUv = obc + 64, oMv = oUv + 4096, obv = oMv + 4096;
         const bool first = l == 0 && in4, last = l == L - 1;
         agg_rows64(g, g->ac_c, first ? g->fv : g->HV[l], first, g->AC[l], batch, 0);
-        dense_update<64>(g, g->HC[l], g->AC[l], W + oUc, W + oMc, P + obc, g->HC[l + 1], NC);
+        k_con_update<<<(int)((NC + kConNodes - 1) / kConNodes), kT, 0, st>>>(g->HC[l], g->AC[l], W + oUc, W + oMc,
+                                                                            P + obc, g->HC[l + 1], NC);
         Node64 p{};
         p.h = g->HC[l + 1];
         p.U = W + oMv;
@@ -1349,10 +1637,14 @@ int forward64(sps_gnn* g, int batch, bool keep) {
 }
 
 // Forward pass over `batch` instances whose features are already on the device.
+// (keep: as forward64)
 template <int H>
-int forward(sps_gnn* g, int batch, bool keep) {
-    if constexpr (H == 64)
-        if (!keep) return forward64(g, batch, keep);
+int forward(sps_gnn* g, int batch, bool keep);
+template <>
+int forward<64>(sps_gnn* g, int batch, bool keep) { return forward64(g, batch, keep); }
+template <>
+int forward<32>(sps_gnn* g, int batch, bool) {
+    constexpr int H = 32;
     const int n = g->n, m = g->m, L = g->L;
     const int64_t NV = (int64_t)n * batch, NC = (int64_t)m * batch;
     const __nv_bfloat16* W = g->PB;
@@ -1365,10 +1657,10 @@ int forward(sps_gnn* g, int batch, bool keep) {
         const int64_t oUc = o, oMc = o + H * H, obc = o + 2 * H * H;
         const int64_t oUv = obc + H, oMv = oUv + H * H, obv = oMv + H * H;
         k_agg<H><<<grid_for(NC * 32, kT), kT, 0, st>>>(g->cptr, g->cidx, g->ac_c, g->HV[l], g->AC[l], m, n, batch, 0);
-        dense_update<H>(g, g->HC[l], g->AC[l], W + oUc, W + oMc, P + obc, g->HC[l + 1], NC);
+        k_update<H><<<g->nb_dense, kT, update_smem<H>(), st>>>(g->HC[l], g->AC[l], W + oUc, W + oMc, P + obc, g->HC[l + 1], NC);
         k_agg<H><<<grid_for(NV * 32, kT), kT, 0, st>>>(g->vptr, g->vidx, g->av_v, g->HC[l + 1], g->AV[l], n, m, batch,
                                                        0);
-        dense_update<H>(g, g->HV[l], g->AV[l], W + oUv, W + oMv, P + obv, g->HV[l + 1], NV);
+        k_update<H><<<g->nb_dense, kT, update_smem<H>(), st>>>(g->HV[l], g->AV[l], W + oUv, W + oMv, P + obv, g->HV[l + 1], NV);
     }
     k_head<H><<<grid_for(NV * 32, kT), kT, 0, st>>>(g->HV[L], W + g->oWx, P + g->obx, g->x0, NV);
     k_head<H><<<grid_for(NC * 32, kT), kT, 0, st>>>(g->HC[L], W + g->oWy, P + g->oby, g->y0, NC);
@@ -1378,6 +1670,148 @@ int forward(sps_gnn* g, int batch, bool keep) {
                                               P + g->obo, g->pool, g->lw);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : g->fail(-2, std::string("forward: ") + cudaGetErrorString(e));
+}
+
+// Blocks of a tensor-core node kernel over `nodes` nodes.
+int node_blocks(int64_t nodes) { return (int)std::min<int64_t>((nodes + 127) / 128, 2 * 152); }
+
+// The weight gradients of all layers (H = 64) into g->G, given the losses' output
+// gradients dx0, dy0, dlw: see k_back64 for what each side keeps.
+int backward64(sps_gnn* g, int batch) {
+    const int n = g->n, m = g->m, L = g->L;
+    const int64_t NV = (int64_t)n * batch, NC = (int64_t)m * batch;
+    const __nv_bfloat16* W = g->PB;
+    const float* P = g->P;
+    cudaStream_t st = g->st;
+    const int bv = node_blocks(NV), bc = node_blocks(NC);
+    SumJobs jobs;
+    int nj = 0;
+    float* part = g->part;                                      // handed out piece by piece
+    auto take = [&](int blocks, int stride) {
+        float* p = part;
+        part += (int64_t)blocks * stride;
+        return p;
+    };
+    auto sum = [&](const float* p, int blocks, int stride, int width, int64_t off) {
+        jobs.job[nj++] = SumJob{p, g->G + off, blocks, stride, width};
+    };
+    Back64 var{};                                               // what the variable side's passes share
+    var.ptr = g->vptr;
+    var.idx = g->vidx;
+    var.val = g->ac_v;
+    var.rows = m;
+    var.Win = W + g->oWv;
+    var.bin = P + g->obv;
+    var.n = n;
+    var.nodes = NV;
+    var.err = g->d_err;
+    Back64 con{};
+    con.Win = W + g->oWc;
+    con.bin = P + g->obc;
+    con.n = m;
+    con.nodes = NC;
+    con.err = g->d_err;
+    const bool in4 = g->Fv == 4;
+    float *dhv = g->dHV, *dhc = g->dHC, *dhc_next = g->dHC2;
+    for (int l = L - 1; l >= 0; --l) {
+        const int64_t o = g->layer_off(l);
+        const int64_t oUc = o, oMc = o + 4096, obc = o + 8192;
+        const int64_t oUv = obc + 64, oMv = oUv + 4096, obv = oMv + 4096;
+        const bool first = l == 0 && in4, last = l == L - 1;
+        // variable update: z, dh (in place of dout) and the gradients of Uv, bv (and of the x head)
+        Back64 a = var;
+        a.dout = last ? nullptr : dhv;
+        a.Q = last ? nullptr : g->dA;
+        a.dhead = g->dx0;
+        a.whead = W + g->oWx;
+        a.dlw = g->dlw;
+        a.wpool = W + g->oWo + 64;
+        a.out = g->HV[l + 1];
+        a.h = first ? g->fv : g->HV[l];
+        a.W = W + oUv;
+        a.z = g->dHV2;
+        a.dh = dhv;
+        a.part = take(bv, bk::kOut);
+        a.hpart = last ? take(bv, bk::kHeadOut) : nullptr;
+        if (first) k_back64<true><<<bv, bk::kThreads, bk::kSmem, st>>>(a);
+        else k_back64<false><<<bv, bk::kThreads, bk::kSmem, st>>>(a);
+        sum(a.part, bv, bk::kOut, 4096, oUv);
+        sum(a.part + 4096, bv, bk::kOut, 64, obv);
+        if (last) sum(a.hpart, bv, bk::kHeadOut, 65, g->oWx);
+        // sum_j a_ij z_j: the gradients of Mv and, added to the y head's or the next layer's, of HC[l + 1]
+        agg_rows64(g, g->av_c, g->dHV2, false, g->AG, batch, 0);
+        Back64 b = con;
+        b.dout = g->AG;
+        b.h = g->HC[l + 1];
+        b.W = W + oMv;
+        b.dh = dhc;
+        b.accumulate = 1;
+        b.part = take(bc, bk::kOut);
+        if (last) {     // the y head: dHC = dy0 wy + dlw wo / m
+            k_head_back<64><<<g->nb_dense, kT, 0, st>>>(g->HC[L], g->dy0, W + g->oWy, g->dlw, W + g->oWo, m, batch, dhc,
+                                                        take(g->nb_dense, 65));
+            sum(part - (int64_t)g->nb_dense * 65, g->nb_dense, 65, 65, g->oWy);
+        }
+        k_back64<false><<<bc, bk::kThreads, bk::kSmem, st>>>(b);
+        sum(b.part, bc, bk::kOut, 4096, oMv);
+        // constraint update: dHC[l], and dA of the aggregation for the variables
+        Back64 c = con;
+        c.dout = dhc;
+        c.out = g->HC[l + 1];
+        c.h = g->HC[l];
+        c.W = W + oUc;
+        c.dh = dhc_next;
+        c.part = take(bc, bk::kOut);
+        k_back64<false><<<bc, bk::kThreads, bk::kSmem, st>>>(c);
+        sum(c.part, bc, bk::kOut, 4096, oUc);
+        sum(c.part + 4096, bc, bk::kOut, 64, obc);
+        c.h = g->AC[l];
+        c.W = W + oMc;
+        c.dh = g->dA;
+        c.part = take(bc, bk::kOut);
+        k_back64<false><<<bc, bk::kThreads, bk::kSmem, st>>>(c);
+        sum(c.part, bc, bk::kOut, 4096, oMc);
+        std::swap(dhc, dhc_next);
+    }
+    // input layers
+    if (in4) {
+        Back64 a = var;
+        a.dout = dhv;
+        a.Q = g->dA;
+        a.h = g->fv;
+        a.part = take(2 * 152, kInOut);
+        k_in_back64<<<2 * 152, bk::kThreads, 0, st>>>(a);
+        sum(a.part, 2 * 152, kInOut, 320, g->oWv);
+    } else {
+        k_agg<64><<<grid_for(NV * 32, kT), kT, 0, st>>>(g->vptr, g->vidx, g->ac_v, g->dA, dhv, n, m, batch, 1);
+        const int w = 64 * g->Fv + 64;
+        float* p = take(g->nb_dense, w);
+        k_input_back<64><<<g->nb_dense, kT, 0, st>>>(dhv, g->HV[0], g->fv, g->Fv, NV, p);
+        sum(p, g->nb_dense, w, w, g->oWv);
+    }
+    {
+        const int w = 64 * g->Fc + 64;
+        float* p = take(g->nb_dense, w);
+        k_input_back<64><<<g->nb_dense, kT, 0, st>>>(dhc, g->HC[0], g->fc, g->Fc, NC, p);
+        sum(p, g->nb_dense, w, w, g->oWc);
+    }
+    k_sum_jobs<<<dim3(16, nj), kT, 0, st>>>(jobs);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? 0 : g->fail(-2, std::string("backward: ") + cudaGetErrorString(e));
+}
+
+// The loss from its partials (waits for the stream).
+int read_loss(sps_gnn* g, int batch, double* loss) {
+    if (!loss) return 0;
+    const int nbl = g->nb_loss;
+    std::vector<double> lp(2 * nbl + 1);
+    GNN_CK(cudaMemcpyAsync(lp.data(), g->lpart, sizeof(double) * lp.size(), cudaMemcpyDeviceToHost, g->st));
+    GNN_CK(cudaStreamSynchronize(g->st));
+    double sx = 0, sy = 0;
+    for (int b = 0; b < nbl; ++b) { sx += lp[b]; sy += lp[nbl + b]; }
+    const float ax = g->opt.loss_x, ay = g->opt.loss_y, ao = g->opt.loss_omega;
+    *loss = (ax * sx / g->n + ay * sy / g->m + ao * lp[2 * nbl]) / batch;
+    return 0;
 }
 
 // Loss (host value) and gradient into g->G (zeroed here) for `batch` instances
@@ -1395,51 +1829,48 @@ int backward(sps_gnn* g, int batch, double* loss) {
     k_sq_loss<<<nbl, kT, 0, st>>>(g->x0, g->xt, NV, 2.f * ax / (float(n) * batch), g->dx0, g->lpart);
     k_sq_loss<<<nbl, kT, 0, st>>>(g->y0, g->yt, NC, 2.f * ay / (float(m) * batch), g->dy0, g->lpart + nbl);
     k_sq_loss<<<1, kT, 0, st>>>(g->lw, g->lt, batch, 2.f * ao / float(batch), g->dlw, g->lpart + 2 * nbl);
-    // heads
-    const int nbh = g->nb_dense;
-    k_head_back<H><<<nbh, kT, 0, st>>>(g->HV[L], g->dx0, W + g->oWx, g->dlw, W + g->oWo + H, n, batch, g->dHV,
-                                       g->part);
-    k_sum_parts<<<4, 256, 0, st>>>(g->part, nbh, H + 1, 1.f, g->G + g->oWx);
-    k_head_back<H><<<nbh, kT, 0, st>>>(g->HC[L], g->dy0, W + g->oWy, g->dlw, W + g->oWo, m, batch, g->dHC, g->part);
-    k_sum_parts<<<4, 256, 0, st>>>(g->part, nbh, H + 1, 1.f, g->G + g->oWy);
-    k_omega_back<H><<<1, 2 * H, 0, st>>>(g->dlw, g->pool, batch, g->G + g->oWo, g->G + g->obo);
-    // layers, last to first.  dHV / dHC hold the gradient of HV[l+1] / HC[l+1].
-    float *dhv = g->dHV, *dhc = g->dHC, *dhv_next = g->dHV2, *dhc_next = g->dHC2;
-    const int width = 2 * H * H + H;
-    for (int l = L - 1; l >= 0; --l) {
-        const int64_t o = g->layer_off(l);
-        const int64_t oUc = o, oMc = o + H * H;
-        const int64_t oUv = oMc + H * H + H, oMv = oUv + H * H;
-        // variable update: HV[l+1] = relu(Uv HV[l] + Mv AV[l] + bv)
-        k_update_back<H><<<nbh, kT, update_back_smem<H>(), st>>>(dhv, g->HV[l + 1], g->HV[l], g->AV[l], W + oUv,
-                                                                 W + oMv, dhv_next, 0, g->dA, g->part, NV);
-        k_sum_parts<<<32, 256, 0, st>>>(g->part, nbh, width, 1.f, g->G + oUv);
-        // AV[l] = agg_v(HC[l+1]): dHC[l+1] += agg over constraints with a_v values
-        k_agg<H><<<grid_for(NC * 32, kT), kT, 0, st>>>(g->cptr, g->cidx, g->av_c, g->dA, dhc, m, n, batch, 1);
-        // constraint update: HC[l+1] = relu(Uc HC[l] + Mc AC[l] + bc)
-        k_update_back<H><<<nbh, kT, update_back_smem<H>(), st>>>(dhc, g->HC[l + 1], g->HC[l], g->AC[l], W + oUc,
-                                                                 W + oMc, dhc_next, 0, g->dA, g->part, NC);
-        k_sum_parts<<<32, 256, 0, st>>>(g->part, nbh, width, 1.f, g->G + oUc);
-        // AC[l] = agg_c(HV[l]): dHV[l] += agg over variables with a_c values
-        k_agg<H><<<grid_for(NV * 32, kT), kT, 0, st>>>(g->vptr, g->vidx, g->ac_v, g->dA, dhv_next, n, m, batch, 1);
-        std::swap(dhv, dhv_next);
-        std::swap(dhc, dhc_next);
+    if constexpr (H == 64) {
+        k_omega_back<H><<<1, 2 * H, 0, st>>>(g->dlw, g->pool, batch, g->G + g->oWo, g->G + g->obo);
+        if (int rc = backward64(g, batch)) return rc;
+    } else {
+        // heads
+        const int nbh = g->nb_dense;
+        k_head_back<H><<<nbh, kT, 0, st>>>(g->HV[L], g->dx0, W + g->oWx, g->dlw, W + g->oWo + H, n, batch, g->dHV,
+                                           g->part);
+        k_sum_parts<<<4, 256, 0, st>>>(g->part, nbh, H + 1, 1.f, g->G + g->oWx);
+        k_head_back<H><<<nbh, kT, 0, st>>>(g->HC[L], g->dy0, W + g->oWy, g->dlw, W + g->oWo, m, batch, g->dHC, g->part);
+        k_sum_parts<<<4, 256, 0, st>>>(g->part, nbh, H + 1, 1.f, g->G + g->oWy);
+        k_omega_back<H><<<1, 2 * H, 0, st>>>(g->dlw, g->pool, batch, g->G + g->oWo, g->G + g->obo);
+        // layers, last to first.  dHV / dHC hold the gradient of HV[l+1] / HC[l+1].
+        float *dhv = g->dHV, *dhc = g->dHC, *dhv_next = g->dHV2, *dhc_next = g->dHC2;
+        const int width = 2 * H * H + H;
+        for (int l = L - 1; l >= 0; --l) {
+            const int64_t o = g->layer_off(l);
+            const int64_t oUc = o, oMc = o + H * H;
+            const int64_t oUv = oMc + H * H + H, oMv = oUv + H * H;
+            // variable update: HV[l+1] = relu(Uv HV[l] + Mv AV[l] + bv)
+            k_update_back<H><<<nbh, kT, update_back_smem<H>(), st>>>(dhv, g->HV[l + 1], g->HV[l], g->AV[l], W + oUv,
+                                                                     W + oMv, dhv_next, 0, g->dA, g->part, NV);
+            k_sum_parts<<<32, 256, 0, st>>>(g->part, nbh, width, 1.f, g->G + oUv);
+            // AV[l] = agg_v(HC[l+1]): dHC[l+1] += agg over constraints with a_v values
+            k_agg<H><<<grid_for(NC * 32, kT), kT, 0, st>>>(g->cptr, g->cidx, g->av_c, g->dA, dhc, m, n, batch, 1);
+            // constraint update: HC[l+1] = relu(Uc HC[l] + Mc AC[l] + bc)
+            k_update_back<H><<<nbh, kT, update_back_smem<H>(), st>>>(dhc, g->HC[l + 1], g->HC[l], g->AC[l], W + oUc,
+                                                                     W + oMc, dhc_next, 0, g->dA, g->part, NC);
+            k_sum_parts<<<32, 256, 0, st>>>(g->part, nbh, width, 1.f, g->G + oUc);
+            // AC[l] = agg_c(HV[l]): dHV[l] += agg over variables with a_c values
+            k_agg<H><<<grid_for(NV * 32, kT), kT, 0, st>>>(g->vptr, g->vidx, g->ac_v, g->dA, dhv_next, n, m, batch, 1);
+            std::swap(dhv, dhv_next);
+            std::swap(dhc, dhc_next);
+        }
+        // input layers
+        k_input_back<H><<<nbh, kT, 0, st>>>(dhv, g->HV[0], g->fv, g->Fv, NV, g->part);
+        k_sum_parts<<<4, 256, 0, st>>>(g->part, nbh, H * g->Fv + H, 1.f, g->G + g->oWv);
+        k_input_back<H><<<nbh, kT, 0, st>>>(dhc, g->HC[0], g->fc, g->Fc, NC, g->part);
+        k_sum_parts<<<4, 256, 0, st>>>(g->part, nbh, H * g->Fc + H, 1.f, g->G + g->oWc);
     }
-    // input layers
-    k_input_back<H><<<nbh, kT, 0, st>>>(dhv, g->HV[0], g->fv, g->Fv, NV, g->part);
-    k_sum_parts<<<4, 256, 0, st>>>(g->part, nbh, H * g->Fv + H, 1.f, g->G + g->oWv);
-    k_input_back<H><<<nbh, kT, 0, st>>>(dhc, g->HC[0], g->fc, g->Fc, NC, g->part);
-    k_sum_parts<<<4, 256, 0, st>>>(g->part, nbh, H * g->Fc + H, 1.f, g->G + g->oWc);
     GNN_CK(cudaGetLastError());
-    if (loss) {
-        std::vector<double> lp(2 * nbl + 1);
-        GNN_CK(cudaMemcpyAsync(lp.data(), g->lpart, sizeof(double) * lp.size(), cudaMemcpyDeviceToHost, st));
-        GNN_CK(cudaStreamSynchronize(st));
-        double sx = 0, sy = 0;
-        for (int b = 0; b < nbl; ++b) { sx += lp[b]; sy += lp[nbl + b]; }
-        *loss = (ax * sx / n + ay * sy / m + ao * lp[2 * nbl]) / batch;
-    }
-    return 0;
+    return read_loss(g, batch, loss);
 }
 
 int upload_inputs(sps_gnn* g, int batch, const float* vf, const float* cf, const float* xt, const float* yt,
@@ -1656,11 +2087,18 @@ int sps_gnn_create(const sps_gnn_graph* gr, const sps_gnn_options* opt_in, sps_g
             }
             GNN_CK(g->alloc(&g->xt, NV)); GNN_CK(g->alloc(&g->yt, NC)); GNN_CK(g->alloc(&g->lt, B));
             g->HV.resize(g->L + 1); g->HC.resize(g->L + 1); g->AV.resize(g->L); g->AC.resize(g->L);
-            for (int l = 0; l <= g->L; ++l) { GNN_CK(g->alloc(&g->HV[l], NV * H)); GNN_CK(g->alloc(&g->HC[l], NC * H)); }
-            for (int l = 0; l < g->L; ++l) { GNN_CK(g->alloc(&g->AV[l], NV * H)); GNN_CK(g->alloc(&g->AC[l], NC * H)); }
+            // (H = 64: the input layer of four features and the variables' aggregates are not stored)
+            for (int l = 0; l <= g->L; ++l) {
+                if (l > 0 || H == 32 || g->Fv != 4) GNN_CK(g->alloc(&g->HV[l], NV * H));
+                GNN_CK(g->alloc(&g->HC[l], NC * H));
+            }
+            for (int l = 0; l < g->L; ++l) {
+                if (H == 32) GNN_CK(g->alloc(&g->AV[l], NV * H));
+                GNN_CK(g->alloc(&g->AC[l], NC * H));
+            }
             GNN_CK(g->alloc(&g->dHV, NV * H)); GNN_CK(g->alloc(&g->dHV2, NV * H));
             GNN_CK(g->alloc(&g->dHC, NC * H)); GNN_CK(g->alloc(&g->dHC2, NC * H));
-            GNN_CK(g->alloc(&g->dA, std::max(NV, NC) * H));
+            GNN_CK(g->alloc(&g->dA, (H == 64 ? NC : std::max(NV, NC)) * H));
             GNN_CK(g->alloc(&g->x0, NV)); GNN_CK(g->alloc(&g->y0, NC)); GNN_CK(g->alloc(&g->lw, B));
             GNN_CK(g->alloc(&g->dx0, NV)); GNN_CK(g->alloc(&g->dy0, NC)); GNN_CK(g->alloc(&g->dlw, B));
             GNN_CK(g->alloc(&g->pool, 2 * H * B));
@@ -1671,11 +2109,16 @@ int sps_gnn_create(const sps_gnn_graph* gr, const sps_gnn_options* opt_in, sps_g
             g->nb_pool_c = std::max(1, std::min(64, (m + 31) / 32));
             g->nb_pool_v = std::max(1, std::min(152, (n + 31) / 32));
             g->part_floats = (int64_t)g->nb_dense * (2 * H * H + H);
+            if (H == 64) {      // backward64's partials, all layers
+                const int64_t bv = node_blocks(NV), bc = node_blocks(NC);
+                g->part_floats = g->L * (bv + 3 * bc) * bk::kOut + bv * bk::kHeadOut +
+                                 (int64_t)g->nb_dense * (65 + kInOut + 2 * (64 * kMaxF + 64));
+            }
             GNN_CK(g->alloc(&g->part, g->part_floats));
             GNN_CK(g->alloc(&g->lpart, 2 * g->nb_loss + 1));
             GNN_CK(g->alloc(&g->pcp, (int64_t)g->nb_pool_c * H * B));
             GNN_CK(g->alloc(&g->pvp, std::max<int64_t>((int64_t)g->nb_pool_v * H * B, (NV + 127) / 128 * 128)));
-            if (H == 64) GNN_CK(g->alloc(&g->MH, NC * H));
+            if (H == 64) { GNN_CK(g->alloc(&g->MH, NC * H)); GNN_CK(g->alloc(&g->AG, NC * H)); }
             std::vector<float> p(g->np);
             init_params(p, g);
             GNN_CK(up(g->P, p.data(), sizeof(float) * g->np));

@@ -12,6 +12,7 @@ import pytest
 import scipy.sparse as sp
 
 import sovereign_solver_gb300 as sps
+from sovereign_solver_gb300 import gnn
 from sovereign_solver_gb300.gnn import WarmStartGNN
 from oracle import gnn_ref
 
@@ -33,8 +34,11 @@ def _relu_biases(lay):
     return e
 
 
-@pytest.mark.parametrize("n,m,density,B,L,H", SHAPES)
-def test_forward_and_gradient_match_oracle(n, m, density, B, L, H):
+@pytest.mark.parametrize("n,m,density,B,L,H,F", [(*s, (4, 4)) for s in SHAPES]
+                         + [(300, 40, 0.06, 3, 2, 64, (3, 5)), (300, 40, 0.06, 3, 2, 64, (8, 1))])
+def test_forward_and_gradient_match_oracle(n, m, density, B, L, H, F, monkeypatch):
+    monkeypatch.setattr(gnn, "FV", F[0])                 # feature widths of the network's inputs
+    monkeypatch.setattr(gnn, "FC", F[1])
     rng = np.random.default_rng(n + m)
     A = sp.random(m, n, density=density, random_state=n, format="csr")
     A.data = rng.standard_normal(A.nnz)
@@ -43,12 +47,12 @@ def test_forward_and_gradient_match_oracle(n, m, density, B, L, H):
                     lb=np.zeros(n), ub=np.full(n, np.inf), integer_mask=np.zeros(n, bool))
     with WarmStartGNN(p, hidden=H, layers=L, seed=n, max_batch=B, lp_features=False) as net:
         f32 = lambda *s: rng.standard_normal(s).astype(np.float32)                      # noqa: E731
-        fvs, fcs = [f32(n, 4) for _ in range(B)], [f32(m, 4) for _ in range(B)]
+        fvs, fcs = [f32(n, F[0]) for _ in range(B)], [f32(m, F[1]) for _ in range(B)]
         xts, yts, lts = [f32(n) for _ in range(B)], [f32(m) for _ in range(B)], f32(B)
         params = net.params()
         params += 0.1 * f32(params.size)                                                 # biases too
         net.set_params(params)
-        lay = gnn_ref.Layout(H, L, 4, 4)
+        lay = gnn_ref.Layout(H, L, *F)
         X, Y, Lw = net.predict_features(fvs, fcs)
         loss, g = net.loss_grad(fvs, fcs, xts, yts, lts)
         loss2, g2 = net.loss_grad(fvs, fcs, xts, yts, lts)

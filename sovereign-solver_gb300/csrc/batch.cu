@@ -46,13 +46,17 @@ struct Gather1 {
 // point 0 aliases the current iterate.
 __device__ __forceinline__ float ld_vec(const float* p, bool coh) { return coh ? __ldcg(p) : __ldg(p); }
 
+// The block's dynamic shared memory: the check's partial slots, which the
+// steps use as the staging buffer.
+extern __shared__ double s_slots[];
+#define s_stage reinterpret_cast<float*>(s_slots)
+
 // Gathers of the FP32 steps from a copy of the vector in shared memory (when
 // it fits the 7168-float staging buffer): an instance's gathers are random,
 // one 32-byte L1 sector (one L1 wavefront) per nonzero even on an L1 hit,
 // while a warp's 32 random shared-memory reads cost a few bank cycles.
 struct GatherS {
-    const float* s;
-    __device__ __forceinline__ float operator()(int, int j) const { return s[j]; }
+    __device__ __forceinline__ float operator()(int, int j) const { return s_stage[j]; }
 };
 
 // Copy x[0, n) into the staging buffer (coherent loads in a team, where other
@@ -207,11 +211,13 @@ struct View {                 // one instance's arrays
     float *Y[2], *AX[2], *ys, *yl, *axa;
     float *xb, *yb;
     float *axl, *atyl;
+    const int32_t *roff, *coff;   // slices (null: the side's passes walk the CSR)
+    const uint4 *rsteps, *csteps;
 };
 
-__device__ __forceinline__ View make_view(const Args& A, const Inst& I, int G) {
+// Fills the block's view of instance k (one thread).
+__device__ __forceinline__ void make_view(View& v, const Args& A, const Inst& I, int k, int G) {
     const Arrays& a = A.a;
-    View v;
     v.n = I.n; v.m = I.m; v.G = G & 0xFF; v.Gr = G >> 8 ? G >> 8 : 32;
     v.rptr = a.rptr + I.rp; v.ridx = a.ridx + I.re; v.rval = a.rval + I.re;
     v.cptr = a.cptr + I.cp; v.cidx = a.cidx + I.ce; v.cval = a.cval + I.ce;
@@ -226,7 +232,39 @@ __device__ __forceinline__ View make_view(const Args& A, const Inst& I, int G) {
     v.yb = a.yb ? a.yb + I.vr : nullptr;
     v.axl = a.axl + I.vr;
     v.atyl = a.atyl + I.vc;
-    return v;
+    v.roff = v.coff = nullptr;
+    if (a.slice) {
+        const Slice S = a.slice[k];
+        if (S.rstep >= 0) {
+            v.roff = a.soff + S.rchunk;
+            v.rsteps = a.steps + S.rstep * 64;
+        }
+        if (S.cstep >= 0) {
+            v.coff = a.soff + S.cchunk;
+            v.csteps = a.steps + S.cstep * 64;
+        }
+    }
+}
+
+// This thread's slots of the block's ring, behind the staging buffer.
+__device__ __forceinline__ Ring block_ring() {
+    return Ring{reinterpret_cast<uint4*>(s_slots + kColPartials * kBlock) + threadIdx.x};
+}
+
+// Row and column passes of a block (or its share of a team's).
+template <bool Sliced, int NV, class Acc, class Gather, class Epi>
+__device__ __forceinline__ void row_pass(const View& v, const Gather& g, Epi& e, const Team& T) {
+    if constexpr (Sliced) {
+        if (v.roff) return slice_rows<NV, Acc>(v.Gr, v.roff, v.rsteps, v.m, g, e, T.rank, T.size, block_ring());
+    }
+    group_rows_r<NV, Acc>(v.Gr, v.rptr, v.ridx, v.rval, v.m, g, e, T.rank, T.size);
+}
+template <bool Sliced, int NV, class Acc, class Gather, class Epi>
+__device__ __forceinline__ void col_pass(const View& v, const Gather& g, Epi& e, const Team& T) {
+    if constexpr (Sliced) {
+        if (v.coff) return slice_rows<NV, Acc>(v.G, v.coff, v.csteps, v.n, g, e, T.rank, T.size, block_ring());
+    }
+    group_rows_dyn<NV, Acc>(v.G, v.cptr, v.cidx, v.cval, v.n, g, e, T.rank, T.size);
 }
 
 // KKT check of average and current point, decision, and the restart copies.
@@ -262,7 +300,8 @@ struct Handoff {
     bool eligible;            // instance large enough (and hand-off on)
 };
 
-__device__ bool check_and_apply(const View& v, const Inst& I, Ctl& c, double* sm, double* slots, const uint64_t* dl,
+template <bool Sliced>
+__device__ __noinline__ bool check_and_apply(const View& v, const Inst& I, Ctl& c, double* sm, double* slots, const uint64_t* dl,
                                 const Team& T, const Handoff& H) {
     __shared__ bool s_handoff;
     const int chc = kWarps * (32 / v.G), chr = kWarps * (32 / v.Gr);
@@ -274,16 +313,14 @@ __device__ bool check_and_apply(const View& v, const Inst& I, Ctl& c, double* sm
     for (int q = 0; q < kRowPartials; ++q) mine[q * kBlock] = 0.0;
     RowCheckE er{v.b, has_avg ? v.ys : v.Y[cur], has_avg ? v.yl : nullptr, v.Y[cur], v.yl, v.dr, v.kind, v.axa, inv_w,
                  v.axl, mine};
-    group_rows_r<2, double>(v.Gr, v.rptr, v.ridx, v.rval, v.m,
-                            Gather2{has_avg ? v.xs : v.X[cur], has_avg ? v.xl : nullptr, v.X[cur], inv_w, T.size > 1}, er,
-                            T.rank, T.size);
+    row_pass<Sliced, 2, double>(v, Gather2{has_avg ? v.xs : v.X[cur], has_avg ? v.xl : nullptr, v.X[cur], inv_w, T.size > 1}, er,
+                        T);
     slot_sums<kRowPartials>(slots, sm);            // sm[0..10]: row partials
     for (int q = 0; q < kColPartials; ++q) mine[q * kBlock] = 0.0;
     ColCheckE ec{v.c, v.lo, v.hi, has_avg ? v.xs : v.X[cur], has_avg ? v.xl : nullptr, v.X[cur], v.xl, v.dc, v.atya,
                  inv_w, v.atyl, mine};
-    group_rows_dyn<2, double>(v.G, v.cptr, v.cidx, v.cval, v.n,
-                              Gather2{has_avg ? v.ys : v.Y[cur], has_avg ? v.yl : nullptr, v.Y[cur], inv_w, T.size > 1}, ec,
-                              T.rank, T.size);
+    col_pass<Sliced, 2, double>(v, Gather2{has_avg ? v.ys : v.Y[cur], has_avg ? v.yl : nullptr, v.Y[cur], inv_w, T.size > 1}, ec,
+                        T);
     slot_sums<kColPartials>(slots, sm + kRowPartials);   // then the column partials
     // team totals of the partials and of the deadline test (any block past it stops all)
     constexpr int NT = kRowPartials + kColPartials;
@@ -372,7 +409,8 @@ __device__ bool check_and_apply(const View& v, const Inst& I, Ctl& c, double* sm
 // Start point of instance k (cold: x = clip(0, lo, hi), y = 0; warm: the caller's
 // point scaled and projected, with its primal weight), its products K x0 and
 // K^T y0, and the init-phase check that records its relative KKT error.
-__device__ bool start_point(const Args& A, int k, const Inst& I, const View& v, bool warm, Ctl& c, double* sm,
+template <bool Sliced>
+__device__ __noinline__ bool start_point(const Args& A, int k, const Inst& I, const View& v, bool warm, Ctl& c, double* sm,
                             double* slots, const Team& T) {
     const int chc = kWarps * (32 / v.G), chr = kWarps * (32 / v.Gr);
     if (!team_barrier(T)) return false;
@@ -404,18 +442,24 @@ __device__ bool start_point(const Args& A, int k, const Inst& I, const View& v, 
     }
     if (!team_barrier(T)) return false;
     StoreE sx{v.AX[0]};
-    group_rows_r<1, float>(v.Gr, v.rptr, v.ridx, v.rval, v.m, Gather1{v.X[0], T.size > 1}, sx, T.rank, T.size);
+    row_pass<Sliced, 1, float>(v, Gather1{v.X[0], T.size > 1}, sx, T);
     StoreE sy{v.ATY[0]};
-    group_rows_dyn<1, float>(v.G, v.cptr, v.cidx, v.cval, v.n, Gather1{v.Y[0], T.size > 1}, sy, T.rank, T.size);
+    col_pass<Sliced, 1, float>(v, Gather1{v.Y[0], T.size > 1}, sy, T);
     if (!team_barrier(T)) return false;
-    return check_and_apply(v, I, c, sm, slots, A.deadline, T, Handoff{A.idle, A.idle_need, false});
+    return check_and_apply<Sliced>(v, I, c, sm, slots, A.deadline, T, Handoff{A.idle, A.idle_need, false});
 }
 
 // The whole solve of instance k by this block (T.size == 1) or by the team of
 // blocks of a cluster.  Returns false when a team barrier timed out.
-__device__ bool solve_one(const Args& A, int k, int G, Ctl& c, double* sm, double* slots, const Team& T) {
-    const Inst I = A.inst[k];
-    const View v = make_view(A, I, G);
+template <bool Sliced>
+__device__ __forceinline__ bool solve_one(const Args& A, int k, int G, Ctl& c, double* sm, double* slots, const Team& T) {
+    __shared__ Inst I;
+    __shared__ View v;
+    if (threadIdx.x == 0) {
+        I = A.inst[k];
+        make_view(v, A, I, k, G);
+    }
+    __syncthreads();
     const int chc = kWarps * (32 / v.G), chr = kWarps * (32 / v.Gr);
     const uint64_t t_begin = global_ns();
     const bool warm = A.warm != 0;
@@ -424,17 +468,17 @@ __device__ bool solve_one(const Args& A, int k, int G, Ctl& c, double* sm, doubl
         // keep the warm point only if its relative KKT error is not above the cold start's
         double cold = A.cold_rel[k];
         if (!(cold >= 0.0)) {
-            if (!start_point(A, k, I, v, false, c, sm, slots, T)) return false;
+            if (!start_point<Sliced>(A, k, I, v, false, c, sm, slots, T)) return false;
             cold = c.rel_kkt;
             if (threadIdx.x == 0 && T.rank == 0) A.cold_rel[k] = cold;
         }
-        if (!start_point(A, k, I, v, true, c, sm, slots, T)) return false;
+        if (!start_point<Sliced>(A, k, I, v, true, c, sm, slots, T)) return false;
         if (!(c.rel_kkt <= cold)) {
             used = false;
-            if (!start_point(A, k, I, v, false, c, sm, slots, T)) return false;
+            if (!start_point<Sliced>(A, k, I, v, false, c, sm, slots, T)) return false;
         }
     } else {
-        if (!start_point(A, k, I, v, warm, c, sm, slots, T)) return false;
+        if (!start_point<Sliced>(A, k, I, v, warm, c, sm, slots, T)) return false;
     }
     // Step sizes of the next attempt, computed once by thread 0 (FP64 products
     // and divisions per thread would occupy this GPU's FP64 pipe, 1/64 of the
@@ -443,7 +487,7 @@ __device__ bool solve_one(const Args& A, int k, int G, Ctl& c, double* sm, doubl
     float* smf = reinterpret_cast<float*>(sm);
     const Handoff H{A.idle, A.idle_need, A.handoff_nnz > 0 && I.nnz >= A.handoff_nnz};
     // the staging buffer shares its memory with the check's partial slots
-    float* stage = reinterpret_cast<float*>(slots);
+    float* const stage = s_stage;
     const bool stage_x = v.n <= A.stage_cap, stage_y = v.m <= A.stage_cap;
     if (threadIdx.x == 0) {
         c.t_begin = t_begin;
@@ -458,10 +502,9 @@ __device__ bool solve_one(const Args& A, int k, int G, Ctl& c, double* sm, doubl
             RowStepE er{v.b, v.AX[cur], v.Y[cur], v.kind, v.AX[1 - cur], v.Y[1 - cur], s_sigma};
             if (stage_x) {
                 stage_vector(stage, v.X[1 - cur], v.n, T.size > 1);
-                group_rows_r<1, float>(v.Gr, v.rptr, v.ridx, v.rval, v.m, GatherS{stage}, er, T.rank, T.size);
+                row_pass<Sliced, 1, float>(v, GatherS{}, er, T);
             } else {
-                group_rows_r<1, float>(v.Gr, v.rptr, v.ridx, v.rval, v.m, Gather1{v.X[1 - cur], T.size > 1}, er,
-                                       T.rank, T.size);
+                row_pass<Sliced, 1, float>(v, Gather1{v.X[1 - cur], T.size > 1}, er, T);
             }
             float f2[2] = {er.dy2, er.inter};
             block_sum<2>(f2, smf);
@@ -481,10 +524,9 @@ __device__ bool solve_one(const Args& A, int k, int G, Ctl& c, double* sm, doubl
                 ColStepE ec{v.X[cur], v.c, v.lo, v.hi, v.xl, v.ATY[cur], v.X[1 - cur], v.xs, tau, wgt};
                 if (stage_y) {
                     stage_vector(stage, v.Y[cur], v.m, T.size > 1);
-                    group_rows_dyn<1, float>(v.G, v.cptr, v.cidx, v.cval, v.n, GatherS{stage}, ec, T.rank, T.size);
+                    col_pass<Sliced, 1, float>(v, GatherS{}, ec, T);
                 } else {
-                    group_rows_dyn<1, float>(v.G, v.cptr, v.cidx, v.cval, v.n, Gather1{v.Y[cur], T.size > 1}, ec,
-                                             T.rank, T.size);
+                    col_pass<Sliced, 1, float>(v, Gather1{v.Y[cur], T.size > 1}, ec, T);
                 }
                 dx2 = ec.dx2;
                 TEAM_OWNED(i, v.m, chr) v.ys[i] += wgt * (v.Y[cur][i] - v.yl[i]);
@@ -509,7 +551,7 @@ __device__ bool solve_one(const Args& A, int k, int G, Ctl& c, double* sm, doubl
             __syncthreads();
         }
         if (c.done) break;
-        if (!check_and_apply(v, I, c, sm, slots, A.deadline, T, H)) return false;
+        if (!check_and_apply<Sliced>(v, I, c, sm, slots, A.deadline, T, H)) return false;
         if (c.done) break;
         if (threadIdx.x == 0) s_sigma = float(c.eta * c.omega);
         __syncthreads();
@@ -527,12 +569,21 @@ __device__ bool solve_one(const Args& A, int k, int G, Ctl& c, double* sm, doubl
 // 0 takes it for the whole cluster (every block reads the index from rank 0's
 // shared memory between two team barriers) and the team solves it; from the
 // first smaller instance on, every block takes its own instances.
-__global__ void __launch_bounds__(kBlock, 4) k_batch_solve(Args A, int G) {
+//
+// Sliced: the passes read the slices of the instances (sides) that have them,
+// two blocks on an SM with kRing steps per warp in flight each (640 planted LPs:
+// 521 ms a solve with four blocks on the CSR, 342 ms now; 40 children of a
+// 200 x 2000 node: 33.2 ms, now 25.6).  The other form, four blocks and no ring,
+// times the schedules, since the schedule fixes the order of the sums, and
+// serves a batch without slices.  The grid is the four-block one for both: its
+// blocks past the resident ones start when others end.
+template <bool Sliced>
+__global__ void __launch_bounds__(kBlock, Sliced ? 2 : 4) k_batch_solve(Args A, int G) {
     __shared__ Ctl c;
     __shared__ double sm[kWarps * 10];
     // dynamic: the check partial slots (kColPartials * kBlock doubles), reused as the
     // steps' staging buffer of A.stage_cap floats
-    extern __shared__ double slots[];
+    double* const slots = s_slots;
     __shared__ double xch[2 * kXch];
     __shared__ uint32_t counter;
     __shared__ int s_inst, s_err;
@@ -549,16 +600,15 @@ __global__ void __launch_bounds__(kBlock, 4) k_batch_solve(Args A, int G) {
         asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
     }
     __syncthreads();
-    const Team team{C, rank, &counter, &gen, xch, &phase, &s_err};
-    const Team solo{1, 0, &counter, &gen, xch, &phase, &s_err};
     bool together = C > 1;
     for (;;) {
         int k;
+        if (threadIdx.x == 0 && (!together || rank == 0)) {
+            const uint32_t q = atomicAdd(A.counter, 1u);
+            s_inst = q < (uint32_t)A.count ? A.order[q] : -1;
+        }
         if (together) {
-            if (threadIdx.x == 0 && rank == 0) {
-                const uint32_t q = atomicAdd(A.counter, 1u);
-                s_inst = q < (uint32_t)A.count ? A.order[q] : -1;
-            }
+            const Team team{C, rank, &counter, &gen, xch, &phase, &s_err};
             if (!team_barrier(team)) break;
             if (threadIdx.x == 0) {
                 int r0;
@@ -569,22 +619,17 @@ __global__ void __launch_bounds__(kBlock, 4) k_batch_solve(Args A, int G) {
             k = int(sm[0]);
             if (!team_barrier(team)) break;       // rank 0 may overwrite s_inst only after every block read it
             if (k < 0) break;
-            if (A.inst[k].nnz >= A.team_nnz) {
-                if (!solve_one(A, k, G, c, sm, slots, team)) break;
-                continue;
+            if (A.inst[k].nnz < A.team_nnz) {
+                together = false;                  // smaller instances: one block each from now on
+                if (rank != 0) continue;
             }
-            together = false;                      // smaller instances: one block each from now on
-            if (rank != 0) continue;
         } else {
-            if (threadIdx.x == 0) {
-                const uint32_t q = atomicAdd(A.counter, 1u);
-                s_inst = q < (uint32_t)A.count ? A.order[q] : -1;
-            }
             __syncthreads();
             k = s_inst;
             if (k < 0) break;
         }
-        solve_one(A, k, G, c, sm, slots, solo);
+        const Team T{together ? C : 1, together ? rank : 0, &counter, &gen, xch, &phase, &s_err};
+        if (!solve_one<Sliced>(A, k, G, c, sm, slots, T) && together) break;
         __syncthreads();
     }
     // this block found the queue empty (or its team gave up): it counts towards
@@ -719,6 +764,82 @@ __global__ void __launch_bounds__(kBlock) k_batch_setup(SetupArgs S) {
     }
 }
 
+// Steps of every chunk's slice: one block per (instance, side); the offsets of
+// its chunks (exclusive sums, one more at the end) go to soff.  per_warp rows
+// make a chunk; a lane's share of a row of `len` entries is its every G-th, in
+// fours.
+__global__ void __launch_bounds__(kBlock) k_slice_count(const Inst* inst, const Slice* slice, Arrays a, int G, int Gr,
+                                                        int32_t* soff) {
+    const int k = blockIdx.x;
+    const bool col = blockIdx.y;
+    const Inst& I = inst[k];
+    const int count = col ? I.n : I.m, lanes = col ? G : Gr, per_warp = 32 / lanes;
+    const int32_t* ptr = col ? a.cptr + I.cp : a.rptr + I.rp;
+    int32_t* out = soff + (col ? slice[k].cchunk : slice[k].rchunk);
+    const int chunks = (count + per_warp - 1) / per_warp;
+    __shared__ int warp_sum[kWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int base = 0;
+    for (int c0 = 0; c0 < chunks; c0 += kBlock) {
+        const int ch = c0 + threadIdx.x;
+        int steps = 0;
+        if (ch < chunks) {
+            int len = 0;
+            for (int r = ch * per_warp; r < min((ch + 1) * per_warp, count); ++r) len = max(len, ptr[r + 1] - ptr[r]);
+            steps = max((len + 4 * lanes - 1) / (4 * lanes), 1);
+        }
+        int s = steps;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += t;
+        }
+        if (lane == 31) warp_sum[warp] = s;
+        __syncthreads();
+        int before = base, all = 0;
+        for (int w = 0; w < kWarps; ++w) {
+            if (w < warp) before += warp_sum[w];
+            all += warp_sum[w];
+        }
+        if (ch < chunks) out[ch] = before + s - steps;
+        base += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) out[chunks] = base;
+}
+
+// The slices' entries: one block per (instance, side), a warp per chunk.
+__global__ void __launch_bounds__(kBlock) k_slice_fill(const Inst* inst, const Slice* slice, Arrays a, int G, int Gr,
+                                                       const int32_t* soff, uint4* steps) {
+    const int k = blockIdx.x;
+    const bool col = blockIdx.y;
+    const Inst& I = inst[k];
+    const int64_t first = col ? slice[k].cstep : slice[k].rstep;
+    if (first < 0) return;
+    const int count = col ? I.n : I.m, lanes = col ? G : Gr, per_warp = 32 / lanes;
+    const int32_t* ptr = col ? a.cptr + I.cp : a.rptr + I.rp;
+    const int32_t* idx = col ? a.cidx + I.ce : a.ridx + I.re;
+    const float* val = col ? a.cval + I.ce : a.rval + I.re;
+    const int32_t* off = soff + (col ? slice[k].cchunk : slice[k].rchunk);
+    const int chunks = (count + per_warp - 1) / per_warp, wl = threadIdx.x & 31;
+    for (int ch = threadIdx.x >> 5; ch < chunks; ch += kWarps) {
+        const int r = ch * per_warp + wl / lanes, lane = wl & (lanes - 1);
+        const int s = r < count ? ptr[r] + lane : 0, t = r < count ? ptr[r + 1] : 0;
+        for (int p = off[ch]; p < off[ch + 1]; ++p) {
+            const int q0 = s + 4 * (p - off[ch]) * lanes;
+            uint32_t j[4];
+            float f[4];
+            for (int u = 0; u < 4; ++u) {
+                const int q = q0 + u * lanes;
+                j[u] = q < t ? idx[q] : 0;
+                f[u] = q < t ? val[q] : 0.f;
+            }
+            uint4* at = steps + (first + p) * 64 + wl;
+            at[0] = make_uint4(j[0], j[1], j[2], j[3]);
+            at[32] = make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3]));
+        }
+    }
+}
+
 // Inputs of the warm-start network for instances s0 .. s0+cnt-1 from the batch's
 // scaled data: c = c~ / dc, b = b~ / dr (the original costs and right-hand sides).
 __global__ void __launch_bounds__(kBlock) k_gnn_inputs(const Inst* inst, int s0, int cnt, Arrays a, int n, int m,
@@ -798,7 +919,7 @@ struct HostBuf {
 struct sps_batch {
     int32_t count = 0;
     sps_options opt{};
-    int32_t G = 8, Gr = 32, blocks = 0;      // lanes per column / per row, persistent blocks
+    int32_t G = 0, Gr = 0, blocks = 0;       // lanes per column / per row, persistent blocks
     int32_t stage_cap = 0;                    // floats of the kernel's shared staging buffer
     size_t dyn_smem = 0;                      // dynamic shared memory of the solve launch
     int32_t team = 1;                         // cluster size of the solve launch
@@ -967,6 +1088,82 @@ int continue_single(sps_batch* b, int32_t k, double used_s, std::string* why) {
     c.choice = r.returned_average;
     b->escalated[k] = handoff ? (int8_t)r.escalated : 1;
     b->handed_off[k] = handoff ? 1 : 0;
+    return SPS_OK;
+}
+
+// Lays the entries of every instance out for the batch's schedule (slice_rows).
+// A side stays on its CSR where it has no entries or where padding makes the
+// slices more than three times as long as the entries (a few long rows among
+// short ones): a column of four entries, one lane each, pads to 2.5 times its
+// length in a chunk of 32 and still gains.  Without memory for them the batch runs on the CSR alone.
+int build_slices(sps_batch* b) {
+    const int32_t count = b->count;
+    std::vector<sps::batch::Slice> sl(count);
+    int64_t chunks = 0;
+    for (int32_t k = 0; k < count; ++k) {
+        const Inst& I = b->inst[k];
+        sl[k].rchunk = chunks;
+        chunks += (I.m + 32 / b->Gr - 1) / (32 / b->Gr) + 1;
+        sl[k].cchunk = chunks;
+        chunks += (I.n + 32 / b->G - 1) / (32 / b->G) + 1;
+        sl[k].rstep = sl[k].cstep = -1;
+    }
+    const int smem = (int)b->dyn_smem + sps::batch::kRingBytes;
+    SPB_CK(cudaFuncSetAttribute(sps::batch::k_batch_solve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    if (b->team > 1) {                    // its clusters have to fit too
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = b->team;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(b->blocks);
+        cfg.blockDim = dim3(sps::kBlock);
+        cfg.dynamicSmemBytes = smem;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int ncl = 0;
+        if (cudaOccupancyMaxActiveClusters(&ncl, sps::batch::k_batch_solve<true>, &cfg) != cudaSuccess || ncl < 1) {
+            cudaGetLastError();
+            return SPS_OK;
+        }
+    }
+    sps::batch::Slice* d_slice = nullptr;
+    int32_t* d_off = nullptr;
+    uint4* d_steps = nullptr;
+    std::vector<int32_t> off(chunks);
+    if (b->alloc(&d_slice, count) != cudaSuccess || b->alloc(&d_off, chunks) != cudaSuccess) {
+        cudaGetLastError();
+        return SPS_OK;
+    }
+    SPB_CK(cudaMemcpyAsync(d_slice, sl.data(), sizeof(sl[0]) * count, cudaMemcpyHostToDevice, b->st));
+    sps::batch::k_slice_count<<<dim3(count, 2), sps::kBlock, 0, b->st>>>(b->d_inst, d_slice, b->arr, b->G, b->Gr, d_off);
+    SPB_CK(cudaGetLastError());
+    SPB_CK(cudaMemcpyAsync(off.data(), d_off, sizeof(int32_t) * chunks, cudaMemcpyDeviceToHost, b->st));
+    SPB_CK(cudaStreamSynchronize(b->st));
+    int64_t steps = 0;
+    for (int32_t k = 0; k < count; ++k) {
+        const Inst& I = b->inst[k];
+        const int64_t rs = off[sl[k].cchunk - 1], cs = off[(k + 1 < count ? sl[k + 1].rchunk : chunks) - 1];
+        const auto fits = [&](int64_t s) {
+            return I.nnz > 0 && s * 128 <= 3 * (int64_t)I.nnz + 128 * sps::kWarps;
+        };
+        if (fits(rs)) { sl[k].rstep = steps; steps += rs; }
+        if (fits(cs)) { sl[k].cstep = steps; steps += cs; }
+    }
+    if (steps == 0) return SPS_OK;
+    if (b->alloc(&d_steps, steps * 64) != cudaSuccess) {
+        cudaGetLastError();
+        return SPS_OK;
+    }
+    SPB_CK(cudaMemcpyAsync(d_slice, sl.data(), sizeof(sl[0]) * count, cudaMemcpyHostToDevice, b->st));
+    sps::batch::k_slice_fill<<<dim3(count, 2), sps::kBlock, 0, b->st>>>(b->d_inst, d_slice, b->arr, b->G, b->Gr, d_off,
+                                                                         d_steps);
+    SPB_CK(cudaGetLastError());
+    SPB_CK(cudaStreamSynchronize(b->st));
+    b->arr.slice = d_slice;
+    b->arr.soff = d_off;
+    b->arr.steps = d_steps;
     return SPS_OK;
 }
 
@@ -1199,7 +1396,7 @@ extern "C" int sps_batch_create(int32_t count, const sps_problem_desc* probs, co
         // 80k-column transportation family).
         b->dyn_smem = sizeof(double) * sps::kColPartials * sps::kBlock;
         b->stage_cap = (int32_t)(b->dyn_smem / sizeof(float));
-        SPB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, sps::batch::k_batch_solve, sps::kBlock,
+        SPB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, sps::batch::k_batch_solve<false>, sps::kBlock,
                                                              b->dyn_smem));
         SPB_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         const int64_t slots = (int64_t)std::max(nb, 1) * sms;      // resident blocks of one wave
@@ -1244,7 +1441,7 @@ extern "C" int sps_batch_create(int32_t count, const sps_problem_desc* probs, co
             cfg.attrs = attr;
             cfg.numAttrs = 1;
             int ncl = 0;
-            if (cudaOccupancyMaxActiveClusters(&ncl, sps::batch::k_batch_solve, &cfg) == cudaSuccess && ncl > 0) {
+            if (cudaOccupancyMaxActiveClusters(&ncl, sps::batch::k_batch_solve<false>, &cfg) == cudaSuccess && ncl > 0) {
                 b->team = want;
                 b->blocks = (int)((need / want) * want);
             }
@@ -1272,11 +1469,9 @@ extern "C" int sps_batch_create(int32_t count, const sps_problem_desc* probs, co
         if (it != g_schedules.end()) {
             b->G = it->second.first;
             b->Gr = it->second.second;
-            *out = b.release();
-            return SPS_OK;
         }
     }
-    {
+    if (b->G == 0) {
         sps_batch* bb = bp;
         // A sample spread over the whole size range (every stride-th instance of the
         // largest-first order); a candidate's cost is the SUM of its instances' device
@@ -1294,7 +1489,7 @@ extern "C" int sps_batch_create(int32_t count, const sps_problem_desc* probs, co
                                bb->d_counter, 0};
             A.stage_cap = bb->stage_cap;
             cudaMemsetAsync(bb->d_counter, 0, sizeof(uint32_t), bb->st);
-            sps::batch::k_batch_solve<<<std::min(bb->blocks, sample), sps::kBlock, bb->dyn_smem, bb->st>>>(A, sched);
+            sps::batch::k_batch_solve<false><<<std::min(bb->blocks, sample), sps::kBlock, bb->dyn_smem, bb->st>>>(A, sched);
             cudaMemcpyAsync(outs.data(), bb->d_out, sizeof(Ctl) * count, cudaMemcpyDeviceToHost, bb->st);
             if (cudaStreamSynchronize(bb->st) != cudaSuccess) return false;
             double tot = 0.0;
@@ -1330,6 +1525,11 @@ extern "C" int sps_batch_create(int32_t count, const sps_problem_desc* probs, co
         std::lock_guard<std::mutex> lk(g_schedule_mu);
         g_schedules[key] = {gc, gr};
     }
+    const int rc = build_slices(bp);
+    if (rc != SPS_OK) {
+        sps::set_create_error(bp->err);
+        return rc;
+    }
     *out = b.release();
     return SPS_OK;
 }
@@ -1351,6 +1551,9 @@ extern "C" int sps_batch_solve(sps_batch* b, sps_batch_stats* stats) {
         cudaMemsetAsync(b->d_team_error, 0, sizeof(int32_t), s);
         cudaMemsetAsync(b->d_idle, 0, sizeof(uint32_t), s);
         const int sched = sps::batch::pack_schedule(b->G, b->Gr);
+        const bool sliced = b->arr.slice != nullptr;
+        const auto kernel = sliced ? sps::batch::k_batch_solve<true> : sps::batch::k_batch_solve<false>;
+        const size_t smem = b->dyn_smem + (sliced ? sps::batch::kRingBytes : 0);
         if (b->team > 1) {
             cudaLaunchConfig_t cfg = {};
             cudaLaunchAttribute attr[1];
@@ -1360,13 +1563,13 @@ extern "C" int sps_batch_solve(sps_batch* b, sps_batch_stats* stats) {
             attr[0].val.clusterDim.z = 1;
             cfg.gridDim = dim3(b->blocks);
             cfg.blockDim = dim3(sps::kBlock);
-            cfg.dynamicSmemBytes = b->dyn_smem;
+            cfg.dynamicSmemBytes = smem;
             cfg.stream = s;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
-            cudaLaunchKernelEx(&cfg, sps::batch::k_batch_solve, A, sched);
+            cudaLaunchKernelEx(&cfg, kernel, A, sched);
         } else {
-            sps::batch::k_batch_solve<<<b->blocks, sps::kBlock, b->dyn_smem, s>>>(A, sched);
+            kernel<<<b->blocks, sps::kBlock, smem, s>>>(A, sched);
         }
     };
     SPB_CK(cudaEventRecord(b->e0, b->st));

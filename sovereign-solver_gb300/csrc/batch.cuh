@@ -3,7 +3,8 @@
 //
 // Layout: every instance's CSR (rows: A_ub then A_eq) and CSC are packed back
 // to back (offsets inside an instance are local, 0-based); column vectors and
-// row vectors likewise.  One block of 256 threads owns one instance at a time
+// row vectors likewise; and for the schedule that the batch runs, slices of the
+// entries in the order in which the passes read them (below).  One block of 256 threads owns one instance at a time
 // and runs the whole adaptive PDHG loop on it with block barriers only: rows
 // one warp each, columns `G` lanes each (G in 1..32, autotuned), FP32 iterates, FP64
 // block reductions, the same step/restart/termination decisions as the
@@ -24,6 +25,13 @@ struct Inst {                 // per-instance descriptor
     double inv_nb, inv_nc;    // 1 / (1 + ||rhs||), 1 / (1 + ||c||) of the original data
 };
 
+// Where an instance's slices lie (base of its chunk offsets and of its steps;
+// step < 0: this side of the instance has none and its passes walk the CSR).
+struct Slice {
+    int64_t rchunk, cchunk;
+    int64_t rstep, cstep;
+};
+
 struct Arrays {
     const int32_t *rptr, *ridx, *cptr, *cidx;
     const float *rval, *cval;
@@ -35,6 +43,9 @@ struct Arrays {
     float *y0, *y1, *ax0, *ax1, *ys, *yl, *axa;
     float *xb, *yb;           // best point of the stall test (null when it is off)
     float *axl, *atyl;        // K x_last, K^T y_last (infeasibility tests)
+    const Slice* slice;       // null: no instance has slices
+    const int32_t* soff;      // per chunk: first step (local to the instance), one more at the end
+    const uint4* steps;       // per step 32 lanes' four indices, then their four values
 };
 
 struct Args {
@@ -162,6 +173,7 @@ __device__ __forceinline__ void group_rows(const int32_t* __restrict__ ptr, cons
                                            int trank = 0, int tsize = 1) {
     constexpr int per_warp = 32 / G;
     const int warp = threadIdx.x >> 5, wl = threadIdx.x & 31, lane = wl & (G - 1);
+#pragma unroll 1
     for (int base = (trank * kWarps + warp) * per_warp; base < count; base += tsize * kWarps * per_warp) {
         const int r = base + wl / G;
         const bool valid = r < count;
@@ -171,6 +183,7 @@ __device__ __forceinline__ void group_rows(const int32_t* __restrict__ ptr, cons
         Acc acc[NV];
 #pragma unroll
         for (int q = 0; q < NV; ++q) acc[q] = Acc(0);
+#pragma unroll 1
         for (int k = s + lane; k < t; k += 4 * G) {
             int j[4];
             Acc a[4];
@@ -214,6 +227,132 @@ __device__ __forceinline__ void group_rows_r(int G, const int32_t* ptr, const in
         case 8: group_rows<8, NV, Acc>(ptr, idx, val, count, g, e, tr, ts); break;
         case 16: group_rows<16, NV, Acc>(ptr, idx, val, count, g, e, tr, ts); break;
         default: group_rows<32, NV, Acc>(ptr, idx, val, count, g, e, tr, ts); break;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Slices: the entries of a chunk (the 32 / G rows a warp takes at once) laid out
+// in the order in which its lanes read them.  Step p of a chunk holds, for every
+// lane of a row, its four entries lane + (4 p + u) G, u < 4: 32 lanes' indices
+// (16 bytes each), then their values.  Lanes past their row's end hold index 0
+// and value 0, as group_rows takes there, and every lane adds in group_rows'
+// order: the sums have the same bits.
+//
+// What bounds the passes is the latency of the entries (a batch of 640 planted
+// LPs holds 240 MB of them, twice the L2).  group_rows has one group of four
+// entries per lane in flight and spends about eight instructions on each; here a
+// step is two 16-byte copies into the lane's own part of a ring in shared
+// memory, kRing steps ahead, and two instructions per entry (gather, multiply).
+// 192 attempts of every instance: 31.3 ms on the CSR, 24.0 with two steps ahead
+// in registers, 17.0 with the ring (2.7 TB/s from DRAM); a lone 200 x 2000 child
+// LP of 4 entries per column: 17,100 cycles per column pass, now 14,800.
+constexpr int kRing = 8;                  // steps in flight per warp: 64 KB a block, two blocks an SM.  The same
+                                          // 192 attempts: 20.3 ms with 10, and with three blocks 21.2 with 4
+constexpr int kRingBytes = kRing * 32 * kBlock;
+
+// A lane's own slots of the block's ring: kRing steps on their way from global
+// memory (32 bytes per lane and step, read by the lane that copied them, so no
+// lane waits for another).
+struct Ring {
+    uint4* own;               // slot d: indices at own[2 d kBlock], values one kBlock further
+    __device__ __forceinline__ void copy(int slot, const uint4* from) const {
+        const uint32_t to = (uint32_t)__cvta_generic_to_shared(own + slot * (2 * kBlock));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(from) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 16 * kBlock), "l"(from + 32) : "memory");
+    }
+    __device__ __forceinline__ static void commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+    // all but the newest N requests have arrived
+    template <int N>
+    __device__ __forceinline__ static void wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+};
+
+// The steps of a warp's chunks in the order in which it takes them, requested
+// kRing ahead (one commit group per step, empty past the end).
+struct Feed {
+    const int32_t* off;
+    const uint4* steps;       // this lane's part of step 0
+    int ch, chunks, stride;   // chunk of the next request
+    int p, e, np, ne;         // its next step and end; the chunk after it
+    __device__ __forceinline__ void range(int c, int& a, int& b) const {
+        a = b = 0;
+        if (c < chunks) {
+            a = __ldg(off + c);
+            b = __ldg(off + c + 1);
+        }
+    }
+    __device__ __forceinline__ void request(const Ring& ring, int slot) {
+        if (p < e) {
+            ring.copy(slot, steps + (int64_t)p * 64);
+            if (++p == e) {
+                p = np;
+                e = ne;
+                ch += stride;
+                range(ch + stride, np, ne);
+            }
+        }
+        Ring::commit();
+    }
+};
+
+// Row chunks of a pass by one block of a team.  Every chunk has at least one step.
+template <int NV, class Acc, class Gather, class Epi>
+__device__ __forceinline__ void slice_rows(int G, const int32_t* __restrict__ off, const uint4* __restrict__ steps,
+                                           int count, const Gather& g, Epi& e, int trank, int tsize, const Ring& ring) {
+    const int per_warp = 32 / G, chunks = (count + per_warp - 1) / per_warp, stride = tsize * kWarps;
+    const int wl = threadIdx.x & 31;
+    int ch = trank * kWarps + (threadIdx.x >> 5);
+    if (ch >= chunks) return;
+    Feed f{off, steps + wl, ch, chunks, stride, 0, 0, 0, 0};
+    f.range(ch, f.p, f.e);
+    f.range(ch + stride, f.np, f.ne);
+    int P = f.e - f.p;
+#pragma unroll 1
+    for (int d = 0; d < kRing; ++d) f.request(ring, d);
+    int slot = 0;
+    Acc acc[NV];
+    const auto take = [&](int at) {
+        const uint4 jj = ring.own[at * (2 * kBlock)], aa = ring.own[at * (2 * kBlock) + kBlock];
+        const uint32_t j[4] = {jj.x, jj.y, jj.z, jj.w}, a[4] = {aa.x, aa.y, aa.z, aa.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) acc[q] += Acc(__uint_as_float(a[u])) * g(q, int(j[u]));
+    };
+    const auto next = [&](int at) { return at + 1 == kRing ? 0 : at + 1; };
+#pragma unroll 1
+    for (;;) {
+        int oa, ea;
+        f.range(ch + stride, oa, ea);
+        const int r = ch * per_warp + wl / G;
+        const bool lead = r < count && (wl & (G - 1)) == 0;
+        typename Epi::Pre pre;
+        if (lead) pre = e.pre(r);
+#pragma unroll
+        for (int q = 0; q < NV; ++q) acc[q] = Acc(0);
+#pragma unroll 1
+        for (int p = 0; p + 1 < P; p += 2) {
+            const int second = next(slot);
+            Ring::wait<kRing - 2>();
+            take(slot);
+            take(second);
+            f.request(ring, slot);
+            f.request(ring, second);
+            slot = next(second);
+        }
+        if (P & 1) {
+            Ring::wait<kRing - 1>();
+            take(slot);
+            f.request(ring, slot);
+            slot = next(slot);
+        }
+#pragma unroll 1
+        for (int s = G / 2; s > 0; s >>= 1)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], s);
+        if (lead) e(r, acc, pre);
+        ch += stride;
+        if (ch >= chunks) break;
+        P = ea - oa;
     }
 }
 

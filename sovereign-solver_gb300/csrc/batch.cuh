@@ -45,6 +45,7 @@ struct Arrays {
     float *axl, *atyl;        // K x_last, K^T y_last (infeasibility tests)
     const Slice* slice;       // null: no instance has slices
     const int32_t* soff;      // per chunk: first step (local to the instance), one more at the end
+    double2* pts;             // per column, then per row of an instance: both points of a check in FP64
     const uint4* steps;       // per step 32 lanes' four indices, then their four values
 };
 

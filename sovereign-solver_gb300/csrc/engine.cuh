@@ -842,10 +842,10 @@ __device__ __forceinline__ void visit_slab_unit(const Bin& b, int u, const Layou
     }
 }
 
-// Dispatch: find the bin of pass block `block`; its warp `warp` walks the bin's
-// units with a grid stride.
+// Dispatch: find the bin of pass block `block`; its warps walk the bin's units
+// with a grid stride.
 template <int NV, class Acc, class V, class Gather, class Epi>
-__device__ __forceinline__ void visit_bins(const BinTable& bt, int block, int warp, const Layout<V>& L,
+__device__ __forceinline__ void visit_bins(const BinTable& bt, int block, const Layout<V>& L,
                                            const Gather& g, Epi& e) {
     int bi = -1;
 #pragma unroll
@@ -855,7 +855,7 @@ __device__ __forceinline__ void visit_bins(const BinTable& bt, int block, int wa
     if (bi < 0) return;
     const Bin& b = bt.bin[bi];
     const int stride = b.nblocks * kWarps;
-    const int w0 = (block - b.block_begin) * kWarps + warp;
+    const int w0 = (block - b.block_begin) * kWarps + (threadIdx.x >> 5);
     if (b.mode == BM_SLICED) {
         // rows of one or two nonzeros each (the columns of transportation and assignment
         // LPs): the exact-length loop (FP32 iterates; in the FP64 engine its extra code
@@ -878,12 +878,6 @@ __device__ __forceinline__ void visit_bins(const BinTable& bt, int block, int wa
         for (int u = w0; u < b.units; u += stride) visit_slab_unit<NV, Acc>(b, u, L, g, e);
     }
 }
-template <int NV, class Acc, class V, class Gather, class Epi>
-__device__ __forceinline__ void visit_bins(const BinTable& bt, int block, const Layout<V>& L,
-                                           const Gather& g, Epi& e) {
-    visit_bins<NV, Acc>(bt, block, threadIdx.x >> 5, L, g, e);
-}
-
 // Epilogue helper with nothing to prefetch.
 struct NoPre {};
 

@@ -120,19 +120,11 @@ struct GatherOne {
 // Adaptive mode
 // ============================================================================
 
-// What a step's epilogue does with its new vector entry besides storing it (the
-// resident kernels copy it to the shared memory their next pass gathers from).
-struct NoSink {
-    template <class V>
-    __device__ __forceinline__ void operator()(int, V) const {}
-};
-
-template <class V, class Sink = NoSink>
+template <class V>
 struct AdRowStepEpi {
     const V *b, *axo, *yo;
     V *axn, *yn;
     V sigma;
-    Sink sink = Sink{};
     V dy2 = V(0), inter = V(0);          // per-thread partials; FP64 from the block sum on
     struct Pre { V ao, yv, br; };
     static constexpr int NP = 2;
@@ -146,7 +138,6 @@ struct AdRowStepEpi {
         V y2 = mad(sigma, p.br - (ax + ax - p.ao), p.yv);
         if (kind) y2 = fmin(y2, V(0));
         yn[r] = y2;
-        sink(r, y2);
         const V dy = y2 - p.yv;
         dy2 = mad(dy, dy, dy2);
         inter = mad(dy, ax - p.ao, inter);
@@ -194,7 +185,7 @@ SPS_PASS_KERNEL ad_row_step(Args<V> a) {
     decide_step(*ctl, double(t[0]), double(t[1]));
 }
 
-template <class V, class Sink = NoSink>
+template <class V>
 struct AdColStepEpi {
     const Args<V>* a;
     const V *xc, *cc, *atyo;
@@ -202,7 +193,6 @@ struct AdColStepEpi {
     V *aty, *xn, *xs;
     V tau, wgt;
     bool accepted;
-    Sink sink = Sink{};
     V dx2 = V(0);
     struct Pre { V xj, cj, lo, hi, s, l; };
     static constexpr int NP = 1;
@@ -223,7 +213,6 @@ struct AdColStepEpi {
         if (accepted) { aty[j] = atyj; xs[j] = mad(wgt, p.xj - p.l, p.s); }
         const V x2 = clampv(mad(-tau, p.cj - atyj, p.xj), p.lo, p.hi);
         xn[j] = x2;
-        sink(j, x2);
         const V d = x2 - p.xj;
         dx2 = mad(d, d, dx2);
     }
@@ -597,11 +586,10 @@ SPS_CHECK_KERNEL spmv_cols(Args<V> a, const V* y, V* out) {
 // reference's own order of operations.
 // ============================================================================
 
-template <class V, class Sink = NoSink>
+template <class V>
 struct RfColStepEpi {
     const V *tau, *c;
     V *x, *xbar, *xs;
-    Sink sink = Sink{};
     struct Pre { V xv, t, cj, s; };
     static constexpr int NP = 0;
     __device__ __forceinline__ Pre pre(int j) const { return Pre{x[j], tau[j], c[j], xs[j]}; }
@@ -610,7 +598,6 @@ struct RfColStepEpi {
         x2 = fmax(x2, V(0));
         const V xb = rn_sub(rn_mul(V(2), x2), p.xv);
         xbar[j] = xb;
-        sink(j, xb);
         x[j] = x2;
         xs[j] = rn_add(p.s, x2);
     }
@@ -624,18 +611,16 @@ SPS_PASS_KERNEL rf_col_step(Args<V> a) {
     visit_bins<1, V>(a.cols, blockIdx.x, a.csc, GatherOne<V>{a.Y[0]}, e);
 }
 
-template <class V, class Sink = NoSink>
+template <class V>
 struct RfRowStepEpi {
     const V *sigma, *b;
     V *y, *ys;
-    Sink sink = Sink{};
     struct Pre { V yv, s, br, acc_s; };
     static constexpr int NP = 0;
     __device__ __forceinline__ Pre pre(int r) const { return Pre{y[r], sigma[r], b[r], ys[r]}; }
     __device__ __forceinline__ void operator()(int r, int, const V (&acc)[1], const Pre& p) {
         const V y2 = rn_add(p.yv, rn_mul(p.s, rn_sub(p.br, acc[0])));
         y[r] = y2;
-        sink(r, y2);
         ys[r] = rn_add(p.acc_s, y2);
     }
 };

@@ -655,9 +655,9 @@ def run_warmstart(args, rank, world):
     per_it = 16 * nnz + 4 * (m_ + 1) + 4 * n_ + 20 * m_ + 4 * (n_ + 1) + 4 * m_ + 28 * n_ + 16 * m_
     solve_s = np.mean([s_[1] for s_ in steps])
     achieved = float(wi.sum()) * per_it / solve_s / 1e9
-    # per chunk of 16 instances: 2 LP-feature kernels + 19 network kernels (L = 3) +
-    # the batch's input and output kernels; per step 3 batch kernels
-    fwd_launches = 9 + 4 * net.layers + 2
+    # per chunk of 16 instances: 2 LP-feature kernels, the input layer, 4 kernels per
+    # layer and 3 of the heads + the batch's input and output kernels; per step 3 batch kernels
+    fwd_launches = 6 + 4 * net.layers + 2
     line = {
         "metric": METRIC,
         "value": value, "unit": "solves/s",

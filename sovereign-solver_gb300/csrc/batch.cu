@@ -597,14 +597,18 @@ __device__ __forceinline__ bool solve_one(const Args& A, int k, int G, Ctl& c, d
 // first smaller instance on, every block takes its own instances.
 //
 // Sliced: the passes read the slices of the instances (sides) that have them,
-// two blocks on an SM with kRing steps per warp in flight each (640 planted LPs:
-// 521 ms a solve with four blocks on the CSR, 342 ms now; 40 children of a
-// 200 x 2000 node: 33.2 ms, now 25.6).  The other form, four blocks and no ring,
-// times the schedules, since the schedule fixes the order of the sums, and
-// serves a batch without slices.  The grid is the four-block one for both: its
-// blocks past the resident ones start when others end.
-template <bool Sliced>
-__global__ void __launch_bounds__(kBlock, Sliced ? 2 : 4) k_batch_solve(Args A, int G) {
+// PerSm blocks on an SM with kRing steps per warp in flight each.  Two for a
+// batch of more blocks than SMs (three sets of 640 planted LPs: 549, 389 and 338
+// ms a solve with four blocks on the CSR, 297, 172 and 152 now); one, whose
+// registers do not spill, where an SM has no second block to run (40 children of
+// a 200 x 2000 node: 20.5 ms with two, 18.9 now; 640 LPs at their start, before
+// the small ones end, 15.0 ms for 192 attempts with two and 18.3 with one).  The
+// other form, four blocks and no ring, times the schedules, since the schedule
+// fixes the order of the sums, and serves a batch without slices.  The grid is
+// the four-block one for all: its blocks past the resident ones start when others
+// end.
+template <bool Sliced, int PerSm>
+__global__ void __launch_bounds__(kBlock, PerSm) k_batch_solve(Args A, int G) {
     __shared__ Ctl c;
     __shared__ double sm[kWarps * 10];
     // dynamic: the check partial slots (kColPartials * kBlock doubles), reused as the
@@ -947,6 +951,7 @@ struct sps_batch {
     sps_options opt{};
     int32_t G = 0, Gr = 0, blocks = 0;       // lanes per column / per row, persistent blocks
     int32_t stage_cap = 0;                    // floats of the kernel's shared staging buffer
+    void (*sliced_kernel)(sps::batch::Args, int) = nullptr;   // the form of the solve for a batch with slices
     size_t dyn_smem = 0;                      // dynamic shared memory of the solve launch
     int32_t team = 1;                         // cluster size of the solve launch
     int32_t team_nnz = 65536;                 // instances at least this large are solved by a team
@@ -1135,7 +1140,10 @@ int build_slices(sps_batch* b) {
         sl[k].rstep = sl[k].cstep = -1;
     }
     const int smem = (int)b->dyn_smem + sps::batch::kRingBytes;
-    SPB_CK(cudaFuncSetAttribute(sps::batch::k_batch_solve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    int sms = 152;
+    SPB_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->opt.device));
+    b->sliced_kernel = b->blocks <= sms ? sps::batch::k_batch_solve<true, 1> : sps::batch::k_batch_solve<true, 2>;
+    SPB_CK(cudaFuncSetAttribute(b->sliced_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     if (b->team > 1) {                    // its clusters have to fit too
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
@@ -1149,7 +1157,7 @@ int build_slices(sps_batch* b) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int ncl = 0;
-        if (cudaOccupancyMaxActiveClusters(&ncl, sps::batch::k_batch_solve<true>, &cfg) != cudaSuccess || ncl < 1) {
+        if (cudaOccupancyMaxActiveClusters(&ncl, b->sliced_kernel, &cfg) != cudaSuccess || ncl < 1) {
             cudaGetLastError();
             return SPS_OK;
         }
@@ -1425,7 +1433,7 @@ extern "C" int sps_batch_create(int32_t count, const sps_problem_desc* probs, co
         // 80k-column transportation family).
         b->dyn_smem = sizeof(double) * sps::kColPartials * sps::kBlock;
         b->stage_cap = (int32_t)(b->dyn_smem / sizeof(float));
-        SPB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, sps::batch::k_batch_solve<false>, sps::kBlock,
+        SPB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, sps::batch::k_batch_solve<false, 4>, sps::kBlock,
                                                              b->dyn_smem));
         SPB_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         const int64_t slots = (int64_t)std::max(nb, 1) * sms;      // resident blocks of one wave
@@ -1470,7 +1478,7 @@ extern "C" int sps_batch_create(int32_t count, const sps_problem_desc* probs, co
             cfg.attrs = attr;
             cfg.numAttrs = 1;
             int ncl = 0;
-            if (cudaOccupancyMaxActiveClusters(&ncl, sps::batch::k_batch_solve<false>, &cfg) == cudaSuccess && ncl > 0) {
+            if (cudaOccupancyMaxActiveClusters(&ncl, sps::batch::k_batch_solve<false, 4>, &cfg) == cudaSuccess && ncl > 0) {
                 b->team = want;
                 b->blocks = (int)((need / want) * want);
             }
@@ -1518,7 +1526,7 @@ extern "C" int sps_batch_create(int32_t count, const sps_problem_desc* probs, co
                                bb->d_counter, 0};
             A.stage_cap = bb->stage_cap;
             cudaMemsetAsync(bb->d_counter, 0, sizeof(uint32_t), bb->st);
-            sps::batch::k_batch_solve<false><<<std::min(bb->blocks, sample), sps::kBlock, bb->dyn_smem, bb->st>>>(A, sched);
+            sps::batch::k_batch_solve<false, 4><<<std::min(bb->blocks, sample), sps::kBlock, bb->dyn_smem, bb->st>>>(A, sched);
             cudaMemcpyAsync(outs.data(), bb->d_out, sizeof(Ctl) * count, cudaMemcpyDeviceToHost, bb->st);
             if (cudaStreamSynchronize(bb->st) != cudaSuccess) return false;
             double tot = 0.0;
@@ -1581,7 +1589,7 @@ extern "C" int sps_batch_solve(sps_batch* b, sps_batch_stats* stats) {
         cudaMemsetAsync(b->d_idle, 0, sizeof(uint32_t), s);
         const int sched = sps::batch::pack_schedule(b->G, b->Gr);
         const bool sliced = b->arr.slice != nullptr;
-        const auto kernel = sliced ? sps::batch::k_batch_solve<true> : sps::batch::k_batch_solve<false>;
+        const auto kernel = sliced ? b->sliced_kernel : sps::batch::k_batch_solve<false, 4>;
         const size_t smem = b->dyn_smem + (sliced ? sps::batch::kRingBytes : 0);
         if (b->team > 1) {
             cudaLaunchConfig_t cfg = {};

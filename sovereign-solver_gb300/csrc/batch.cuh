@@ -245,10 +245,14 @@ __device__ __forceinline__ void group_rows_r(int G, const int32_t* ptr, const in
 // step is two 16-byte copies into the lane's own part of a ring in shared
 // memory, kRing steps ahead, and two instructions per entry (gather, multiply).
 // 192 attempts of every instance: 31.3 ms on the CSR, 24.0 with two steps ahead
-// in registers, 17.0 with the ring (2.7 TB/s from DRAM); a lone 200 x 2000 child
+// in registers, 17.0 with a ring of eight and 15.0 as it is now (3.7 TB/s from
+// DRAM); a lone 200 x 2000 child
 // LP of 4 entries per column: 17,100 cycles per column pass, now 14,800.
-constexpr int kRing = 8;                  // steps in flight per warp: 64 KB a block, two blocks an SM.  The same
-                                          // 192 attempts: 20.3 ms with 10, and with three blocks 21.2 with 4
+// Steps in flight per warp: 48 KB a block.  More leaves two blocks on an
+// SM too little L1 (three sets of 640 planted LPs: 314, 186
+// and 165 ms a solve with 8 steps, 297, 172 and 152 with 6, 292, 176 and 152 with
+// 5; three blocks of 4 steps 390, 271 and 225: their 80 registers spill).
+constexpr int kRing = 6;
 constexpr int kRingBytes = kRing * 32 * kBlock;
 
 // A lane's own slots of the block's ring: kRing steps on their way from global

@@ -72,3 +72,13 @@ def test_slices_of_a_team():
         assert b.stats.team == 4
     for p, r in zip(probs, res):
         _check(p, r)
+
+
+def test_more_instances_than_sms():
+    """The form with two blocks on an SM (the batches above run one)."""
+    probs = [wl.batch_planted_lp(k, m_range=(20, 90))[0] for k in range(330)]
+    with sps.PDHGBatch(probs, tol=TOL, max_iters=200000) as b:
+        res = b.solve()
+        assert b.stats.blocks > 152
+    for p, r in zip(probs, res):
+        _check(p, r)

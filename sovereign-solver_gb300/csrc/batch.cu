@@ -1125,8 +1125,16 @@ int continue_single(sps_batch* b, int32_t k, double used_s, std::string* why) {
 // Lays the entries of every instance out for the batch's schedule (slice_rows).
 // A side stays on its CSR where it has no entries or where padding makes the
 // slices more than three times as long as the entries (a few long rows among
-// short ones): a column of four entries, one lane each, pads to 2.5 times its
-// length in a chunk of 32 and still gains.  Without memory for them the batch runs on the CSR alone.
+// short ones).  In a batch of more blocks than SMs it also needs a step's four
+// entries per lane on average: shorter rows are one group of loads on the CSR, all
+// in flight at once, and padding only adds traffic (1000 transportation LPs of
+// 80 000 two-entry columns: 3.0 ms each on the CSR, 3.75 on slices; 640 planted
+// LPs, 15 entries per lane, three sets: 521, 389 and 338 ms on the CSR, 297, 172
+// and 152 on slices).  There an instance has both sides sliced or neither, and
+// the batch runs on its CSR if more than a quarter of its entries would.  With one
+// block on an SM short columns gain too (children with four entries per column:
+// 33.4 ms on the CSR, 18.9 on slices).  Without memory for the slices, or clusters
+// for the teams, the batch runs on the CSR.
 int build_slices(sps_batch* b) {
     const int32_t count = b->count;
     std::vector<sps::batch::Slice> sl(count);
@@ -1176,17 +1184,22 @@ int build_slices(sps_batch* b) {
     SPB_CK(cudaGetLastError());
     SPB_CK(cudaMemcpyAsync(off.data(), d_off, sizeof(int32_t) * chunks, cudaMemcpyDeviceToHost, b->st));
     SPB_CK(cudaStreamSynchronize(b->st));
-    int64_t steps = 0;
+    const bool spread = b->blocks <= sms;
+    int64_t steps = 0, left = 0, entries = 0;
     for (int32_t k = 0; k < count; ++k) {
         const Inst& I = b->inst[k];
         const int64_t rs = off[sl[k].cchunk - 1], cs = off[(k + 1 < count ? sl[k + 1].rchunk : chunks) - 1];
-        const auto fits = [&](int64_t s) {
-            return I.nnz > 0 && s * 128 <= 3 * (int64_t)I.nnz + 128 * sps::kWarps;
+        const auto fits = [&](int64_t s, int64_t rows, int lanes) {
+            return I.nnz > 0 && s * 128 <= 3 * (int64_t)I.nnz + 128 * sps::kWarps &&
+                   (spread || I.nnz >= 4 * rows * lanes);
         };
-        if (fits(rs)) { sl[k].rstep = steps; steps += rs; }
-        if (fits(cs)) { sl[k].cstep = steps; steps += cs; }
+        const bool row = fits(rs, I.m, b->Gr), col = fits(cs, I.n, b->G);
+        entries += I.nnz;
+        if (!spread && !(row && col)) { left += I.nnz; continue; }
+        if (row) { sl[k].rstep = steps; steps += rs; }
+        if (col) { sl[k].cstep = steps; steps += cs; }
     }
-    if (steps == 0) return SPS_OK;
+    if (steps == 0 || 4 * left > entries) return SPS_OK;
     if (b->alloc(&d_steps, steps * 64) != cudaSuccess ||
         b->alloc(&d_pts, (size_t)(b->sum_n + b->sum_m)) != cudaSuccess) {
         cudaGetLastError();

@@ -74,9 +74,12 @@ def test_slices_of_a_team():
         _check(p, r)
 
 
-def test_more_instances_than_sms():
-    """The form with two blocks on an SM (the batches above run one)."""
-    probs = [wl.batch_planted_lp(k, m_range=(20, 90))[0] for k in range(330)]
+@pytest.mark.parametrize("kind", ["planted", "two_entry_columns", "mixed"])
+def test_more_instances_than_sms(kind):
+    """Two blocks on an SM (the batches above run one): sliced, on the CSR, and some of each."""
+    planted = [wl.batch_planted_lp(k, m_range=(40, 90))[0] for k in range(200)]
+    short = [wl.transportation_lp(5 + k % 7, 9 + k % 5, seed=k)[0] for k in range(200)]
+    probs = {"planted": planted, "two_entry_columns": short, "mixed": planted + short}[kind]
     with sps.PDHGBatch(probs, tol=TOL, max_iters=200000) as b:
         res = b.solve()
         assert b.stats.blocks > 152

@@ -271,6 +271,10 @@ __device__ __forceinline__ void split(const float4& x, uint2 (&p)[3]) {
     for (int q = 0; q < 3; ++q) {
         p[q] = make_uint2(upper(r.x, r.y), upper(r.z, r.w));
         if (q < 2) r = make_float4(r.x - cut(r.x), r.y - cut(r.y), r.z - cut(r.z), r.w - cut(r.w));
+        // an infinity is its own first part: inf - inf would make the sum of the parts NaN, and a ReLU 0 of that
+        if (q == 0 && !(fabsf(x.x) + fabsf(x.y) + fabsf(x.z) + fabsf(x.w) < INFINITY))
+            r = make_float4(isfinite(x.x) ? r.x : 0.f, isfinite(x.y) ? r.y : 0.f, isfinite(x.z) ? r.z : 0.f,
+                            isfinite(x.w) ? r.w : 0.f);
     }
 }
 // piece f (four floats) of row r of a tile's parts
@@ -931,6 +935,8 @@ __device__ __forceinline__ void add2(float p, float& hi, float& lo) {
     lo += __fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(p, b));
     hi = t;
 }
+// the sum of the two: lo is NaN (inf - inf) once hi has left the finite numbers
+__device__ __forceinline__ float sum2(float hi, float lo) { return isfinite(hi) ? hi + lo : hi; }
 
 // Aggregation over long rows (H = 64): a block per destination row of one instance,
 // each warp a stretch of its edges (lane l: features 2 l, 2 l + 1; eight rows in
@@ -986,14 +992,15 @@ __global__ void __launch_bounds__(kT) k_agg_rows(const int32_t* __restrict__ ptr
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             if (First) v[u] = make_float2(InW::one(w0, b0, ff[u]), InW::one(w1, b1, ff[u]));
+            if (e + u >= e1) continue;             // no edge: node 0 may be infinite
             t.x = fmaf(a[u], v[u].x, t.x);
             t.y = fmaf(a[u], v[u].y, t.y);
         }
         add2(t.x, acc.x, low.x);
         add2(t.y, acc.y, low.y);
     }
-    acc.x += low.x;
-    acc.y += low.y;
+    acc.x = sum2(acc.x, low.x);
+    acc.y = sum2(acc.y, low.y);
     part[warp][lane] = acc;
     __syncthreads();
     if (warp) return;
@@ -1059,7 +1066,7 @@ __global__ void __launch_bounds__(kT) k_con_update(const float* __restrict__ h, 
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-        if (v0 + g + 4 * i < nodes) out[(v0 + g + 4 * i) * 64 + o] = relu(hi[i] + lo[i]);
+        if (v0 + g + 4 * i < nodes) out[(v0 + g + 4 * i) * 64 + o] = relu(sum2(hi[i], lo[i]));
 }
 
 // The pooled head from k_node64's column sums of the variables (per tile, in order) and k_colsum_part's of the constraints.

@@ -1031,11 +1031,12 @@ __global__ void __launch_bounds__(kT) k_con_update(const float* __restrict__ h, 
                                                    const __nv_bfloat16* __restrict__ M,
                                                    const float* __restrict__ bias, float* __restrict__ out,
                                                    int64_t nodes) {
-    __shared__ float Wt[128 * 64];             // [k][o]
+    __shared__ float Wt[128 * 65];             // [k][o], rows of 65: a warp stages a row of U or M and reads along o
     __shared__ float4 X[kConNodes][32];
-    for (int t = threadIdx.x; t < 128 * 64; t += kT) {
-        const int o = t & 63, k = t >> 6;
-        Wt[t] = __bfloat162float(k < 64 ? U[o * 64 + k] : M[o * 64 + k - 64]);
+    for (int t = threadIdx.x; t < 64 * 64; t += kT) {
+        const int o = t >> 6, k = t & 63;
+        Wt[k * 65 + o] = __bfloat162float(U[t]);
+        Wt[(k + 64) * 65 + o] = __bfloat162float(M[t]);
     }
     const int64_t v0 = (int64_t)blockIdx.x * kConNodes;
     for (int t = threadIdx.x; t < kConNodes * 32; t += kT) {
@@ -1055,7 +1056,7 @@ __global__ void __launch_bounds__(kT) k_con_update(const float* __restrict__ h, 
     for (int q = 0; q < 32; q += 2) {
         float w[8];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) w[c] = Wt[(4 * q + c) * 64 + o];
+        for (int c = 0; c < 8; ++c) w[c] = Wt[(4 * q + c) * 65 + o];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const float4 x = X[g + 4 * i][q], y = X[g + 4 * i][q + 1];

@@ -4,12 +4,13 @@
 // Activations are kept per instance and node, row-major with the hidden width
 // innermost ([instance][node][H], FP32), so every per-node kernel runs over the
 // flattened node list of the whole batch and the weight gradients are sums
-// over it.  With H = 64 the variable side's dense updates, forward and backward, run
-// on the tensor cores (k_node64, k_back64: tcgen05, FP32 as three BF16 parts) and
-// the constraint side's M products are made there (k_con_update, k_agg_rows);
-// H = 32 keeps register-tiled FP32 contractions and CSR SpMM aggregations.  Every
-// reduction (weight gradients, losses, pooling) writes per-block partials that
-// are summed in block order: training is bitwise reproducible.
+// over it.  With H = 64 the dense updates, forward and backward, run on the tensor
+// cores (k_node64, k_back64: tcgen05, FP32 as three BF16 parts); on graphs with few
+// rows the M products are made on the constraint side, whose own update is
+// compensated FP32 (k_con_update).  H = 32 keeps register-tiled FP32 contractions and
+// CSR SpMM aggregations.  Every reduction (weight gradients, losses, pooling) writes
+// per-block partials that are summed in block order: training is bitwise
+// reproducible.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -233,7 +234,8 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 // relu(U h + M a + b) with a_j = sum_i a_ij hc_i is relu(U h + sum_i a_ij (M hc_i) + b):
 // M is applied to the constraint nodes (a few thousand) instead of to every
 // variable node's aggregate, so the aggregate is neither written nor read and
-// the large contraction has K = 64 instead of 128.  What is left is a stream: h
+// the large contraction has K = 64 instead of 128 (graphs with few rows, forward64;
+// on others Two adds the second product of the aggregate).  What is left is a stream: h
 // in, out (512 bytes a node), the rows of M hc from L2.  On 1.28M nodes (16
 // instances of the 200 x 400 family) a layer's aggregation and update took 180 +
 // 300 us; now 229 us (0.66 GB, 96 us at the measured HBM rate: the chain staging ->
@@ -323,6 +325,7 @@ struct Node64 {
     const float* h;                           // nodes x 64, or with First the features (nodes x 4)
     const __nv_bfloat16* Win; const float* bin;   // First: the input layer
     const __nv_bfloat16* U;                   // 64 x 64
+    const float* a; const __nv_bfloat16* M;   // Two: the second input (nodes x 64) and its weights
     const float* P;                           // rows added along the edges (null: none)
     const int32_t *ptr, *idx; const float* val;   // edges of a node; rows of instance s at P + s * rows * 64
     int n, rows;                              // nodes and rows of an instance
@@ -334,24 +337,25 @@ struct Node64 {
     int32_t* err;
 };
 
-constexpr int kNode64Smem = bf::kW + 3 * bf::kPart + 1024;   // + alignment
+constexpr int node64_smem(bool two) { return (two ? 2 : 1) * bf::kW + 3 * bf::kPart + 1024; }   // + alignment
 // 512 threads, two blocks an SM: 16 threads a row of 256 contiguous bytes, four
 // rows a thread.  The node's edges are a chain of three dependent loads; with
 // 256 threads (eight rows each, half the warps to overlap) a layer of 1.28M
 // nodes took 230 us.
 constexpr int kN64T = 512;
 
-template <bool First, bool Heads>
+template <bool First, bool Heads, bool Two>
 __global__ void __launch_bounds__(kN64T, 2) k_node64(const Node64 a) {
     extern __shared__ __align__(16) unsigned char n64_smem[];
     unsigned char* base = n64_smem + ((1024 - (tc::smem_u32(n64_smem) & 1023)) & 1023);
     unsigned char* Ws = base;
-    unsigned char* As = base + bf::kW;
+    unsigned char* As = base + (Two ? 2 : 1) * bf::kW;
     __shared__ uint64_t bar;
     __shared__ uint32_t tmem_slot;
     __shared__ float4 cs[2][kN64T / 32][16];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     bf::put_weights<false>(Ws, a.U);
+    if (Two) bf::put_weights<false>(Ws + bf::kW, a.M);
     if (threadIdx.x == 0) {
         tc::mbar_init(tc::smem_u32(&bar), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -400,19 +404,36 @@ __global__ void __launch_bounds__(kN64T, 2) k_node64(const Node64 a) {
     for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) bf::put(As, r0 + 32 * i, f, First ? in(x[i]) : x[i]);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        tc::fence_before();
-        __syncthreads();
-        tc::fence_after();
-        if (threadIdx.x == 0) {
-            const uint32_t as = tc::smem_u32(As), ws = tc::smem_u32(Ws);
+        const auto multiply = [&](int half) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            tc::fence_before();
+            __syncthreads();
+            tc::fence_after();
+            if (threadIdx.x == 0) {
+                const uint32_t as = tc::smem_u32(As), ws = tc::smem_u32(Ws) + half * bf::kW;
 #pragma unroll
-            for (int q = 2; q >= 0; --q)                       // the small parts first
+                for (int q = 2; q >= 0; --q)                   // the small parts first
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-                    bf::mma<bf::idesc(128, 64, false, false)>(tmem, tc::desc_sw128(as + q * bf::kPart + 32 * kk),
-                                                             tc::desc_sw128(ws + 32 * kk), (q == 2 && kk == 0) ? 0u : 1u);
-            tc::mma_commit(tc::smem_u32(&bar));
+                    for (int kk = 0; kk < 4; ++kk)
+                        bf::mma<bf::idesc(128, 64, false, false)>(tmem, tc::desc_sw128(as + q * bf::kPart + 32 * kk),
+                                                                 tc::desc_sw128(ws + 32 * kk),
+                                                                 (half == 0 && q == 2 && kk == 0) ? 0u : 1u);
+                tc::mma_commit(tc::smem_u32(&bar));
+            }
+        };
+        multiply(0);
+        if constexpr (Two) {                                   // the second input into the same accumulators
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int v = tile * 128 + r0 + 32 * i;
+                x[i] = v < nodes ? __ldg(reinterpret_cast<const float4*>(a.a) + (int64_t)v * 16 + f)
+                                 : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            if (!tc::mbar_wait(tc::smem_u32(&bar), parity)) ok = false;   // the operands are read
+            parity ^= 1u;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) bf::put(As, r0 + 32 * i, f, x[i]);
+            multiply(1);
         }
         // the edges' rows, while the MMAs run
         float4 y[4];
@@ -1475,6 +1496,9 @@ struct sps_gnn {
     sps_gnn_graph g{};
     sps_gnn_options opt{};
     int H = 64, L = 3, Fv = 1, Fc = 1, n = 0, m = 0, B = 1;
+    // H = 64: the route of forward64; the input layer of the variables' four features is
+    // recomputed where it is read (16 bytes a node instead of 256)
+    bool few_rows = false, in4 = false;
     int lpf = 0;                 // lp_features: inputs are scaled c and b, expanded on the device
     float *craw = nullptr, *braw = nullptr, *cmin = nullptr;
     int8_t* kind = nullptr;
@@ -1543,10 +1567,16 @@ size_t update_back_smem() { return sizeof(float) * (2 * H * H + 3 * kTile * (H +
 template <int H>
 int set_smem_attrs() {
     if constexpr (H == 64) {
-        for (auto k : {k_node64<false, false>, k_node64<false, true>, k_node64<true, false>, k_node64<true, true>})
-            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kNode64Smem) != cudaSuccess) return -2;
+        const auto size = [](auto k, int bytes) {
+            return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+        };
+        for (auto k : {k_node64<false, false, false>, k_node64<false, true, false>, k_node64<true, false, false>,
+                       k_node64<true, true, false>})
+            if (!size(k, node64_smem(false))) return -2;
+        for (auto k : {k_node64<false, false, true>, k_node64<false, true, true>})
+            if (!size(k, node64_smem(true))) return -2;
         for (auto k : {k_back64<false>, k_back64<true>})
-            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bk::kSmem) != cudaSuccess) return -2;
+            if (!size(k, bk::kSmem)) return -2;
         return 0;
     } else {
         if (cudaFuncSetAttribute(k_update<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)update_smem<H>()) !=
@@ -1584,7 +1614,9 @@ void agg_rows64(sps_gnn* g, const float* val, const float* in, bool first, float
     const float* b = g->P + g->obv;
     const int rows = g->m * batch;
     const bool long_rows = g->nnz >= 64 * (int64_t)g->m, block = long_rows && rows < 16384;
-    if (!first && !long_rows) {
+    // plain sums where rows are short, or so many beside the variables that one instance's
+    // fill the GPU (20 000 x 20 000 of 100 edges a row, predict 1.41 ms compensated)
+    if (!first && (!long_rows || (!g->few_rows && g->m >= 16 * 152))) {
         k_agg<64><<<grid_for((int64_t)rows * 32, kT), kT, 0, g->st>>>(g->cptr, g->cidx, val, in, out, g->m, g->n, batch,
                                                                      accumulate);
         return;
@@ -1595,49 +1627,74 @@ void agg_rows64(sps_gnn* g, const float* val, const float* in, bool first, float
                                                                          g->n, rows, accumulate);
 }
 
-template <bool First, bool Heads>
+template <bool First, bool Heads, bool Two = false>
 void node64(sps_gnn* g, const Node64& a) {
     const int64_t tiles = (a.nodes + 127) / 128;
-    k_node64<First, Heads><<<(int)std::min<int64_t>(tiles, 2 * 152), kN64T, kNode64Smem, g->st>>>(a);
+    k_node64<First, Heads, Two><<<(int)std::min<int64_t>(tiles, 2 * 152), kN64T, node64_smem(Two), g->st>>>(a);
 }
 
-// Forward pass, H = 64: M on the constraint side (k_node64).  keep: the variables'
-// last activations are stored too (the backward pass reads them).
+// Forward pass, H = 64.  keep: the variables' last activations are stored too (the
+// backward pass reads them).
+// M is applied on the constraint side (k_node64 with edges), and the constraints'
+// sums are compensated (k_con_update), where there are few rows for the variables and
+// their columns are short: edges per variable at most a quarter of the variables per
+// row (sps_gnn::few_rows).  Elsewhere both sides add up their neighbours first and
+// apply U and M in one pass (k_node64 with two inputs).  predict, ms, few rows' form
+// against the other: 500 x 60 000 of 2 edges a column, 16 instances 1.25 / 1.63; 400 x
+// 40 000 of 4 0.48 / 0.50, of 16 0.74 / 0.69; 8000 x 128 000 of 4 0.77 / 0.65 (its
+// gradient 1.62 / 1.79); 8000 x 40 000 of 13 0.64 / 0.44; 200 000 x 200 000 of 5 3.07 /
+// 0.93; 40 000 x 500 of 1570 4.4 / 0.90.
 int forward64(sps_gnn* g, int batch, bool keep) {
     const int n = g->n, m = g->m, L = g->L;
     const int64_t NV = (int64_t)n * batch, NC = (int64_t)m * batch;
     const __nv_bfloat16* W = g->PB;
     const float* P = g->P;
     cudaStream_t st = g->st;
-    // the input layer of four features is recomputed where it is read (16 bytes a node instead of 256)
-    const bool in4 = g->Fv == 4;
-    if (!in4) k_input<64><<<grid_for(NV * 64, kT), kT, 0, st>>>(g->fv, NV, g->Fv, W + g->oWv, P + g->obv, g->HV[0]);
+    const bool few = g->few_rows;
+    if (!g->in4) k_input<64><<<grid_for(NV * 64, kT), kT, 0, st>>>(g->fv, NV, g->Fv, W + g->oWv, P + g->obv, g->HV[0]);
     k_input<64><<<grid_for(NC * 64, kT), kT, 0, st>>>(g->fc, NC, g->Fc, W + g->oWc, P + g->obc, g->HC[0]);
     const bool heads = n >= 128;                  // a tile of 128 nodes then has at most two instances
     for (int l = 0; l < L; ++l) {
         const int64_t o = g->layer_off(l);
         const int64_t oUc = o, oMc = o + 4096, obc = o + 8192;
         const int64_t oUv = obc + 64, oMv = oUv + 4096, obv = oMv + 4096;
-        const bool first = l == 0 && in4, last = l == L - 1;
+        const bool first = l == 0 && g->in4, last = l == L - 1;
         agg_rows64(g, g->ac_c, first ? g->fv : g->HV[l], first, g->AC[l], batch, 0);
-        k_con_update<<<(int)((NC + kConNodes - 1) / kConNodes), kT, 0, st>>>(g->HC[l], g->AC[l], W + oUc, W + oMc,
-                                                                            P + obc, g->HC[l + 1], NC);
         Node64 p{};
-        p.h = g->HC[l + 1];
-        p.U = W + oMv;
-        p.out = g->MH;
         p.nodes = NC;
         p.err = g->d_err;
-        node64<false, false>(g, p);
+        if (few) {
+            k_con_update<<<(int)((NC + kConNodes - 1) / kConNodes), kT, 0, st>>>(g->HC[l], g->AC[l], W + oUc, W + oMc,
+                                                                                P + obc, g->HC[l + 1], NC);
+            p.h = g->HC[l + 1];
+            p.U = W + oMv;
+            p.out = g->MH;
+            node64<false, false>(g, p);
+        } else {
+            p.h = g->HC[l];
+            p.U = W + oUc;
+            p.a = g->AC[l];
+            p.M = W + oMc;
+            p.bias = P + obc;
+            p.out = g->HC[l + 1];
+            node64<false, false, true>(g, p);
+            // the aggregate passes through the backward pass's buffer
+            k_agg<64><<<grid_for(NV * 32, kT), kT, 0, st>>>(g->vptr, g->vidx, g->av_v, g->HC[l + 1], g->dHV2, n, m, batch, 0);
+        }
         Node64 a{};
         a.h = first ? g->fv : g->HV[l];
         a.Win = W + g->oWv;
         a.bin = P + g->obv;
         a.U = W + oUv;
-        a.P = g->MH;
-        a.ptr = g->vptr;
-        a.idx = g->vidx;
-        a.val = g->av_v;
+        if (few) {
+            a.P = g->MH;
+            a.ptr = g->vptr;
+            a.idx = g->vidx;
+            a.val = g->av_v;
+        } else {
+            a.a = g->dHV2;
+            a.M = W + oMv;
+        }
         a.n = n;
         a.rows = m;
         a.bias = P + obv;
@@ -1648,7 +1705,8 @@ int forward64(sps_gnn* g, int batch, bool keep) {
         a.x0 = g->x0;
         a.pool = g->pvp;
         a.err = g->d_err;
-        if (last && heads) { if (first) node64<true, true>(g, a); else node64<false, true>(g, a); }
+        if (!few) { if (last && heads) node64<false, true, true>(g, a); else node64<false, false, true>(g, a); }
+        else if (last && heads) { if (first) node64<true, true>(g, a); else node64<false, true>(g, a); }
         else { if (first) node64<true, false>(g, a); else node64<false, false>(g, a); }
     }
     k_head<64><<<grid_for(NC * 32, kT), kT, 0, st>>>(g->HC[L], W + g->oWy, P + g->oby, g->y0, NC);
@@ -1741,17 +1799,25 @@ int backward64(sps_gnn* g, int batch) {
     con.n = m;
     con.nodes = NC;
     con.err = g->d_err;
-    const bool in4 = g->Fv == 4;
+    const bool in4 = g->in4;
+    // rows of the constraint side's gradient are added along a variable's edges where it is
+    // read, or first: a tile's chain of edges outlasts the stream it saves from about eight
+    // edges a column on (gradient, along the edges / first: 200 000 x 200 000 of 5 2.92 /
+    // 2.83 ms, 500 x 60 000 of 2 4.60 / 4.79, 8000 x 40 000 of 13 1.15 / 1.08, 500 x 8000 of 31
+    // 0.58 / 0.52, 40 000 x 500 of 1570 4.3 / 1.9)
+    const bool edges = g->nnz < 8 * (int64_t)n;
     float *dhv = g->dHV, *dhc = g->dHC, *dhc_next = g->dHC2;
     for (int l = L - 1; l >= 0; --l) {
         const int64_t o = g->layer_off(l);
         const int64_t oUc = o, oMc = o + 4096, obc = o + 8192;
         const int64_t oUv = obc + 64, oMv = oUv + 4096, obv = oMv + 4096;
         const bool first = l == 0 && in4, last = l == L - 1;
+        if (!last && !edges)
+            k_agg<64><<<grid_for(NV * 32, kT), kT, 0, st>>>(g->vptr, g->vidx, g->ac_v, g->dA, dhv, n, m, batch, 1);
         // variable update: z, dh (in place of dout) and the gradients of Uv, bv (and of the x head)
         Back64 a = var;
         a.dout = last ? nullptr : dhv;
-        a.Q = last ? nullptr : g->dA;
+        a.Q = last || !edges ? nullptr : g->dA;
         a.dhead = g->dx0;
         a.whead = W + g->oWx;
         a.dlw = g->dlw;
@@ -1807,7 +1873,7 @@ int backward64(sps_gnn* g, int batch) {
     if (in4) {
         Back64 a = var;
         a.dout = dhv;
-        a.Q = g->dA;
+        a.Q = g->dA;                // (in4: short columns)
         a.h = g->fv;
         a.part = take(2 * 152, kInOut);
         k_in_back64<<<2 * 152, bk::kThreads, 0, st>>>(a);
@@ -2055,6 +2121,8 @@ int sps_gnn_create(const sps_gnn_graph* gr, const sps_gnn_options* opt_in, sps_g
     g->Fc = g->lpf ? 4 : gr->f_con;
     g->n = n; g->m = m; g->B = opt.max_batch; g->nnz = nnz;
     const int H = g->H;
+    g->few_rows = 4.0 * double(m) * double(nnz) <= double(n) * double(n);
+    g->in4 = H == 64 && g->Fv == 4 && g->few_rows;
     // parameter offsets
     int64_t o = 0;
     g->oWv = o; o += (int64_t)H * g->Fv; g->obv = o; o += H;
@@ -2117,9 +2185,9 @@ int sps_gnn_create(const sps_gnn_graph* gr, const sps_gnn_options* opt_in, sps_g
             }
             GNN_CK(g->alloc(&g->xt, NV)); GNN_CK(g->alloc(&g->yt, NC)); GNN_CK(g->alloc(&g->lt, B));
             g->HV.resize(g->L + 1); g->HC.resize(g->L + 1); g->AV.resize(g->L); g->AC.resize(g->L);
-            // (H = 64: the input layer of four features and the variables' aggregates are not stored)
+            // (H = 64: the variables' aggregates are not stored, nor an input layer that is recomputed)
             for (int l = 0; l <= g->L; ++l) {
-                if (l > 0 || H == 32 || g->Fv != 4) GNN_CK(g->alloc(&g->HV[l], NV * H));
+                if (l > 0 || !g->in4) GNN_CK(g->alloc(&g->HV[l], NV * H));
                 GNN_CK(g->alloc(&g->HC[l], NC * H));
             }
             for (int l = 0; l < g->L; ++l) {

@@ -1,7 +1,9 @@
 """Warm-start network on graphs that are not the transportation family: as many rows as
 columns, more rows than columns, long columns, short rows, many rows.  Outputs and
 gradient against the FP64 oracle with the tolerances of test_gpu_gnn_shapes; the same
-bits whatever the batch."""
+bits whatever the batch; and the time of such a graph against its transpose's."""
+
+import time
 
 import numpy as np
 import pytest
@@ -69,3 +71,29 @@ def test_same_bits_in_every_batch(m, n, per_row):
         for s in (0, 17, B - 1):
             x, y, _ = net.predict_features(fvs[s:s + 1], fcs[s:s + 1])
             assert np.array_equal(x[0], X[s]) and np.array_equal(y[0], Y[s])
+
+
+def test_many_rows_and_long_columns_keep_pace():
+    """40 000 rows of 20 edges on 500 columns (1600 edges each) against the transpose, the same
+    edges and nodes: 2 times its time (with the few rows' form 10 times)."""
+    def best(p):
+        with WarmStartGNN(p, layers=3, seed=1, max_batch=1) as net:
+            rng = np.random.default_rng(0)
+            f = lambda k: [rng.random((k, 1)).astype(np.float32)]                          # noqa: E731
+            fv, fc, xt, yt = f(net.n), f(net.m), [rng.random(net.n)], [rng.random(net.m)]
+            calls = (lambda: net.predict_features(fv, fc),
+                     lambda: net.loss_grad(fv, fc, xt, yt, np.zeros(1, np.float32)))
+            out = []
+            for call in calls:
+                ts = []
+                for _ in range(12):
+                    t = time.perf_counter()
+                    call()
+                    ts.append(time.perf_counter() - t)
+                out.append(min(ts[3:]))
+            return np.array(out)
+    p = _graph(40_000, 500, 20)
+    A = sp.vstack([p.A_ub, p.A_eq]).T.tocsr()
+    q = sps.Problem(c=np.ones(40_000), A_ub=A[:250], b_ub=np.ones(250), A_eq=A[250:], b_eq=np.ones(250),
+                    lb=np.zeros(40_000), ub=np.ones(40_000), integer_mask=np.zeros(40_000, bool))
+    assert (best(p) < 4 * best(q)).all()

@@ -328,7 +328,7 @@ struct Node64 {
     const float* a; const __nv_bfloat16* M;   // Two: the second input (nodes x 64) and its weights
     const float* P;                           // rows added along the edges (null: none)
     const int32_t *ptr, *idx; const float* val;   // edges of a node; rows of instance s at P + s * rows * 64
-    int n, rows;                              // nodes and rows of an instance
+    int n, rows;                              // nodes (at least 1: the kernel divides by it) and rows of an instance
     const float* bias;                        // null: neither bias nor ReLU
     float* out;                               // null: not stored
     int64_t nodes;
@@ -1633,6 +1633,15 @@ void node64(sps_gnn* g, const Node64& a) {
     k_node64<First, Heads, Two><<<(int)std::min<int64_t>(tiles, 2 * 152), kN64T, node64_smem(Two), g->st>>>(a);
 }
 
+// The arguments that every launch of k_node64 has: nodes of an instance, of the batch.
+Node64 node_args(const sps_gnn* g, int n, int64_t nodes) {
+    Node64 a{};
+    a.n = n;
+    a.nodes = nodes;
+    a.err = g->d_err;
+    return a;
+}
+
 // Forward pass, H = 64.  keep: the variables' last activations are stored too (the
 // backward pass reads them).
 // M is applied on the constraint side (k_node64 with edges), and the constraints'
@@ -1660,9 +1669,7 @@ int forward64(sps_gnn* g, int batch, bool keep) {
         const int64_t oUv = obc + 64, oMv = oUv + 4096, obv = oMv + 4096;
         const bool first = l == 0 && g->in4, last = l == L - 1;
         agg_rows64(g, g->ac_c, first ? g->fv : g->HV[l], first, g->AC[l], batch, 0);
-        Node64 p{};
-        p.nodes = NC;
-        p.err = g->d_err;
+        Node64 p = node_args(g, m, NC);
         if (few) {
             k_con_update<<<(int)((NC + kConNodes - 1) / kConNodes), kT, 0, st>>>(g->HC[l], g->AC[l], W + oUc, W + oMc,
                                                                                 P + obc, g->HC[l + 1], NC);
@@ -1681,7 +1688,7 @@ int forward64(sps_gnn* g, int batch, bool keep) {
             // the aggregate passes through the backward pass's buffer
             k_agg<64><<<grid_for(NV * 32, kT), kT, 0, st>>>(g->vptr, g->vidx, g->av_v, g->HC[l + 1], g->dHV2, n, m, batch, 0);
         }
-        Node64 a{};
+        Node64 a = node_args(g, n, NV);
         a.h = first ? g->fv : g->HV[l];
         a.Win = W + g->oWv;
         a.bin = P + g->obv;
@@ -1695,16 +1702,13 @@ int forward64(sps_gnn* g, int batch, bool keep) {
             a.a = g->dHV2;
             a.M = W + oMv;
         }
-        a.n = n;
         a.rows = m;
         a.bias = P + obv;
         a.out = last && heads && !keep ? nullptr : g->HV[l + 1];
-        a.nodes = NV;
         a.wx = W + g->oWx;
         a.bx = P + g->obx;
         a.x0 = g->x0;
         a.pool = g->pvp;
-        a.err = g->d_err;
         if (!few) { if (last && heads) node64<false, true, true>(g, a); else node64<false, false, true>(g, a); }
         else if (last && heads) { if (first) node64<true, true>(g, a); else node64<false, true>(g, a); }
         else { if (first) node64<true, false>(g, a); else node64<false, false>(g, a); }

@@ -1,0 +1,21 @@
+"""Rules of the kernels' sources that no run shows: operations that are undefined
+although today's compiler makes something harmless of them."""
+
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "sovereign-solver_gb300", "csrc")
+
+
+def _source(name):
+    src = open(os.path.join(CSRC, name)).read()
+    return re.sub(r"//[^\n]*", "", src)
+
+
+def test_node_map_has_its_divisor():
+    """k_node64 divides by the nodes of an instance: every launch's arguments come from
+    node_args, which sets them."""
+    src = _source("gnn.cu")
+    assert re.findall(r"Node64 \w+\{\};", src) == ["Node64 a{};"]
+    helper = src[src.index("Node64 node_args("):]
+    assert "a.n = n;" in helper[:helper.index("return a;")]

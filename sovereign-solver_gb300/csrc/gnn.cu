@@ -645,10 +645,10 @@ __global__ void __launch_bounds__(bk::kThreads, 2) k_back64(const Back64 a) {
         const int v0 = tile * 128 + r0;
         // z
         float4 z[4];
-        if (a.dout) {
+        if (a.dout) {           // plain loads: dh may take dout's place
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-                z[i] = v0 + 32 * i < nodes ? __ldg(reinterpret_cast<const float4*>(a.dout) + (int64_t)(v0 + 32 * i) * 16 + f)
+                z[i] = v0 + 32 * i < nodes ? reinterpret_cast<const float4*>(a.dout)[(int64_t)(v0 + 32 * i) * 16 + f]
                                            : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         if (a.Q || !a.dout) {

@@ -19,3 +19,11 @@ def test_node_map_has_its_divisor():
     assert re.findall(r"Node64 \w+\{\};", src) == ["Node64 a{};"]
     helper = src[src.index("Node64 node_args("):]
     assert "a.n = n;" in helper[:helper.index("return a;")]
+
+
+def test_gradient_in_place_is_read_with_plain_loads():
+    """k_back64 writes dh over dout: __ldg needs memory that the launch does not write."""
+    src = _source("gnn.cu")
+    body = src[src.index("k_back64(const Back64 a)"):src.index("k_in_back64(const Back64 a)")]
+    assert "a.dout)" in body
+    assert not re.search(r"__ldg\([^;]*a\.dout", body)

@@ -568,14 +568,15 @@ __global__ void __launch_bounds__(kN64T, 2) k_node64(const Node64 a) {
 // 128-node tile, rows of 128 bytes with the 128-byte swizzle: as the K-major A of
 // dh (M = nodes, K = 64 features, 16 per step), and as MN-major operands of dW
 // (K = nodes, 16 per step): A = [z1; z2] (M = 128: two parts one above the other), B =
-// [h1 | h2 | h3] (N = 192), and A = [z2; z3], B = h1 for z3 h1, whose accumulators take the
-// place of dh's once that is read.  z2 h2 and smaller products are below FP32.
-// The tensor core adds FP32 accumulators without rounding to nearest, so dW is
-// moved to registers and added there after every tile.
+// [h1 | h2 | h3] (N = 192), then A = [z2; z3] with B = h1, h2 and h3 in one set of
+// accumulators (only z3's rows are taken), which have dh's place once that is read:
+// all nine products, so nothing of z h is left out.  The tensor core adds FP32
+// accumulators without rounding to nearest, so dW is moved to registers and added
+// there after every tile.
 namespace bk {
 constexpr int kThreads = 512;
 constexpr int kSmem = bf::kW + 6 * bf::kPart + 1024;
-constexpr uint32_t kTmem = 256;               // columns: dW parts 0..191, dh then z3 h1 192..255
+constexpr uint32_t kTmem = 256;               // columns: dW parts 0..191, dh then z3 h 192..255
 constexpr int kOut = 64 * 64 + 64;            // a block's partial: dW, db
 constexpr int kHeadOut = 65;                  // dw, db of a head
 // MN-major operand, 128-byte swizzle: 64-element blocks `block` bytes apart, 8-row groups 1024
@@ -770,13 +771,16 @@ __global__ void __launch_bounds__(bk::kThreads, 2) k_back64(const Back64 a) {
         uint32_t dh[16];
         tc::tmem_ld16(tq + 192, dh);
         tc::fence_before();
-        ok = __syncthreads_and(ok) != 0;                        // dh read: its columns take z3 h1
+        ok = __syncthreads_and(ok) != 0;                        // dh read: its columns take z3 h
         tc::fence_after();
         if (threadIdx.x == 0 && ok) {
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk)
-                bf::mma<bf::idesc(128, 64, true, true)>(tmem + 192, bk::desc_mn(zs + bf::kPart + 2048 * kk, bf::kPart),
-                                                       bk::desc_mn(hs + 2048 * kk, bf::kPart), kk ? 1u : 0u);
+            for (int p = 2; p >= 0; --p)                       // the small parts first
+#pragma unroll
+                for (int kk = 0; kk < 8; ++kk)
+                    bf::mma<bf::idesc(128, 64, true, true)>(
+                        tmem + 192, bk::desc_mn(zs + bf::kPart + 2048 * kk, bf::kPart),
+                        bk::desc_mn(hs + p * bf::kPart + 2048 * kk, bf::kPart), (p == 2 && kk == 0) ? 0u : 1u);
             tc::mma_commit(tc::smem_u32(&bars[2]));
         }
         if (!ok) break;

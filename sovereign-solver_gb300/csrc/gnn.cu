@@ -267,22 +267,25 @@ __device__ __forceinline__ uint32_t upper(float a, float b) {
     return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
 }
 __device__ __forceinline__ float cut(float v) { return __uint_as_float(__float_as_uint(v) & 0xffff0000u); }
+template <bool Infinite>
 __device__ __forceinline__ void split(const float4& x, uint2 (&p)[3]) {
     float4 r = x;
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
         p[q] = make_uint2(upper(r.x, r.y), upper(r.z, r.w));
         if (q < 2) r = make_float4(r.x - cut(r.x), r.y - cut(r.y), r.z - cut(r.z), r.w - cut(r.w));
-        // an infinity is its own first part: inf - inf would make the sum of the parts NaN, and a ReLU 0 of that
-        if (q == 0 && !(fabsf(x.x) + fabsf(x.y) + fabsf(x.z) + fabsf(x.w) < INFINITY))
+        // Infinite: an infinity is its own first part.  inf - inf makes the sum of the parts NaN,
+        // and a ReLU makes 0 of that (gradients pass through none: they stay NaN)
+        if (Infinite && q == 0 && !(fabsf(x.x) + fabsf(x.y) + fabsf(x.z) + fabsf(x.w) < INFINITY))
             r = make_float4(isfinite(x.x) ? r.x : 0.f, isfinite(x.y) ? r.y : 0.f, isfinite(x.z) ? r.z : 0.f,
                             isfinite(x.w) ? r.w : 0.f);
     }
 }
 // piece f (four floats) of row r of a tile's parts
+template <bool Infinite>
 __device__ __forceinline__ void put(unsigned char* parts, int r, int f, const float4& x) {
     uint2 p[3];
-    split(x, p);
+    split<Infinite>(x, p);
     const int off = r * 128 + (((f >> 1) ^ (r & 7)) << 4) + ((f & 1) << 3);
 #pragma unroll
     for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(parts + q * kPart + off) = p[q];
@@ -403,7 +406,7 @@ __global__ void __launch_bounds__(kN64T, 2) k_node64(const Node64 a) {
     if (blockIdx.x < tiles) fetch(blockIdx.x);
     for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) bf::put(As, r0 + 32 * i, f, First ? in(x[i]) : x[i]);
+        for (int i = 0; i < 4; ++i) bf::put<true>(As, r0 + 32 * i, f, First ? in(x[i]) : x[i]);
         const auto multiply = [&](int half) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             tc::fence_before();
@@ -432,7 +435,7 @@ __global__ void __launch_bounds__(kN64T, 2) k_node64(const Node64 a) {
             if (!tc::mbar_wait(tc::smem_u32(&bar), parity)) ok = false;   // the operands are read
             parity ^= 1u;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) bf::put(As, r0 + 32 * i, f, x[i]);
+            for (int i = 0; i < 4; ++i) bf::put<true>(As, r0 + 32 * i, f, x[i]);
             multiply(1);
         }
         // the edges' rows, while the MMAs run
@@ -726,7 +729,7 @@ __global__ void __launch_bounds__(bk::kThreads, 2) k_back64(const Back64 a) {
             zsum.y += z[i].y;
             zsum.z += z[i].z;
             zsum.w += z[i].w;
-            bf::put(Zs, r0 + 32 * i, f, z[i]);
+            bf::put<false>(Zs, r0 + 32 * i, f, z[i]);
         }
         // h
         if constexpr (First) {
@@ -735,7 +738,7 @@ __global__ void __launch_bounds__(bk::kThreads, 2) k_back64(const Back64 a) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int v = v0 + 32 * i;
-                bf::put(Hs, r0 + 32 * i, f, v < nodes ? in(__ldg(reinterpret_cast<const float4*>(a.h) + v))
+                bf::put<false>(Hs, r0 + 32 * i, f, v < nodes ? in(__ldg(reinterpret_cast<const float4*>(a.h) + v))
                                                      : make_float4(0.f, 0.f, 0.f, 0.f));
             }
         } else {
@@ -745,7 +748,7 @@ __global__ void __launch_bounds__(bk::kThreads, 2) k_back64(const Back64 a) {
                 x[i] = v0 + 32 * i < nodes ? __ldg(reinterpret_cast<const float4*>(a.h) + (int64_t)(v0 + 32 * i) * 16 + f)
                                            : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) bf::put(Hs, r0 + 32 * i, f, x[i]);
+            for (int i = 0; i < 4; ++i) bf::put<false>(Hs, r0 + 32 * i, f, x[i]);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         tc::fence_before();

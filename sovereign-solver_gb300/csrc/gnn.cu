@@ -407,12 +407,13 @@ __global__ void __launch_bounds__(kN64T, 2) k_node64(const Node64 a) {
     for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) bf::put<true>(As, r0 + 32 * i, f, First ? in(x[i]) : x[i]);
+        bool second = true;                                    // Two: thread 0 issues the second product
         const auto multiply = [&](int half) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             tc::fence_before();
             __syncthreads();
             tc::fence_after();
-            if (threadIdx.x == 0) {
+            if (threadIdx.x == 0 && second) {
                 const uint32_t as = tc::smem_u32(As), ws = tc::smem_u32(Ws) + half * bf::kW;
 #pragma unroll
                 for (int q = 2; q >= 0; --q)                   // the small parts first
@@ -433,6 +434,7 @@ __global__ void __launch_bounds__(kN64T, 2) k_node64(const Node64 a) {
                                  : make_float4(0.f, 0.f, 0.f, 0.f);
             }
             if (!tc::mbar_wait(tc::smem_u32(&bar), parity)) ok = false;   // the operands are read
+            second = ok;
             parity ^= 1u;
 #pragma unroll
             for (int i = 0; i < 4; ++i) bf::put<true>(As, r0 + 32 * i, f, x[i]);
@@ -549,6 +551,8 @@ __global__ void __launch_bounds__(kN64T, 2) k_node64(const Node64 a) {
         tc::fence_before();
         ok = __syncthreads_and(ok) != 0;                       // shared and tensor memory free for the next tile
         tc::fence_after();
+        if (!ok && threadIdx.x == 0)                           // giving up: a last wait for what is in flight
+            tc::mbar_wait(tc::smem_u32(&bar), second ? parity ^ 1u : parity);
     }
     if (!ok && threadIdx.x == 0) atomicExch(a.err, 1);
     __syncthreads();
@@ -786,7 +790,11 @@ __global__ void __launch_bounds__(bk::kThreads, 2) k_back64(const Back64 a) {
                         bk::desc_mn(hs + p * bf::kPart + 2048 * kk, bf::kPart), (p == 2 && kk == 0) ? 0u : 1u);
             tc::mma_commit(tc::smem_u32(&bars[2]));
         }
-        if (!ok) break;
+        if (!ok) {                                              // giving up: a last wait for what is in flight
+            if (threadIdx.x == 0)
+                for (int q = 0; q < 2; ++q) tc::mbar_wait(tc::smem_u32(&bars[q]), parity);
+            break;
+        }
         if (!tc::mbar_wait(tc::smem_u32(&bars[1]), parity)) ok = false;
         tc::fence_after();
         uint32_t q[16];
@@ -812,6 +820,8 @@ __global__ void __launch_bounds__(bk::kThreads, 2) k_back64(const Back64 a) {
         tc::fence_before();
         ok = __syncthreads_and(ok) != 0;
         tc::fence_after();
+        if (!ok && threadIdx.x == 0)
+            for (int q = 1; q < 3; ++q) tc::mbar_wait(tc::smem_u32(&bars[q]), parity ^ 1u);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int row = r0 + 32 * i, v = v0 + 32 * i;

@@ -47,16 +47,17 @@ struct Gather1 {
 __device__ __forceinline__ float ld_vec(const float* p, bool coh) { return coh ? __ldcg(p) : __ldg(p); }
 
 // The block's dynamic shared memory: the check's partial slots, which the
-// steps use as the staging buffer.
-extern __shared__ double s_slots[];
-#define s_stage reinterpret_cast<float*>(s_slots)
+// steps use as the staging buffer, then the ring of the sliced passes (16-byte copies).
+extern __shared__ __align__(16) double s_slots[];
+static_assert(sizeof(double) * kColPartials * kBlock % 16 == 0, "the ring follows the slots on a 16-byte boundary");
+__device__ __forceinline__ float* s_stage() { return reinterpret_cast<float*>(s_slots); }
 
 // Gathers of the FP32 steps from a copy of the vector in shared memory (when
 // it fits the 7168-float staging buffer): an instance's gathers are random,
 // one 32-byte L1 sector (one L1 wavefront) per nonzero even on an L1 hit,
 // while a warp's 32 random shared-memory reads cost a few bank cycles.
 struct GatherS {
-    __device__ __forceinline__ float operator()(int, int j) const { return s_stage[j]; }
+    __device__ __forceinline__ float operator()(int, int j) const { return s_stage()[j]; }
 };
 
 // Copy x[0, n) into the staging buffer (coherent loads in a team, where other
@@ -513,7 +514,7 @@ __device__ __forceinline__ bool solve_one(const Args& A, int k, int G, Ctl& c, d
     float* smf = reinterpret_cast<float*>(sm);
     const Handoff H{A.idle, A.idle_need, A.handoff_nnz > 0 && I.nnz >= A.handoff_nnz};
     // the staging buffer shares its memory with the check's partial slots
-    float* const stage = s_stage;
+    float* const stage = s_stage();
     const bool stage_x = v.n <= A.stage_cap, stage_y = v.m <= A.stage_cap;
     if (threadIdx.x == 0) {
         c.t_begin = t_begin;

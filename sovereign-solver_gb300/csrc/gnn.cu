@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(kT, 2) k_update(const float* __restrict__ h, c
                                                   int64_t nodes) {
     static_assert(H % 32 == 0 && kT == 256, "thread layout: 8 output groups x 32 node groups");
     constexpr int K2 = 2 * H, S = upd_stride<H>(), J = H / 32;
-    extern __shared__ float sm[];
+    extern __shared__ __align__(16) float sm[];
     float* Wt = sm;                           // [k][o], k < H from U, k >= H from M
     float* X = Wt + K2 * H;                   // [node][S]: h (k < H) then a
     for (int t = threadIdx.x; t < K2 * H; t += kT) {
@@ -1286,7 +1286,7 @@ __global__ void __launch_bounds__(kT) k_update_back(const float* __restrict__ do
     constexpr int ZS = H + 1;
     constexpr int WO = kT / 4 >= H ? 1 : H / (kT / 4);         // weight rows per thread
     constexpr int WK = H / 4;                                  // weight columns per thread
-    extern __shared__ float sm[];
+    extern __shared__ __align__(16) float sm[];
     float* Us = sm;                 // [o][k]
     float* Ms = Us + H * H;
     float* Z = Ms + H * H;          // dz tile [kTile][ZS]

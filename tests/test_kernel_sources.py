@@ -27,3 +27,10 @@ def test_gradient_in_place_is_read_with_plain_loads():
     body = src[src.index("k_back64(const Back64 a)"):src.index("k_in_back64(const Back64 a)")]
     assert "a.dout)" in body
     assert not re.search(r"__ldg\([^;]*a\.dout", body)
+
+
+def test_copied_to_shared_memory_is_aligned():
+    """16-byte copies and reads (the sliced passes' ring): every dynamic shared array says so."""
+    for name in sorted(os.listdir(CSRC)):
+        for line in re.findall(r"extern __shared__[^;]*;", _source(name)):
+            assert "__align__(16)" in line, (name, line)

@@ -267,6 +267,12 @@ int sps_batch_set_warm_starts(sps_batch *b, const double *x0, const double *y0, 
  * res->solve_ms is the instance's own device time inside the persistent launch
  * (plus its FP64 continuation, if any); setup_ms is the batch's. */
 int sps_batch_get(sps_batch *b, int32_t k, double *x, double *y, sps_result *res);
+/* Give back the device memory of the batch's second layout of its matrices (about 18
+ * bytes per nonzero and side, made by sps_batch_create where it speeds the solves up and
+ * takes at most half of the free memory): later solves walk the first one, slower, with
+ * the same results bit for bit.  Returns 1, or 0 if the batch has none.  The library does
+ * so itself where warm starts or a continuation do not fit beside it. */
+int sps_batch_release_slices(sps_batch *b);
 const char *sps_batch_last_error(const sps_batch *b);
 void sps_batch_destroy(sps_batch *b);
 

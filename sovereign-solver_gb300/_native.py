@@ -137,6 +137,7 @@ def load() -> C.CDLL:
         "sps_batch_solve": (C.c_int, [H, C.POINTER(BatchStats)]),
         "sps_batch_get": (C.c_int, [H, C.c_int32, _f64p, _f64p, C.POINTER(Result)]),
         "sps_batch_set_warm_starts": (C.c_int, [H, _f64p, _f64p, _f64p]),
+        "sps_batch_release_slices": (C.c_int, [H]),
         "sps_batch_last_error": (C.c_char_p, [H]),
         "sps_batch_destroy": (None, [H]),
         "sps_gnn_options_init": (C.c_int, [C.POINTER(GnnOptions)]),

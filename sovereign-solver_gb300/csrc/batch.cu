@@ -965,6 +965,8 @@ struct sps_batch {
     std::vector<Inst> inst;
     std::vector<int32_t> order;
     std::vector<void*> dev;                 // device allocations
+    std::vector<void*> slice_dev;           // the slices' (release_slices gives them back early)
+    std::mutex slice_mu;                    // taken by the continuations' threads
     Inst* d_inst = nullptr;
     int32_t* d_order = nullptr;
     Ctl* d_out = nullptr;
@@ -995,17 +997,50 @@ struct sps_batch {
     ~sps_batch() {
         if (gexec) cudaGraphExecDestroy(gexec);
         for (void* p : dev) cudaFree(p);
+        for (void* p : slice_dev) cudaFree(p);
         if (e0) cudaEventDestroy(e0);
         if (e1) cudaEventDestroy(e1);
         if (st) cudaStreamDestroy(st);
     }
     template <class T>
-    cudaError_t alloc(T** p, size_t count_) {
+    cudaError_t alloc(T** p, size_t count_, std::vector<void*>* keep = nullptr) {
         void* q = nullptr;
         const cudaError_t e = cudaMalloc(&q, std::max<size_t>(count_, 1) * sizeof(T));
-        if (e == cudaSuccess) dev.push_back(q);
+        if (e == cudaSuccess) (keep ? keep : &dev)->push_back(q);
         *p = static_cast<T*>(q);
         return e;
+    }
+    // The slices' memory back (the passes walk the CSR from now on: the same bits); false
+    // if there are none.  Not while a solve's launch runs.
+    bool release_slices() {
+        if (slice_dev.empty()) return false;
+        cudaStreamSynchronize(st);
+        for (void* p : slice_dev) cudaFree(p);
+        slice_dev.clear();
+        arr.slice = nullptr;
+        arr.soff = nullptr;
+        arr.pts = nullptr;
+        arr.steps = nullptr;
+        if (gexec) cudaGraphExecDestroy(gexec);            // captured with the sliced kernel
+        gexec = nullptr;
+        return true;
+    }
+    // Device memory of the warm starts, in one piece; where it does not fit beside the
+    // slices, they go.
+    cudaError_t alloc_warm() {
+        if (d_wx) return cudaSuccess;
+        double* p = nullptr;
+        const size_t need = (size_t)sum_n + (size_t)sum_m + (size_t)count;
+        cudaError_t e = alloc(&p, need);
+        if (e == cudaErrorMemoryAllocation && release_slices()) {
+            cudaGetLastError();
+            e = alloc(&p, need);
+        }
+        if (e != cudaSuccess) return e;
+        d_wx = p;
+        d_wy = d_wx + sum_n;
+        d_wom = d_wy + sum_m;
+        return cudaSuccess;
     }
     int fail(int code, const std::string& m) {
         err = m;
@@ -1094,6 +1129,13 @@ int continue_single(sps_batch* b, int32_t k, double used_s, std::string* why) {
     o.time_limit_s = b->opt.time_limit_s > 0 ? b->opt.time_limit_s - used_s : 0.0;
     sps_handle* h = nullptr;
     int rc = sps_create(&d, &o, &h);
+    if (rc == SPS_ERR_OOM) {              // the launch is over: its slices' memory may be what is missing
+        {
+            std::lock_guard<std::mutex> lk(b->slice_mu);
+            b->release_slices();
+        }
+        rc = sps_create(&d, &o, &h);
+    }
     if (rc != SPS_OK) {
         *why = "instance " + std::to_string(k) + what + sps_last_error(nullptr);
         return rc;
@@ -1135,7 +1177,8 @@ int continue_single(sps_batch* b, int32_t k, double used_s, std::string* why) {
 // the batch runs on its CSR if more than a quarter of its entries would.  With one
 // block on an SM short columns gain too (children with four entries per column:
 // 33.4 ms on the CSR, 18.9 on slices).  Without memory for the slices, or clusters
-// for the teams, the batch runs on the CSR.
+// for the teams, the batch runs on the CSR; what else the batch needs memory for later
+// takes theirs (release_slices).
 int build_slices(sps_batch* b) {
     const int32_t count = b->count;
     std::vector<sps::batch::Slice> sl(count);
@@ -1174,12 +1217,14 @@ int build_slices(sps_batch* b) {
     sps::batch::Slice* d_slice = nullptr;
     int32_t* d_off = nullptr;
     uint4* d_steps = nullptr;
-    double2* d_pts = nullptr;
     std::vector<int32_t> off(chunks);
-    if (b->alloc(&d_slice, count) != cudaSuccess || b->alloc(&d_off, chunks) != cudaSuccess) {
+    const auto on_csr = [&] {
+        b->release_slices();
         cudaGetLastError();
         return SPS_OK;
-    }
+    };
+    if (b->alloc(&d_slice, count, &b->slice_dev) != cudaSuccess || b->alloc(&d_off, chunks, &b->slice_dev) != cudaSuccess)
+        return on_csr();
     SPB_CK(cudaMemcpyAsync(d_slice, sl.data(), sizeof(sl[0]) * count, cudaMemcpyHostToDevice, b->st));
     sps::batch::k_slice_count<<<dim3(count, 2), sps::kBlock, 0, b->st>>>(b->d_inst, d_slice, b->arr, b->G, b->Gr, d_off);
     SPB_CK(cudaGetLastError());
@@ -1200,12 +1245,16 @@ int build_slices(sps_batch* b) {
         if (row) { sl[k].rstep = steps; steps += rs; }
         if (col) { sl[k].cstep = steps; steps += cs; }
     }
-    if (steps == 0 || 4 * left > entries) return SPS_OK;
-    if (b->alloc(&d_steps, steps * 64) != cudaSuccess ||
-        b->alloc(&d_pts, (size_t)(b->sum_n + b->sum_m)) != cudaSuccess) {
-        cudaGetLastError();
-        return SPS_OK;
-    }
+    if (steps == 0 || 4 * left > entries) return on_csr();
+    // in one piece, the steps (1 KB each) then the points of a check, and at most half of
+    // what is free: other handles of the caller need memory too
+    static_assert(sizeof(double2) == sizeof(uint4), "both parts in units of 16 bytes");
+    const size_t need = (size_t)steps * 64 + (size_t)(b->sum_n + b->sum_m);
+    size_t free_bytes = 0, total_bytes = 0;
+    if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess || need > free_bytes / (2 * sizeof(uint4)) ||
+        b->alloc(&d_steps, need, &b->slice_dev) != cudaSuccess)
+        return on_csr();
+    double2* d_pts = reinterpret_cast<double2*>(d_steps + steps * 64);
     SPB_CK(cudaMemcpyAsync(d_slice, sl.data(), sizeof(sl[0]) * count, cudaMemcpyHostToDevice, b->st));
     sps::batch::k_slice_fill<<<dim3(count, 2), sps::kBlock, 0, b->st>>>(b->d_inst, d_slice, b->arr, b->G, b->Gr, d_off,
                                                                          d_steps);
@@ -1729,6 +1778,12 @@ extern "C" int sps_batch_solve(sps_batch* b, sps_batch_stats* stats) {
     return SPS_OK;
 }
 
+extern "C" int sps_batch_release_slices(sps_batch* b) {
+    if (!b) return SPS_ERR_INVALID;
+    SPB_CK(cudaSetDevice(b->opt.device));
+    return b->release_slices() ? 1 : 0;
+}
+
 extern "C" int sps_batch_set_warm_starts(sps_batch* b, const double* x0, const double* y0, const double* omega0) {
     if (!b) return SPS_ERR_INVALID;
     if (!x0 && !y0) {
@@ -1737,11 +1792,7 @@ extern "C" int sps_batch_set_warm_starts(sps_batch* b, const double* x0, const d
     }
     if (b->opt.mode != SPS_MODE_ADAPTIVE) return b->fail(SPS_ERR_STATE, "warm starts need the adaptive mode");
     SPB_CK(cudaSetDevice(b->opt.device));
-    if (!b->d_wx) {
-        SPB_CK(b->alloc(&b->d_wx, b->sum_n));
-        SPB_CK(b->alloc(&b->d_wy, b->sum_m));
-        SPB_CK(b->alloc(&b->d_wom, b->count));
-    }
+    SPB_CK(b->alloc_warm());
     auto finite = [](const double* v, int64_t len) {
         for (int64_t t = 0; t < len; ++t)
             if (!std::isfinite(v[t])) return false;
@@ -1777,11 +1828,7 @@ extern "C" int sps_batch_set_warm_starts_gnn(sps_batch* b, sps_gnn* g, const dou
         if (b->inst[k].n != io.n || b->inst[k].m != io.m)
             return b->fail(SPS_ERR_INVALID, "instance " + std::to_string(k) + " does not have the network's shape");
     SPB_CK(cudaSetDevice(b->opt.device));
-    if (!b->d_wx) {
-        SPB_CK(b->alloc(&b->d_wx, b->sum_n));
-        SPB_CK(b->alloc(&b->d_wy, b->sum_m));
-        SPB_CK(b->alloc(&b->d_wom, b->count));
-    }
+    SPB_CK(b->alloc_warm());
     for (int32_t s0 = 0; s0 < b->count; s0 += io.max_batch) {
         const int cnt = std::min<int32_t>(io.max_batch, b->count - s0);
         const int64_t work = (int64_t)cnt * std::max(io.n, io.m);

@@ -1,0 +1,57 @@
+"""The two layouts of a batch's matrices give the same bits: every case solves with the
+slices, gives them back (which says whether there were any) and solves on the CSR."""
+
+import numpy as np
+import pytest
+
+import sovereign_solver_gb300 as sps
+import sovereign_solver_gb300.workloads as wl
+from test_gpu_batch_slices import TOL, _shapes
+
+pytestmark = pytest.mark.gpu
+
+
+def _both(b, slices=True):
+    got = [b.solve()]
+    assert b.lib.sps_batch_release_slices(b.h) == (1 if slices else 0)
+    assert b.lib.sps_batch_release_slices(b.h) == 0
+    got.append(b.solve())
+    for r, q in zip(*got):
+        assert (r.status, r.iterations, r.rel_kkt, r.objective) == (q.status, q.iterations, q.rel_kkt, q.objective)
+        assert np.array_equal(r.x, q.x) and np.array_equal(r.y, q.y)
+    return got[0]
+
+
+@pytest.mark.parametrize("group", [1, 2, 8, 32])
+@pytest.mark.parametrize("graph_mode", [0, 2])
+def test_edges(group, graph_mode):
+    with sps.PDHGBatch(_shapes(), tol=TOL, max_iters=20000, batch_group=group, escalate="off",
+                       graph_mode=graph_mode) as b:
+        _both(b)
+
+
+@pytest.mark.parametrize("team", [2, 4, 8])
+def test_teams(team):
+    probs = [wl.batch_planted_lp(k, m_range=(60, 300))[0] for k in range(12)]
+    with sps.PDHGBatch(probs, tol=TOL, max_iters=20000, batch_team=team, batch_team_nnz=2000, escalate="off") as b:
+        _both(b)
+        assert b.stats.team == team
+
+
+@pytest.mark.parametrize("kind", ["planted", "two_entry_columns", "mixed"])
+def test_more_instances_than_sms(kind):
+    planted = [wl.batch_planted_lp(k, m_range=(40, 90))[0] for k in range(200)]
+    short = [wl.transportation_lp(5 + k % 7, 9 + k % 5, seed=k)[0] for k in range(200)]
+    probs = {"planted": planted, "two_entry_columns": short, "mixed": planted + short}[kind]
+    with sps.PDHGBatch(probs, tol=TOL, max_iters=2000, escalate="off") as b:
+        _both(b, slices=kind != "two_entry_columns")
+
+
+def test_warm_starts():
+    """The cold starts' errors are kept by the first solve, and the warm points are judged by them in both."""
+    probs = [wl.batch_planted_lp(k, m_range=(60, 200))[0] for k in range(24)]
+    with sps.PDHGBatch(probs, tol=TOL, max_iters=20000, escalate="off") as b:
+        cold = b.solve()
+        b.set_warm_starts([(r.x, r.y, None) for r in cold])
+        warm = _both(b)
+        assert sum(r.iterations for r in warm) < sum(r.iterations for r in cold) / 2

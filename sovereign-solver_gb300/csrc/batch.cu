@@ -69,9 +69,12 @@ __device__ __forceinline__ void stage_vector(float* s, const float* x, int n, bo
     __syncthreads();
 }
 
+// The average point, l + s / w, with one rounding.  Written out, here and in the steps
+// below: the compiler contracts a * b + c one way in one form of the solve and another
+// in the next, and both forms have to give the same bits.
+__device__ __forceinline__ double avg(float s, float l, double inv_w) { return __fma_rn(double(s), inv_w, double(l)); }
 __device__ __forceinline__ double avg_at(const float* s, const float* l, double inv_w, int j, bool coh = false) {
-    const double v = double(ld_vec(s + j, coh)) * inv_w;
-    return l ? v + double(ld_vec(l + j, coh)) : v;
+    return avg(ld_vec(s + j, coh), l ? ld_vec(l + j, coh) : 0.f, inv_w);
 }
 
 struct Gather2 {
@@ -112,12 +115,12 @@ struct RowStepE {
     __device__ __forceinline__ void operator()(int r, const float (&acc)[1], const Pre& p) {
         const float ax = acc[0];
         axn[r] = ax;
-        float y2 = p.yv + sigma * (p.br - (ax + ax - p.ao));
+        float y2 = __fmaf_rn(sigma, p.br - (ax + ax - p.ao), p.yv);
         if (p.kd) y2 = fminf(y2, 0.f);
         yn[r] = y2;
         const float dy = y2 - p.yv;
-        dy2 += dy * dy;
-        inter += dy * (ax - p.ao);
+        dy2 = __fmaf_rn(dy, dy, dy2);
+        inter = __fmaf_rn(dy, ax - p.ao, inter);
     }
 };
 
@@ -131,11 +134,11 @@ struct ColStepE {
     __device__ __forceinline__ Pre pre(int j) const { return Pre{xc[j], c[j], lo[j], hi[j], xs[j], xl[j]}; }
     __device__ __forceinline__ void operator()(int j, const float (&acc)[1], const Pre& p) {
         aty[j] = acc[0];
-        xs[j] = p.s + wgt * (p.xj - p.r);
-        const float x2 = fminf(fmaxf(p.xj - tau * (p.cj - acc[0]), p.l), p.h);
+        xs[j] = __fmaf_rn(wgt, p.xj - p.r, p.s);
+        const float x2 = fminf(fmaxf(__fmaf_rn(-tau, p.cj - acc[0], p.xj), p.l), p.h);
         xn[j] = x2;
         const float d = x2 - p.xj;
-        dx2 += d * d;
+        dx2 = __fmaf_rn(d, d, dx2);
     }
 };
 
@@ -381,10 +384,10 @@ __device__ __noinline__ bool check_and_apply(const View& v, const Inst& I, Ctl& 
     const float tau = block_scalar<float>([&] { return c.eta / c.omega; });
     float dx2 = 0.f;
     TEAM_OWNED(j, v.n, chc) {
-        if (save) v.xb[j] = save_avg ? float(double(v.xl[j]) + double(v.xs[j]) * iw) : v.X[cur][j];
+        if (save) v.xb[j] = save_avg ? float(avg(v.xs[j], v.xl[j], iw)) : v.X[cur][j];
         float xv;
         if (load) {
-            xv = float(double(v.xl[j]) + double(v.xs[j]) * iw);
+            xv = float(avg(v.xs[j], v.xl[j], iw));
             v.X[cur][j] = xv;
             v.ATY[cur][j] = v.atya[j];
         } else {
@@ -396,16 +399,16 @@ __device__ __noinline__ bool check_and_apply(const View& v, const Inst& I, Ctl& 
             v.atyl[j] = v.ATY[cur][j];
         }
         if (cand) {
-            const float x2 = fminf(fmaxf(xv - tau * (v.c[j] - v.ATY[cur][j]), v.lo[j]), v.hi[j]);
+            const float x2 = fminf(fmaxf(__fmaf_rn(-tau, v.c[j] - v.ATY[cur][j], xv), v.lo[j]), v.hi[j]);
             v.X[1 - cur][j] = x2;
-            dx2 += (x2 - xv) * (x2 - xv);
+            dx2 = __fmaf_rn(x2 - xv, x2 - xv, dx2);
         }
     }
     TEAM_OWNED(i, v.m, chr) {
-        if (save) v.yb[i] = save_avg ? float(double(v.yl[i]) + double(v.ys[i]) * iw) : v.Y[cur][i];
+        if (save) v.yb[i] = save_avg ? float(avg(v.ys[i], v.yl[i], iw)) : v.Y[cur][i];
         float yv;
         if (load) {
-            yv = float(double(v.yl[i]) + double(v.ys[i]) * iw);
+            yv = float(avg(v.ys[i], v.yl[i], iw));
             v.Y[cur][i] = yv;
             v.AX[cur][i] = v.axa[i];
         } else {
@@ -556,14 +559,14 @@ __device__ __forceinline__ bool solve_one(const Args& A, int k, int G, Ctl& c, d
                     col_pass<Sliced, 1, float>(v, Gather1{v.Y[cur], T.size > 1}, ec, T);
                 }
                 dx2 = ec.dx2;
-                TEAM_OWNED(i, v.m, chr) v.ys[i] += wgt * (v.Y[cur][i] - v.yl[i]);
+                TEAM_OWNED(i, v.m, chr) v.ys[i] = __fmaf_rn(wgt, v.Y[cur][i] - v.yl[i], v.ys[i]);
             } else {
                 dx2 = 0.f;
                 TEAM_OWNED(j, v.n, chc) {
                     const float xj = v.X[cur][j];
-                    const float x2 = fminf(fmaxf(xj - tau * (v.c[j] - v.ATY[cur][j]), v.lo[j]), v.hi[j]);
+                    const float x2 = fminf(fmaxf(__fmaf_rn(-tau, v.c[j] - v.ATY[cur][j], xj), v.lo[j]), v.hi[j]);
                     v.X[1 - cur][j] = x2;
-                    dx2 += (x2 - xj) * (x2 - xj);
+                    dx2 = __fmaf_rn(x2 - xj, x2 - xj, dx2);
                 }
             }
             float f1[1] = {dx2};

@@ -112,7 +112,8 @@ typedef struct {
     int32_t batch_team;       /* batched solver: blocks (one thread-block cluster) per large
                                  instance, 1..8; 1 = one block per instance; 0 = 4, or in a
                                  batch of fewer instances than half the resident blocks the
-                                 largest of 2, 4, 8 that keeps every instance resident */
+                                 largest of 2, 4, 8 that keeps every instance resident at
+                                 four blocks an SM */
     int32_t batch_team_nnz;   /* batched solver: instances with at least this many nonzeros are
                                  large; 0 = 65536 in such a small batch, else the larger of
                                  65536 and twice the median instance */

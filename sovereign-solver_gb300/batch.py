@@ -29,7 +29,8 @@ class PDHGBatch:
     The lanes per row of the row pass (4, 8, 16, 32) are always timed.
     ``batch_team``: blocks (a thread-block cluster) per large instance, 1 = one
     block per instance, 0 = 4 (or, in a batch of fewer instances than half the
-    resident blocks, the largest of 2, 4, 8 that keeps them all resident);
+    resident blocks, the largest of 2, 4, 8 that keeps them all resident at four
+    blocks an SM);
     ``batch_team_nnz``: nonzeros from which an instance is large (0 = 65 536 in
     such a small batch, else the larger of 65 536 and twice the median).
     ``escalate``: "fp64" (FP64 continuation of stalled instances), "stop"

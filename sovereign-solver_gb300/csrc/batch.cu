@@ -608,9 +608,8 @@ __device__ __forceinline__ bool solve_one(const Args& A, int k, int G, Ctl& c, d
 // a 200 x 2000 node: 20.5 ms with two, 18.9 now; 640 LPs at their start, before
 // the small ones end, 15.0 ms for 192 attempts with two and 18.3 with one).  The
 // other form, four blocks and no ring, times the schedules, since the schedule
-// fixes the order of the sums, and serves a batch without slices.  The grid is
-// the four-block one for all: its blocks past the resident ones start when others
-// end.
+// fixes the order of the sums, and serves a batch without slices.  A launch has the
+// blocks that are resident at once, in whole clusters where it has teams.
 template <bool Sliced, int PerSm>
 __global__ void __launch_bounds__(kBlock, PerSm) k_batch_solve(Args A, int G) {
     __shared__ Ctl c;
@@ -956,6 +955,7 @@ struct sps_batch {
     int32_t G = 0, Gr = 0, blocks = 0;       // lanes per column / per row, persistent blocks
     int32_t stage_cap = 0;                    // floats of the kernel's shared staging buffer
     void (*sliced_kernel)(sps::batch::Args, int) = nullptr;   // the form of the solve for a batch with slices
+    int32_t sliced_blocks = 0;                // its blocks: those of `blocks` that are resident at once
     size_t dyn_smem = 0;                      // dynamic shared memory of the solve launch
     int32_t team = 1;                         // cluster size of the solve launch
     int32_t team_nnz = 65536;                 // instances at least this large are solved by a team
@@ -1197,26 +1197,47 @@ int build_slices(sps_batch* b) {
     const int smem = (int)b->dyn_smem + sps::batch::kRingBytes;
     int sms = 152;
     SPB_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->opt.device));
-    b->sliced_kernel = b->blocks <= sms ? sps::batch::k_batch_solve<true, 1> : sps::batch::k_batch_solve<true, 2>;
-    SPB_CK(cudaFuncSetAttribute(b->sliced_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    if (b->team > 1) {                    // its clusters have to fit too
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = b->team;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.gridDim = dim3(b->blocks);
-        cfg.blockDim = dim3(sps::kBlock);
-        cfg.dynamicSmemBytes = smem;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int ncl = 0;
-        if (cudaOccupancyMaxActiveClusters(&ncl, b->sliced_kernel, &cfg) != cudaSuccess || ncl < 1) {
+    // Resident blocks of a form of the solve: whole clusters where the launch has teams.
+    const auto resident = [&](void (*kernel)(sps::batch::Args, int), int* out) -> cudaError_t {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+        int cnt = 0;
+        if (b->team > 1) {
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = b->team;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            cfg.gridDim = dim3(b->blocks);
+            cfg.blockDim = dim3(sps::kBlock);
+            cfg.dynamicSmemBytes = smem;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            e = cudaOccupancyMaxActiveClusters(&cnt, kernel, &cfg);
+            *out = cnt * b->team;
+        } else {
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cnt, kernel, sps::kBlock, smem);
+            *out = cnt * sms;
+        }
+        return e;
+    };
+    // One block on an SM where all are resident so, else two: an SM's neighbours in a cluster
+    // of 8 leave some SMs out (16 teams of 8 on LPs of 1500 rows: 22.6 ms with one block on
+    // an SM, where two teams wait, 14.9 with two).
+    const bool spread = b->blocks <= sms;
+    int held = 0;
+    b->sliced_kernel = sps::batch::k_batch_solve<true, 1>;
+    if (!spread || resident(b->sliced_kernel, &held) != cudaSuccess || held < b->blocks) {
+        b->sliced_kernel = sps::batch::k_batch_solve<true, 2>;
+        if (resident(b->sliced_kernel, &held) != cudaSuccess || held < 1) {
             cudaGetLastError();
             return SPS_OK;
         }
     }
+    // a persistent launch: blocks past the resident ones would start as others end, find the
+    // queue empty and count as idle for the hand-off
+    b->sliced_blocks = std::min(b->blocks, held);
     sps::batch::Slice* d_slice = nullptr;
     int32_t* d_off = nullptr;
     uint4* d_steps = nullptr;
@@ -1233,7 +1254,6 @@ int build_slices(sps_batch* b) {
     SPB_CK(cudaGetLastError());
     SPB_CK(cudaMemcpyAsync(off.data(), d_off, sizeof(int32_t) * chunks, cudaMemcpyDeviceToHost, b->st));
     SPB_CK(cudaStreamSynchronize(b->st));
-    const bool spread = b->blocks <= sms;
     int64_t steps = 0, left = 0, entries = 0;
     for (int32_t k = 0; k < count; ++k) {
         const Inst& I = b->inst[k];
@@ -1511,7 +1531,11 @@ extern "C" int sps_batch_create(int32_t count, const sps_problem_desc* probs, co
         // only halve the instances in flight.  A batch of fewer than half as many
         // instances as resident blocks (strong branching's children) leaves SMs
         // idle instead: there every instance of 65536 nonzeros or more gets a
-        // team, 2, 4 or 8 blocks, the largest that still fits the resident wave.
+        // team, 2, 4 or 8 blocks, the largest that fits the resident wave of the
+        // four-block form (with slices, two blocks an SM, the last of up to twice the
+        // clusters that are resident wait for one to end; smaller teams would give the
+        // sums another order: 40 LPs of 1500 rows 27.3 ms with teams of 8, 22.0 with
+        // 4; 76 LPs 42.3 and with 2 34.9).
         // Default team in a batch that fills the GPU: 4 blocks (4096 planted LPs of
         // 50-5000 rows: 2.90 s per batch against 3.19 s with 2 and 3.26 s with 8).
         int want = opt.batch_team > 0 ? std::min(opt.batch_team, 8) : 4;
@@ -1643,18 +1667,19 @@ extern "C" int sps_batch_solve(sps_batch* b, sps_batch_stats* stats) {
     SPB_CK(cudaSetDevice(b->opt.device));
     const int64_t W = b->opt.check_interval > 0 ? b->opt.check_interval : 64;
     const uint64_t tl = b->opt.time_limit_s > 0 ? (uint64_t)(b->opt.time_limit_s * 1e9) : 0;
+    const bool sliced = b->arr.slice != nullptr;
+    const int blocks = sliced ? b->sliced_blocks : b->blocks;
     sps::batch::Args A{b->d_inst, b->d_order, b->count, (int32_t)W, b->opt.max_iters, b->opt.tol, b->d_deadline,
                        b->arr, b->d_out, b->d_counter, b->opt.escalate != 0 ? 1 : 0, b->warm,
                        b->opt.warm_fallback ? 1 : 0, b->d_wx, b->d_wy, b->d_wom, b->d_cold_rel,
                        b->team, b->team_nnz, b->d_team_error, b->stage_cap, b->d_idle,
-                       (uint32_t)(b->blocks - b->blocks / 8), b->handoff_nnz};
+                       (uint32_t)(blocks - blocks / 8), b->handoff_nnz};
     auto enqueue = [&](cudaStream_t s) {
         cudaMemsetAsync(b->d_counter, 0, sizeof(uint32_t), s);
         sps::batch::k_set_deadline<<<1, 32, 0, s>>>(b->d_deadline, tl);
         cudaMemsetAsync(b->d_team_error, 0, sizeof(int32_t), s);
         cudaMemsetAsync(b->d_idle, 0, sizeof(uint32_t), s);
         const int sched = sps::batch::pack_schedule(b->G, b->Gr);
-        const bool sliced = b->arr.slice != nullptr;
         const auto kernel = sliced ? b->sliced_kernel : sps::batch::k_batch_solve<false, 4>;
         const size_t smem = b->dyn_smem + (sliced ? sps::batch::kRingBytes : 0);
         if (b->team > 1) {
@@ -1664,7 +1689,7 @@ extern "C" int sps_batch_solve(sps_batch* b, sps_batch_stats* stats) {
             attr[0].val.clusterDim.x = b->team;
             attr[0].val.clusterDim.y = 1;
             attr[0].val.clusterDim.z = 1;
-            cfg.gridDim = dim3(b->blocks);
+            cfg.gridDim = dim3(blocks);
             cfg.blockDim = dim3(sps::kBlock);
             cfg.dynamicSmemBytes = smem;
             cfg.stream = s;
@@ -1672,7 +1697,7 @@ extern "C" int sps_batch_solve(sps_batch* b, sps_batch_stats* stats) {
             cfg.numAttrs = 1;
             cudaLaunchKernelEx(&cfg, kernel, A, sched);
         } else {
-            kernel<<<b->blocks, sps::kBlock, smem, s>>>(A, sched);
+            kernel<<<blocks, sps::kBlock, smem, s>>>(A, sched);
         }
     };
     SPB_CK(cudaEventRecord(b->e0, b->st));
@@ -1770,7 +1795,7 @@ extern "C" int sps_batch_solve(sps_batch* b, sps_batch_stats* stats) {
         stats->lanes_per_column = b->G;
         stats->lanes_per_row = b->Gr;
         stats->team = b->team;
-        stats->blocks = b->blocks;
+        stats->blocks = blocks;
         stats->escalated = n_esc;
         stats->handed_off = n_hand;
         for (const Ctl& c : b->out) {

@@ -55,3 +55,41 @@ def test_warm_starts():
         b.set_warm_starts([(r.x, r.y, None) for r in cold])
         warm = _both(b)
         assert sum(r.iterations for r in warm) < sum(r.iterations for r in cold) / 2
+
+
+def test_grid_is_what_is_resident():
+    """A launch has no blocks that wait for others to end (they would count as idle for the
+    hand-off): two on an SM with slices, four on the CSR; whole clusters with teams."""
+    probs = [wl.batch_planted_lp(k, m_range=(40, 60))[0] for k in range(640)]
+    with sps.PDHGBatch(probs, tol=TOL, max_iters=200, escalate="off") as b:
+        b.solve_raw()
+        sliced = b.stats.blocks
+        assert b.lib.sps_batch_release_slices(b.h) == 1
+        b.solve_raw()
+        assert (sliced, b.stats.blocks) == (2 * 152, 4 * 152)
+    with sps.PDHGBatch(probs[:60], tol=TOL, max_iters=200, escalate="off", batch_team=8, batch_team_nnz=100) as b:
+        b.solve_raw()
+        assert b.stats.team == 8 and b.stats.blocks % 8 == 0 and b.stats.blocks <= 2 * 152
+        assert b.lib.sps_batch_release_slices(b.h) == 1
+        b.solve_raw()
+        assert b.stats.blocks == 480
+
+
+def test_teams_are_resident_at_once():
+    """19 clusters of 8 blocks do not all fit one block per SM: they take the form of two."""
+    probs = [wl.batch_planted_lp(k, m_range=(60, 300))[0] for k in range(19)]
+    with sps.PDHGBatch(probs, tol=TOL, max_iters=20000, batch_team=8, batch_team_nnz=500, escalate="off") as b:
+        _both(b)
+        assert (b.stats.team, b.stats.blocks) == (8, 152)
+
+
+def test_teams_do_not_wait_for_one_another():
+    """16 teams of 8 blocks take 1.3 times as long as 12 (1.9 times where two teams waited)."""
+    probs = [wl.batch_planted_lp(k, m_range=(1500, 1500), n_ratio=(2.0, 2.0))[0] for k in range(16)]
+
+    def best(count):
+        with sps.PDHGBatch(probs[:count], tol=1e-12, max_iters=640, escalate="off") as b:
+            ms = [b.solve_raw().solve_ms for _ in range(6)]
+            assert b.stats.team == 8
+            return min(ms[1:])
+    assert best(16) < 1.6 * best(12)

@@ -172,12 +172,12 @@ struct Grid {
     bool finite;
 };
 
-// All threads of the block; row_blocks: the blocks of the first pass.
-__device__ __forceinline__ Grid grid_of(const sps_device_lp& lp, const double* s, int row_blocks) {
+// All threads of the block; max_blocks: the blocks of the first pass.
+__device__ __forceinline__ Grid grid_of(const sps_device_lp& lp, const double* s, int max_blocks) {
     const int m = lp.m_ub + lp.m_eq;
     const long long nnz = m > 0 ? (long long)max(lp.indptr[m], 0) : 0ll;
     unsigned long long bits = 0ull;
-    for (int b = threadIdx.x; b < row_blocks; b += kThreads)
+    for (int b = threadIdx.x; b < max_blocks; b += kThreads)
         bits = max(bits, __ldcg(reinterpret_cast<const unsigned long long*>(s + kMaxBase) + b));
     bits = block_max(bits);
     Grid g;
@@ -190,25 +190,25 @@ __device__ __forceinline__ Grid grid_of(const sps_device_lp& lp, const double* s
     return g;
 }
 
-// Rows of a warp: four at a time, eight lanes each (most rows hold a few dozen
-// nonzeros: a warp per row left its lanes idle and its next row's offsets one
-// round trip away), rows of over kLongRow nonzeros by the whole warp after
-// them.  visit(i, k, lanes) runs the lane's share of row i: nonzeros k, k +
-// lanes, ...; done(i, lanes) ends it, in all of the row's lanes.
+// Rows of a warp: 32 / Lanes at a time (8, 16 or 32 lanes each: see row_lanes; most
+// rows hold a few dozen nonzeros: a warp per row left its lanes idle and its next row's
+// offsets one round trip away), rows of over kLongRow nonzeros by the whole warp after
+// them.  visit(i, k, end, lanes) runs the lane's share of row i: nonzeros k, k + lanes,
+// ...; done(i, row, lanes) ends it, in all of the row's lanes.
 constexpr int kRowLanes = 8;
 constexpr int kLongRow = 256;
-template <class Visit, class Done>
+template <int Lanes, class Visit, class Done>
 __device__ __forceinline__ void rows_of_warp(const int32_t* __restrict__ ptr, int m, const Visit& visit, const Done& done) {
-    constexpr int per = 32 / kRowLanes;
+    constexpr int per = 32 / Lanes;
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * kThreads) >> 5;
     for (int i0 = ((blockIdx.x * kThreads + threadIdx.x) >> 5) * per; i0 < m; i0 += warps * per) {
-        const int i = i0 + lane / kRowLanes;
+        const int i = i0 + lane / Lanes;
         const int b = i < m ? ptr[i] : 0, e = i < m ? ptr[i + 1] : 0;
-        const bool lng = e - b > kLongRow;
-        if (!lng) visit(i, b + (lane & (kRowLanes - 1)), e, kRowLanes);
-        unsigned todo = __ballot_sync(0xffffffffu, lng && (lane & (kRowLanes - 1)) == 0);
-        done(i, i < m && !lng, kRowLanes);
+        const bool lng = Lanes < 32 && e - b > kLongRow;
+        if (!lng) visit(i, b + (lane & (Lanes - 1)), e, Lanes);
+        unsigned todo = __ballot_sync(0xffffffffu, lng && (lane & (Lanes - 1)) == 0);
+        done(i, i < m && !lng, Lanes);
         while (todo) {                              // warp-uniform
             const int src = __ffs(todo) - 1;
             todo &= todo - 1;
@@ -223,6 +223,7 @@ __device__ __forceinline__ void rows_of_warp(const int32_t* __restrict__ ptr, in
 // Pass 1: largest |a_ij y_i| (as bits: non-negative doubles order like their bit
 // patterns, so an integer max is order-independent), one per block; clears the
 // columns' accumulators for pass 2 and the ticket of pass 3.
+template <int Lanes>
 __global__ void __launch_bounds__(kThreads) na_max(sps_device_lp lp, const double* __restrict__ y,
                                                      double* __restrict__ s) {
     const int m = lp.m_ub + lp.m_eq;
@@ -231,7 +232,7 @@ __global__ void __launch_bounds__(kThreads) na_max(sps_device_lp lp, const doubl
         for (int d = 0; d < kDigits; ++d) s[(size_t)d * kMaxCols + j] = 0.0;
     unsigned long long mx = 0ull;
     const double* __restrict__ val = lp.values;
-    rows_of_warp(lp.indptr, m,
+    rows_of_warp<Lanes>(lp.indptr, m,
         [&](int i, int k, int e, int lanes) {
             if (k >= e) return;
             const double yi = y[i];
@@ -258,19 +259,20 @@ __global__ void __launch_bounds__(kThreads) na_max(sps_device_lp lp, const doubl
 // nonzeros; with two left, 49 us (the 64-bit atomics, up to three per nonzero,
 // are what is left).  The whole call: 60k x 150k, 1.5M nonzeros 578 -> 105 us,
 // 5k x 12k 183 -> 35 us, 300 x 700 48 -> 31 us.
+template <int Lanes>
 __global__ void __launch_bounds__(kThreads) na_rows(sps_device_lp lp, const double* __restrict__ x,
-                                                     const double* __restrict__ y, double* __restrict__ s) {
+                                                     const double* __restrict__ y, double* __restrict__ s, int max_blocks) {
     double v[kParts] = {0.0, 0.0, 0.0, 0.0};
     const int m = lp.m_ub + lp.m_eq;
     const int lane = threadIdx.x & 31;
-    const Grid g = grid_of(lp, s, gridDim.x);
+    const Grid g = grid_of(lp, s, max_blocks);
     unsigned long long* acc = reinterpret_cast<unsigned long long*>(s);
     const int unit = g.e0 - kDigits * g.b;                 // the finest grid's exponent
     const unsigned long long mask = (1ull << g.b) - 1ull;
     const double* __restrict__ val = lp.values;
     const int32_t* __restrict__ idx = lp.indices;
     double sum = 0.0;
-    rows_of_warp(lp.indptr, m,
+    rows_of_warp<Lanes>(lp.indptr, m,
         [&](int i, int k, int e, int lanes) {
             if (k >= e) return;
             const double yi = y[i];
@@ -302,8 +304,7 @@ __global__ void __launch_bounds__(kThreads) na_rows(sps_device_lp lp, const doub
         [&](int i, bool row, int lanes) {
             double t = sum;
             sum = 0.0;
-            if (lanes == 32)
-                for (int o = 16; o >= kRowLanes; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            for (int o = lanes / 2; o >= kRowLanes; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
 #pragma unroll
             for (int o = kRowLanes / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
             if (!row || (lane & (lanes - 1)) != 0) return;
@@ -330,10 +331,10 @@ __device__ __forceinline__ double scaled(double v, int e) {
 // Pass 3, one thread per column, and the final reduction in the last block.
 // out: rel_kkt, rel_primal, rel_dual, rel_gap, primal objective, dual objective.
 __global__ void __launch_bounds__(kThreads) na_cols(sps_device_lp lp, const double* __restrict__ x,
-                                                     double* __restrict__ s, int row_blocks,
+                                                     double* __restrict__ s, int row_blocks, int max_blocks,
                                                      double* __restrict__ out) {
     double v[kParts] = {0.0, 0.0, 0.0, 0.0};
-    const Grid g = grid_of(lp, s, row_blocks);
+    const Grid g = grid_of(lp, s, max_blocks);
     const long long* acc = reinterpret_cast<const long long*>(s);
     for (int j = blockIdx.x * kThreads + threadIdx.x; j < lp.n; j += gridDim.x * kThreads) {
         const double cj = lp.c[j], lo = lp.lb[j], hi = lp.ub[j];
@@ -383,6 +384,19 @@ __global__ void __launch_bounds__(kThreads) na_cols(sps_device_lp lp, const doub
     out[5] = dob;
 }
 
+int blocks_for(int64_t threads) {
+    return (int)std::min<int64_t>(kMaxBlocks, std::max<int64_t>(1, (threads + kThreads - 1) / kThreads));
+}
+
+// Lanes of a row: 32 while the rows then fill one block per SM, down to 8 (the rows'
+// lengths are not known here).  Ten rows of 20 000 nonzeros took 2.00 ms with 8 lanes, four
+// rows to a warp, 0.59 with 32; 5000 rows of 20 take 36 us with 8 and 45 with 32.
+int row_lanes(int64_t m) {
+    int lanes = 32;
+    while (lanes > kRowLanes && m * lanes > 152 * kThreads) lanes /= 2;
+    return lanes;
+}
+
 }  // namespace
 
 extern "C" int sps_kkt_noalloc(const sps_device_lp* lp, const double* x, const double* y, double* out,
@@ -410,12 +424,14 @@ extern "C" int sps_kkt_noalloc(const sps_device_lp* lp, const double* x, const d
     double* s = nullptr;
     if (int rc = scratch_address(&s)) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // a warp takes 32 / kRowLanes rows at a time
-    const int row_blocks = (int)std::min<int64_t>(kMaxBlocks, std::max<int64_t>(1, ((int64_t)m * kRowLanes + kThreads - 1) / kThreads));
-    const int col_blocks = (int)std::min<int64_t>(kMaxBlocks, std::max<int64_t>(1, ((int64_t)lp->n + kThreads - 1) / kThreads));
-    na_max<<<row_blocks, kThreads, 0, st>>>(*lp, y, s);
-    na_rows<<<row_blocks, kThreads, 0, st>>>(*lp, x, y, s);
-    na_cols<<<col_blocks, kThreads, 0, st>>>(*lp, x, s, row_blocks, out);
+    const int lanes = row_lanes(m);
+    const int row_blocks = blocks_for((int64_t)m * lanes), col_blocks = blocks_for(lp->n);
+    const int max_blocks = std::max(row_blocks, col_blocks);      // the first pass clears 3 n accumulators too
+    const auto largest = lanes == 32 ? na_max<32> : lanes == 16 ? na_max<16> : na_max<8>;
+    const auto rows = lanes == 32 ? na_rows<32> : lanes == 16 ? na_rows<16> : na_rows<8>;
+    largest<<<max_blocks, kThreads, 0, st>>>(*lp, y, s);
+    rows<<<row_blocks, kThreads, 0, st>>>(*lp, x, y, s, max_blocks);
+    na_cols<<<col_blocks, kThreads, 0, st>>>(*lp, x, s, row_blocks, max_blocks, out);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         sps::set_create_error(std::string("sps_kkt_noalloc: ") + cudaGetErrorString(e));

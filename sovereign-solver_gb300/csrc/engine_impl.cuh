@@ -1083,18 +1083,20 @@ struct Engine : EngineBase {
     }
 
     // Whether the window's attempts run as one resident launch (resident.cuh), and its
-    // shape.  The line is capacity: wherever every warp's task, the matrix and the
-    // vectors fit one cluster the resident launch won (us per attempt, checks
-    // included, launched -> resident: 40 x 100 15.4 -> 3.7 FP32, 21.9 -> 6.8 FP64;
-    // 200 x 500 18.0 -> 4.3, 25.2 -> 9.1; 2000 x 5000 20.0 -> 7.2, 29.8 -> 13.3;
-    // 100 x 200 transportation 15.2 -> 11.4 FP32; reference mode 200 x 500 FP64 18.8
-    // -> 7.0).  The smallest cluster that fits is taken in FP32: more blocks only
-    // add to the barriers (200 x 500, an earlier form: 6.3 us on one block, 7.5-8.5
-    // on 2-16).  In FP64
-    // a block's products pass a pipe of two per cycle, so up to eight blocks share
-    // them while one holds over kResEntries64 entries (37 x 53 transportation: 12.5
-    // us on 4 blocks, 11.0 on 8; 40 x 100, 1.3k entries: 7.9 on 1, 8.8 on 2).  A
-    // caller who gives the passes' blocks (max_blocks) gets the launched passes.
+    // shape.  The line is capacity, each mode's own: a task per warp of at most 16 blocks
+    // (32 warps a block in FP32, 16 in FP64, less the deciding one in adaptive mode), and the
+    // block's entries and vectors in its shared memory.  Wherever that fits the resident
+    // launch won (us per attempt, checks included, launched -> resident: 40 x 100 15.4 ->
+    // 3.7 FP32, 21.9 -> 6.8 FP64; 200 x 500 18.0 -> 4.3, 25.2 -> 9.1; 2000 x 5000 20.0 -> 7.2,
+    // 29.8 -> 13.3; 100 x 200 transportation 15.2 -> 11.4 FP32; reference mode 200 x 500 FP64
+    // 18.8 -> 7.0, 80 x 160 transportation FP64 15.5 -> 9.2, 3000 x 7500 FP32 16.5 -> 6.7; the
+    // 100 x 200 transportation LP in reference FP64 has 320 column tasks for 256 warps).  The
+    // smallest cluster that fits is taken in FP32: more blocks only add to the barriers (200 x
+    // 500, an earlier form: 6.3 us on one block, 7.5-8.5 on 2-16).  In FP64 a block's products
+    // pass a pipe of two per cycle, so up to eight blocks share them while one holds over
+    // kResEntries64 entries (37 x 53 transportation: 12.5 us on 4 blocks, 11.0 on 8; 40 x 100,
+    // 1.3k entries: 7.9 on 1, 8.8 on 2).  A caller who gives the passes' blocks (max_blocks)
+    // gets the launched passes.
     int choose_resident(const Plan& rp, const Plan& cp) {
         args.res = ResShape{};
         if (opt.max_blocks > 0) return SPS_OK;
@@ -1121,7 +1123,7 @@ struct Engine : EngineBase {
             S.row_warps = rp.bt.total_blocks * kWarps;
             S.row_parts = (S.row_warps + rp.nslots + 3) & ~3;
             S.col_parts = cp.bt.total_blocks * kWarps;
-            const size_t bytes = res_smem_bytes<V>(S, n, m);
+            const size_t bytes = res_smem_bytes<V>(S, n, m, mode == SPS_MODE_ADAPTIVE);
             if (bytes > kResSmem) continue;
             if (sizeof(V) == 8 && C < kResMaxCluster / 2 && S.entries > kResEntries64) continue;
             res_bytes = bytes;

@@ -51,10 +51,12 @@ struct ResTask {
     } u[2];
 };
 
+// The block's shared memory: its entries, y' and the lane partials of SLAB units, and in
+// adaptive mode x, the candidate and all partial sums, in reference mode x'.
 template <class V>
-__host__ __device__ constexpr size_t res_smem_bytes(const ResShape& s, int64_t n, int64_t m) {
-    return (sizeof(V) + 4) * (size_t)s.entries +
-           sizeof(V) * (2 * (size_t)n + m + 2 * (size_t)s.row_parts + 2 * (size_t)s.col_parts + 32 * (size_t)s.slab_rows);
+__host__ __device__ constexpr size_t res_smem_bytes(const ResShape& s, int64_t n, int64_t m, bool adaptive) {
+    return (sizeof(V) + 4) * (size_t)s.entries + sizeof(V) * ((size_t)n + m + 32 * (size_t)s.slab_rows) +
+           (adaptive ? sizeof(V) * ((size_t)n + 2 * (size_t)s.row_parts + 2 * (size_t)s.col_parts) : 0);
 }
 
 __device__ __forceinline__ uint32_t res_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }

@@ -213,6 +213,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     return false;
 }
 
+// Of a kernel that gives up, for the MMAs in flight before it frees their memory: out of line,
+// so that the loops keep their registers.
+__device__ __noinline__ void last_wait(uint32_t bar, uint32_t parity) { mbar_wait(bar, parity); }
+
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
@@ -551,8 +555,10 @@ __global__ void __launch_bounds__(kN64T, 2) k_node64(const Node64 a) {
         tc::fence_before();
         ok = __syncthreads_and(ok) != 0;                       // shared and tensor memory free for the next tile
         tc::fence_after();
-        if (!ok && threadIdx.x == 0)                           // giving up: a last wait for what is in flight
-            tc::mbar_wait(tc::smem_u32(&bar), second ? parity ^ 1u : parity);
+        if (!ok) {
+            if (threadIdx.x == 0) tc::last_wait(tc::smem_u32(&bar), second ? parity ^ 1u : parity);
+            break;
+        }
     }
     if (!ok && threadIdx.x == 0) atomicExch(a.err, 1);
     __syncthreads();
@@ -790,9 +796,9 @@ __global__ void __launch_bounds__(bk::kThreads, 2) k_back64(const Back64 a) {
                         bk::desc_mn(hs + p * bf::kPart + 2048 * kk, bf::kPart), (p == 2 && kk == 0) ? 0u : 1u);
             tc::mma_commit(tc::smem_u32(&bars[2]));
         }
-        if (!ok) {                                              // giving up: a last wait for what is in flight
+        if (!ok) {
             if (threadIdx.x == 0)
-                for (int q = 0; q < 2; ++q) tc::mbar_wait(tc::smem_u32(&bars[q]), parity);
+                for (int q = 0; q < 2; ++q) tc::last_wait(tc::smem_u32(&bars[q]), parity);
             break;
         }
         if (!tc::mbar_wait(tc::smem_u32(&bars[1]), parity)) ok = false;
@@ -821,7 +827,7 @@ __global__ void __launch_bounds__(bk::kThreads, 2) k_back64(const Back64 a) {
         ok = __syncthreads_and(ok) != 0;
         tc::fence_after();
         if (!ok && threadIdx.x == 0)
-            for (int q = 1; q < 3; ++q) tc::mbar_wait(tc::smem_u32(&bars[q]), parity ^ 1u);
+            for (int q = 1; q < 3; ++q) tc::last_wait(tc::smem_u32(&bars[q]), parity ^ 1u);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int row = r0 + 32 * i, v = v0 + 32 * i;

@@ -93,29 +93,25 @@ __global__ void __launch_bounds__(kT) k_agg(const int32_t* __restrict__ ptr, con
     }
 }
 
-// ---- dense node update: out = relu(U h + M a + b) ---------------------------------
+// ---- dense node update, H = 32: out = relu(U h + M a + b) --------------------------
 // A register-tiled FP32 contraction of the tile's [h | a] (kUpdNodes x 2H) with
 // W^T = [U | M]^T (2H x H).  The block stages W^T (BF16 widened to FP32) once
 // and, per tile, the nodes' h and a rows as they lie in memory (16-byte loads
 // and stores).  Thread t owns nodes ng + 32 i (i < 4, ng = t / 8) and outputs
-// 4 og + 32 j + c (og = t % 8, c < 4, j < H / 32): per four input features it
-// reads four 16-byte node vectors and 2 H / 8 16-byte weight vectors from
-// shared memory for 32 (H = 64) FMAs per feature, so the FMA pipe, not
-// shared memory, sets the pace.  Each output is bias + sum over k of W[o][k] x[k]
+// 4 og + c (og = t % 8, c < 4): per four input features it reads four 16-byte node
+// vectors and four 16-byte weight vectors from shared memory for 16 FMAs per
+// feature.  Each output is bias + sum over k of W[o][k] x[k]
 // in k order (h's features, then a's), one fmaf per k.
 constexpr int kUpdNodes = 128;                 // nodes per tile
+constexpr int kUpdStride = 2 * 32 + 4;         // padded tile row: 4 consecutive rows hit distinct banks
 
-template <int H>
-__host__ __device__ constexpr int upd_stride() { return 2 * H + 4; }   // padded tile row: 4 consecutive rows hit distinct banks
-
-template <int H>
 __global__ void __launch_bounds__(kT, 2) k_update(const float* __restrict__ h, const float* __restrict__ a,
                                                   const __nv_bfloat16* __restrict__ U,
                                                   const __nv_bfloat16* __restrict__ M,
                                                   const float* __restrict__ bias, float* __restrict__ out,
                                                   int64_t nodes) {
-    static_assert(H % 32 == 0 && kT == 256, "thread layout: 8 output groups x 32 node groups");
-    constexpr int K2 = 2 * H, S = upd_stride<H>(), J = H / 32;
+    static_assert(kT == 256, "thread layout: 8 output groups x 32 node groups");
+    constexpr int H = 32, K2 = 2 * H, S = kUpdStride;
     extern __shared__ __align__(16) float sm[];
     float* Wt = sm;                           // [k][o], k < H from U, k >= H from M
     float* X = Wt + K2 * H;                   // [node][S]: h (k < H) then a
@@ -124,12 +120,8 @@ __global__ void __launch_bounds__(kT, 2) k_update(const float* __restrict__ h, c
         Wt[k * H + o] = __bfloat162float(k < H ? U[o * H + k] : M[o * H + (k - H)]);
     }
     const int og = threadIdx.x & 7, ng = threadIdx.x >> 3;
-    float4 bo[J];
-#pragma unroll
-    for (int j = 0; j < J; ++j) {
-        const float* b = bias + 4 * og + 32 * j;    // the parameter block's offsets need not be 16-byte aligned
-        bo[j] = make_float4(b[0], b[1], b[2], b[3]);
-    }
+    const float* bp = bias + 4 * og;               // the parameter block's offsets need not be 16-byte aligned
+    const float4 bo = make_float4(bp[0], bp[1], bp[2], bp[3]);
     const int64_t tiles = (nodes + kUpdNodes - 1) / kUpdNodes;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int64_t base = tile * kUpdNodes;
@@ -144,11 +136,9 @@ __global__ void __launch_bounds__(kT, 2) k_update(const float* __restrict__ h, c
             *reinterpret_cast<float4*>(X + nd * S + 4 * q) = val;
         }
         __syncthreads();
-        float4 acc[4][J];
+        float4 acc[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < J; ++j) acc[i][j] = bo[j];
+        for (int i = 0; i < 4; ++i) acc[i] = bo;
 #pragma unroll 2
         for (int k = 0; k < K2; k += 4) {
             float4 xv[4];
@@ -156,33 +146,23 @@ __global__ void __launch_bounds__(kT, 2) k_update(const float* __restrict__ h, c
             for (int i = 0; i < 4; ++i) xv[i] = *reinterpret_cast<const float4*>(X + (ng + 32 * i) * S + k);
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
-                float4 w[J];
-#pragma unroll
-                for (int j = 0; j < J; ++j)
-                    w[j] = *reinterpret_cast<const float4*>(Wt + (k + kk) * H + 4 * og + 32 * j);
+                const float4 w = *reinterpret_cast<const float4*>(Wt + (k + kk) * H + 4 * og);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const float x = kk == 0 ? xv[i].x : kk == 1 ? xv[i].y : kk == 2 ? xv[i].z : xv[i].w;
-#pragma unroll
-                    for (int j = 0; j < J; ++j) {
-                        acc[i][j].x = fmaf(w[j].x, x, acc[i][j].x);
-                        acc[i][j].y = fmaf(w[j].y, x, acc[i][j].y);
-                        acc[i][j].z = fmaf(w[j].z, x, acc[i][j].z);
-                        acc[i][j].w = fmaf(w[j].w, x, acc[i][j].w);
-                    }
+                    acc[i].x = fmaf(w.x, x, acc[i].x);
+                    acc[i].y = fmaf(w.y, x, acc[i].y);
+                    acc[i].z = fmaf(w.z, x, acc[i].z);
+                    acc[i].w = fmaf(w.w, x, acc[i].w);
                 }
             }
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int64_t v = base + ng + 32 * i;
-            if (v >= nodes) continue;
-#pragma unroll
-            for (int j = 0; j < J; ++j) {
-                const float4 r = make_float4(relu(acc[i][j].x), relu(acc[i][j].y), relu(acc[i][j].z),
-                                             relu(acc[i][j].w));
-                *reinterpret_cast<float4*>(out + v * H + 4 * og + 32 * j) = r;
-            }
+            if (v < nodes)
+                *reinterpret_cast<float4*>(out + v * H + 4 * og) =
+                    make_float4(relu(acc[i].x), relu(acc[i].y), relu(acc[i].z), relu(acc[i].w));
         }
     }
 }
@@ -1276,21 +1256,18 @@ __global__ void __launch_bounds__(kT) k_head_back(const float* __restrict__ h, c
     }
 }
 
-// ---- dense node update backward ------------------------------------------------------
+// ---- dense node update backward, H = 32 ----------------------------------------------
 // z = U h + M a + b, out = relu(z), dz = dout * (out > 0):
 //   dh (=/+=) U^T dz, da = M^T dz, partials of dU = sum dz h^T, dM = sum dz a^T, db = sum dz.
 // Thread t: node t / 8 and input features (t % 8) + 8 i for dh / da; weight-gradient
-// entries o = t / 4, k = (t % 4) + 4 i (16 of dU and 16 of dM per thread for H = 64).
-template <int H>
+// entries o = t / 4, k = (t % 4) + 4 i (8 of dU and 8 of dM in half of the threads).
 __global__ void __launch_bounds__(kT) k_update_back(const float* __restrict__ dout, const float* __restrict__ out,
                                                     const float* __restrict__ h, const float* __restrict__ a,
                                                     const __nv_bfloat16* __restrict__ U,
                                                     const __nv_bfloat16* __restrict__ M, float* __restrict__ dh,
                                                     int dh_accumulate, float* __restrict__ da,
                                                     float* __restrict__ part, int64_t nodes) {
-    constexpr int OP = H / 8;
-    constexpr int ZS = H + 1;
-    constexpr int WO = kT / 4 >= H ? 1 : H / (kT / 4);         // weight rows per thread
+    constexpr int H = 32, OP = H / 8, ZS = H + 1;
     constexpr int WK = H / 4;                                  // weight columns per thread
     extern __shared__ __align__(16) float sm[];
     float* Us = sm;                 // [o][k]
@@ -1303,14 +1280,10 @@ __global__ void __launch_bounds__(kT) k_update_back(const float* __restrict__ do
         Ms[t] = __bfloat162float(M[t]);
     }
     const int node = threadIdx.x >> 3, g = threadIdx.x & 7;
-    const int wo0 = threadIdx.x >> 2, wk0 = threadIdx.x & 3;   // weight-gradient ownership
-    float gU[WO][WK], gM[WO][WK], gb[WO];
+    const int o0 = threadIdx.x >> 2, wk0 = threadIdx.x & 3;    // weight-gradient ownership
+    float gU[WK], gM[WK], gb = 0.f;
 #pragma unroll
-    for (int r = 0; r < WO; ++r) {
-        gb[r] = 0.f;
-#pragma unroll
-        for (int i = 0; i < WK; ++i) { gU[r][i] = 0.f; gM[r][i] = 0.f; }
-    }
+    for (int i = 0; i < WK; ++i) gU[i] = gM[i] = 0.f;
     const int64_t tiles = (nodes + kTile - 1) / kTile;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int64_t base = tile * kTile;
@@ -1347,36 +1320,27 @@ __global__ void __launch_bounds__(kT) k_update_back(const float* __restrict__ do
             }
         }
         // weight gradients over the tile
-        for (int nd = 0; nd < kTile; ++nd) {
+        for (int nd = 0; nd < kTile && o0 < H; ++nd) {
+            const float zo = Z[nd * ZS + o0];
+            if (wk0 == 0) gb += zo;
 #pragma unroll
-            for (int r = 0; r < WO; ++r) {
-                const int o = wo0 + r * (kT / 4);
-                if (o >= H) continue;
-                const float zo = Z[nd * ZS + o];
-                if (wk0 == 0) gb[r] += zo;
-#pragma unroll
-                for (int i = 0; i < WK; ++i) {
-                    const int k = wk0 + 4 * i;
-                    gU[r][i] += zo * Hs[nd * ZS + k];
-                    gM[r][i] += zo * As[nd * ZS + k];
-                }
+            for (int i = 0; i < WK; ++i) {
+                const int k = wk0 + 4 * i;
+                gU[i] += zo * Hs[nd * ZS + k];
+                gM[i] += zo * As[nd * ZS + k];
             }
         }
     }
     // block partial: [dU (H*H) | dM (H*H) | db (H)]
     float* P = part + (int64_t)blockIdx.x * (2 * H * H + H);
+    if (o0 >= H) return;
 #pragma unroll
-    for (int r = 0; r < WO; ++r) {
-        const int o = wo0 + r * (kT / 4);
-        if (o >= H) continue;
-#pragma unroll
-        for (int i = 0; i < WK; ++i) {
-            const int k = wk0 + 4 * i;
-            P[o * H + k] = gU[r][i];
-            P[H * H + o * H + k] = gM[r][i];
-        }
-        if (wk0 == 0) P[2 * H * H + o] = gb[r];
+    for (int i = 0; i < WK; ++i) {
+        const int k = wk0 + 4 * i;
+        P[o0 * H + k] = gU[i];
+        P[H * H + o0 * H + k] = gM[i];
     }
+    if (wk0 == 0) P[2 * H * H + o0] = gb;
 }
 
 // input layer backward: dz = dout * (h > 0); partials of dW (H x F) and db (H)
@@ -1582,33 +1546,21 @@ thread_local std::string g_gnn_create_error;
                            std::string(#call) + ": " + cudaGetErrorString(e_));              \
     } while (0)
 
-template <int H>
-size_t update_smem() { return sizeof(float) * (2 * H * H + kUpdNodes * upd_stride<H>()); }
-template <int H>
-size_t update_back_smem() { return sizeof(float) * (2 * H * H + 3 * kTile * (H + 1)); }
+constexpr int kUpdateSmem = sizeof(float) * (2 * 32 * 32 + kUpdNodes * kUpdStride);
+constexpr int kUpdateBackSmem = sizeof(float) * (2 * 32 * 32 + 3 * kTile * (32 + 1));
 
-template <int H>
-int set_smem_attrs() {
-    if constexpr (H == 64) {
-        const auto size = [](auto k, int bytes) {
-            return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
-        };
-        for (auto k : {k_node64<false, false, false>, k_node64<false, true, false>, k_node64<true, false, false>,
-                       k_node64<true, true, false>})
-            if (!size(k, node64_smem(false))) return -2;
-        for (auto k : {k_node64<false, false, true>, k_node64<false, true, true>})
-            if (!size(k, node64_smem(true))) return -2;
-        for (auto k : {k_back64<false>, k_back64<true>})
-            if (!size(k, bk::kSmem)) return -2;
-        return 0;
-    } else {
-        if (cudaFuncSetAttribute(k_update<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)update_smem<H>()) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(k_update_back<H>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)update_back_smem<H>()) != cudaSuccess)
-            return -2;
-        return 0;
-    }
+// Dynamic shared memory of the width's kernels; false if the device refuses.
+bool set_smem_attrs(int H) {
+    const auto size = [](auto k, int bytes) {
+        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+    };
+    if (H == 32) return size(k_update, kUpdateSmem) && size(k_update_back, kUpdateBackSmem);
+    for (auto k : {k_node64<false, false, false>, k_node64<false, true, false>, k_node64<true, false, false>,
+                   k_node64<true, true, false>})
+        if (!size(k, node64_smem(false))) return false;
+    for (auto k : {k_node64<false, false, true>, k_node64<false, true, true>})
+        if (!size(k, node64_smem(true))) return false;
+    return size(k_back64<false>, bk::kSmem) && size(k_back64<true>, bk::kSmem);
 }
 
 int grid_for(int64_t work, int per_block) {
@@ -1772,10 +1724,10 @@ int forward<32>(sps_gnn* g, int batch, bool) {
         const int64_t oUc = o, oMc = o + H * H, obc = o + 2 * H * H;
         const int64_t oUv = obc + H, oMv = oUv + H * H, obv = oMv + H * H;
         k_agg<H><<<grid_for(NC * 32, kT), kT, 0, st>>>(g->cptr, g->cidx, g->ac_c, g->HV[l], g->AC[l], m, n, batch, 0);
-        k_update<H><<<g->nb_dense, kT, update_smem<H>(), st>>>(g->HC[l], g->AC[l], W + oUc, W + oMc, P + obc, g->HC[l + 1], NC);
+        k_update<<<g->nb_dense, kT, kUpdateSmem, st>>>(g->HC[l], g->AC[l], W + oUc, W + oMc, P + obc, g->HC[l + 1], NC);
         k_agg<H><<<grid_for(NV * 32, kT), kT, 0, st>>>(g->vptr, g->vidx, g->av_v, g->HC[l + 1], g->AV[l], n, m, batch,
                                                        0);
-        k_update<H><<<g->nb_dense, kT, update_smem<H>(), st>>>(g->HV[l], g->AV[l], W + oUv, W + oMv, P + obv, g->HV[l + 1], NV);
+        k_update<<<g->nb_dense, kT, kUpdateSmem, st>>>(g->HV[l], g->AV[l], W + oUv, W + oMv, P + obv, g->HV[l + 1], NV);
     }
     k_head<H><<<grid_for(NV * 32, kT), kT, 0, st>>>(g->HV[L], W + g->oWx, P + g->obx, g->x0, NV);
     k_head<H><<<grid_for(NC * 32, kT), kT, 0, st>>>(g->HC[L], W + g->oWy, P + g->oby, g->y0, NC);
@@ -1972,13 +1924,13 @@ int backward(sps_gnn* g, int batch, double* loss) {
             const int64_t oUc = o, oMc = o + H * H;
             const int64_t oUv = oMc + H * H + H, oMv = oUv + H * H;
             // variable update: HV[l+1] = relu(Uv HV[l] + Mv AV[l] + bv)
-            k_update_back<H><<<nbh, kT, update_back_smem<H>(), st>>>(dhv, g->HV[l + 1], g->HV[l], g->AV[l], W + oUv,
+            k_update_back<<<nbh, kT, kUpdateBackSmem, st>>>(dhv, g->HV[l + 1], g->HV[l], g->AV[l], W + oUv,
                                                                      W + oMv, dhv_next, 0, g->dA, g->part, NV);
             k_sum_parts<<<32, 256, 0, st>>>(g->part, nbh, width, 1.f, g->G + oUv);
             // AV[l] = agg_v(HC[l+1]): dHC[l+1] += agg over constraints with a_v values
             k_agg<H><<<grid_for(NC * 32, kT), kT, 0, st>>>(g->cptr, g->cidx, g->av_c, g->dA, dhc, m, n, batch, 1);
             // constraint update: HC[l+1] = relu(Uc HC[l] + Mc AC[l] + bc)
-            k_update_back<H><<<nbh, kT, update_back_smem<H>(), st>>>(dhc, g->HC[l + 1], g->HC[l], g->AC[l], W + oUc,
+            k_update_back<<<nbh, kT, kUpdateBackSmem, st>>>(dhc, g->HC[l + 1], g->HC[l], g->AC[l], W + oUc,
                                                                      W + oMc, dhc_next, 0, g->dA, g->part, NC);
             k_sum_parts<<<32, 256, 0, st>>>(g->part, nbh, width, 1.f, g->G + oUc);
             // AC[l] = agg_c(HV[l]): dHV[l] += agg over variables with a_c values
@@ -2185,8 +2137,7 @@ int sps_gnn_create(const sps_gnn_graph* gr, const sps_gnn_options* opt_in, sps_g
             sps_gnn* g = gg;
             GNN_CK(cudaSetDevice(opt.device));
             GNN_CK(cudaStreamCreateWithFlags(&g->st, cudaStreamNonBlocking));
-            if (H == 64) { if (set_smem_attrs<64>()) return g->fail(-2, "shared-memory attribute"); }
-            else if (set_smem_attrs<32>()) return g->fail(-2, "shared-memory attribute");
+            if (!set_smem_attrs(H)) return g->fail(-2, "shared-memory attribute");
             GNN_CK(g->alloc(&g->cptr, m + 1)); GNN_CK(g->alloc(&g->cidx, nnz));
             GNN_CK(g->alloc(&g->vptr, n + 1)); GNN_CK(g->alloc(&g->vidx, nnz));
             GNN_CK(g->alloc(&g->ac_c, nnz)); GNN_CK(g->alloc(&g->av_c, nnz));

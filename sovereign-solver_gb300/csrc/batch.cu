@@ -603,12 +603,15 @@ __device__ __forceinline__ bool solve_one(const Args& A, int k, int G, Ctl& c, d
 // Sliced: the passes read the slices of the instances (sides) that have them,
 // PerSm blocks on an SM with kRing steps per warp in flight each.  Two for a
 // batch of more blocks than SMs (three sets of 640 planted LPs: 549, 389 and 338
-// ms a solve with four blocks on the CSR, 297, 172 and 152 now); one, whose
-// registers do not spill, where an SM has no second block to run (40 children of
-// a 200 x 2000 node: 20.5 ms with two, 18.9 now; 640 LPs at their start, before
-// the small ones end, 15.0 ms for 192 attempts with two and 18.3 with one).  The
-// other form, four blocks and no ring, times the schedules, since the schedule
-// fixes the order of the sums, and serves a batch without slices.  A launch has the
+// ms a solve with four blocks on the CSR, 297, 172 and 152 now; 128 registers, 432
+// bytes of spills); one, with 255 registers and 140 bytes of spills, where an SM has no second block to run (40
+// children of a 200 x 2000 node: 20.5 ms with two, 18.9 now; 640 LPs at their start,
+// before the small ones end, 15.0 ms for 192 attempts with two and 18.3 with one).  The
+// other form, four blocks and no ring (64 registers, 560 bytes of spills), serves a
+// batch without slices and times the schedules: the schedule fixes the order of the
+// sums, so results stay what that form's are, and its choice is near the sliced form's
+// best (192 attempts of 640 planted LPs, lanes 2/4 as chosen 14.4 ms, best 1/4 13.6;
+// 40 children's LPs 2.86 as chosen, best).  A launch has the
 // blocks that are resident at once, in whole clusters where it has teams.
 template <bool Sliced, int PerSm>
 __global__ void __launch_bounds__(kBlock, PerSm) k_batch_solve(Args A, int G) {

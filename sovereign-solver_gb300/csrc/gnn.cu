@@ -326,7 +326,7 @@ struct Node64 {
 
 constexpr int node64_smem(bool two) { return (two ? 2 : 1) * bf::kW + 3 * bf::kPart + 1024; }   // + alignment
 // 512 threads, two blocks an SM: 16 threads a row of 256 contiguous bytes, four
-// rows a thread.  The node's edges are a chain of three dependent loads; with
+// rows a thread (64 registers: 160 bytes of spills with First, 32 without).  The node's edges are a chain of three dependent loads; with
 // 256 threads (eight rows each, half the warps to overlap) a layer of 1.28M
 // nodes took 230 us.
 constexpr int kN64T = 512;
@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(kN64T, 2) k_node64(const Node64 a) {
 // On CUDA cores, one shared-memory word per FMA, this took 1453 us for 640k nodes
 // of K = 128; now 200-260 us (the stream, five arrays of 164 MB, takes 120 us at
 // the measured HBM rate; each tile's chain of loads, MMAs and read-backs with two
-// blocks an SM is what is left).
+// blocks an SM is what is left; 64 registers, 216-228 bytes of spills).
 //
 // FP32 as three BF16 parts.  Both products read the same shared-memory image of a
 // 128-node tile, rows of 128 bytes with the 128-byte swizzle: as the K-major A of
@@ -966,7 +966,7 @@ __device__ __forceinline__ float sum2(float hi, float lo) { return isfinite(hi) 
 // l: features 2 l, 2 l + 1; eight rows in flight), the stretches' sums added in order.
 // Warps = 8: a block per row, a warp per stretch.  A warp per row left 4 800 warps with
 // up to 400 dependent steps each on the constraint rows of the 200 x 400 family
-// (62 us for 164 MB; now 39).  Warps = 1: a warp per row takes the stretches in turn,
+// (62 us for 164 MB; now 46, compensated).  Warps = 1: a warp per row takes the stretches in turn,
 // the same bits.  Sums of hundreds of terms, compensated.  First: the source is the
 // input layer of the nodes' four features, recomputed per edge (16 bytes instead of
 // 256).

@@ -284,8 +284,8 @@ __device__ __forceinline__ void res_total(V (&tot)[NP], const V* wp, int warps, 
 // while every warp waits.  Here it is a chain of ten such operations with the
 // same values: what depends on the attempt number alone is formed during the
 // row pass, a quotient is a product with a reciprocal corrected once by its
-// remainder, and whether it is the rounded quotient is checked off the chain,
-// by the exact remainder; positive values are compared as integers.  Operands
+// remainder (Markstein's correction), and whether it is the rounded quotient is checked
+// off the chain, by the exact remainder; positive values are compared as integers.  Operands
 // outside the ranges this needs, and the quotients the check leaves open, take
 // decide_step itself.
 __device__ __forceinline__ int64_t res_bits(double v) { return __double_as_longlong(v); }
@@ -381,6 +381,9 @@ struct ResDecide {
 };
 
 // The attempts of one window (check_interval of them, fewer when the solve ends).
+// 200 x 500 on one block: 195 us for 64 attempts, 7.2 cycles per issued instruction at
+// barriers, 2.7 on shared memory.  The 1024-thread form has 64 registers and spills
+// 104-112 bytes.
 template <class V, bool Multi, int Threads>
 __global__ void __launch_bounds__(Threads, 1) ad_resident(const __grid_constant__ Args<V> a) {
     extern __shared__ __align__(16) unsigned char res_buf[];

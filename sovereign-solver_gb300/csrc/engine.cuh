@@ -96,7 +96,9 @@ struct Layout {
     int32_t nsegrows;        // epilogue slots of this orientation (SEGMENT rows, SLAB slices)
 };
 
-constexpr int kMaxEpiPartials = 14;
+// Room of an epilogue slot (doubles): the largest epilogue's partials, the PDLP form's column
+// check (decide.cuh).  Both writers below check their own against it.
+constexpr int kMaxEpiPartials = 18;
 
 // Control block, one per handle, in device memory.  Written only by single
 // threads of "last blocks" or by block 0 thread 0, read by every kernel.
@@ -614,6 +616,7 @@ __device__ __forceinline__ void finish_segment(const Bin& b, int gseg, int r, in
         e(r, b.kind, tot, pre);
     } else {
         using R = typename Epi::R;
+        static_assert(Epi::NP <= kMaxEpiPartials, "the epilogue's partials fit its slot");
         // Which warp finishes a row last varies between runs: the row's share of
         // the kernel's reductions goes to its own slot, summed in row order by
         // the kernel's last block, so every run adds the same numbers in the same order.
@@ -827,6 +830,7 @@ __device__ __forceinline__ void visit_slab_unit(const Bin& b, int u, const Layou
         // the slice's 32 rows' epilogue partials, added over the warp in a fixed
         // butterfly order (lanes past the bin add zeros): one slot per slice
         using R = typename Epi::R;
+        static_assert(Epi::NP <= kMaxEpiPartials, "the epilogue's partials fit its slot");
         Epi one = e;
         one.zero();
         if (r < b.end) one(r, b.kind, acc, pre);

@@ -34,3 +34,12 @@ def test_copied_to_shared_memory_is_aligned():
     for name in sorted(os.listdir(CSRC)):
         for line in re.findall(r"extern __shared__[^;]*;", _source(name)):
             assert "__align__(16)" in line, (name, line)
+
+
+def test_epilogue_slots_hold_every_check():
+    """A SEGMENT column's slot holds the partials of the PDLP form's check, the most there are (the
+    writers assert it at compile time too)."""
+    n = {k: int(v) for name in ("engine.cuh", "decide.cuh")
+         for k, v in re.findall(r"constexpr int (k\w+) = (\d+);", _source(name))}
+    assert n["kMaxEpiPartials"] >= max(n["kColPartials"] + n["kLagPartials"], n["kRowPartials"])
+    assert _source("engine.cuh").count("static_assert(Epi::NP <= kMaxEpiPartials") == 2

@@ -264,7 +264,10 @@ SPS_PASS_KERNEL ad_col_step(Args<V> a) {
     V* part = reinterpret_cast<V*>(a.part_col);
     if (!publish_partials<1>(v, part, &ctl->ticket[T_COL_STEP], sm, &last)) return;
     V t[1];
-    gather_all_partials<1>(t, part, gridDim.x, a.csc, sm);
+    // (a rejected attempt visits no bins: its movement is all in the block partials, and the
+    // slots of SEGMENT columns hold an earlier kernel's)
+    if (acc) gather_all_partials<1>(t, part, gridDim.x, a.csc, sm);
+    else gather_partials<1>(t, part, gridDim.x, sm);
     if (threadIdx.x != 0) return;
     ctl->ticket[T_COL_STEP] = 0;
     ctl->dx2 = double(t[0]);

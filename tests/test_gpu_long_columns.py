@@ -33,3 +33,20 @@ def test_long_columns(m, n, precision, form):
     assert kkt.box_rel_kkt(p, a.x, a.y, form=form)["err"] < 1.5 * tol
     if n <= m - m // 3:
         assert np.abs(a.x - x).max() < 0.05                    # the '=' rows alone fix x
+
+
+@pytest.mark.parametrize("form", ["pdlp", "lagrangian"])
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("m,n", [(700, 2), (600, 17), (2000, 40)])
+def test_rejected_attempts(m, n, precision, form):
+    """From an optimal point the first attempts are rejected; their movement is the candidate's own
+    (the long columns' slots hold another kernel's sums then)."""
+    p, _ = _narrow(m, n, m + n)
+    tol = 1e-4
+    with sps.PDHGEngine(p, tol=tol, precision=precision, kkt_form=form, max_iters=20000) as e:
+        a = e.solve()
+        e.warm_start(a.x, a.y)
+        b = e.solve()
+    assert a.status == "optimal" and b.status == "optimal" and b.iterations <= a.iterations
+    assert b.stats["step_size"] > 0 and b.stats["accepted_steps"] < b.iterations
+    assert kkt.box_rel_kkt(p, b.x, b.y, form=form)["err"] < 1.5 * tol

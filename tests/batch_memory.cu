@@ -1,8 +1,9 @@
 // Test helper (host code only, no GPU needed): the batch's device memory
 // (sovereign-solver_gb300/csrc/batch.cu) on a device of a given size, for
 // tests/test_batch_memory.py.  The runtime calls of the host code are replaced by
-// stand-ins over host memory; launches do nothing.  Every check prints one line; the
-// exit status is 0 when all hold.
+// stand-ins over host memory.  It runs on the CPU alone: no device may be visible, so that
+// the launches among the host code do nothing (it ends at once where one is).  Every
+// check prints one line; the exit status is 0 when all hold.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -10,6 +11,12 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+
+// (the runtime's own, before its names are replaced)
+static bool device_visible() {
+    int n = 0;
+    return cudaGetDeviceCount(&n) == cudaSuccess && n > 0;
+}
 
 static size_t g_size = 0, g_used = 0;
 static std::map<void*, size_t> g_held;
@@ -126,6 +133,11 @@ static bool check(const char* name, bool ok) {
 }
 
 int main() {
+    setenv("CUDA_VISIBLE_DEVICES", "", 1);
+    if (device_visible()) {
+        printf("a device is visible: its kernels would be given host memory\n");
+        return 1;
+    }
     bool all = true;
     const std::vector<double> x(kCount * kN, 0.5), y(kCount * kM, 0.5);
     {   // room for the slices, then none for the warm starts beside them

@@ -17,5 +17,6 @@ def test_slices_give_way(tmp_path):
            "-lpthread", "-ldl"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     assert r.returncode == 0, r.stderr[-4000:]
-    r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
+    env = dict(os.environ, CUDA_VISIBLE_DEVICES="")                # its launches must find no device
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=60, env=env)
     assert r.returncode == 0 and "FAILED" not in r.stdout, r.stdout + r.stderr

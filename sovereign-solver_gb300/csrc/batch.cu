@@ -1577,6 +1577,13 @@ extern "C" int sps_batch_create(int32_t count, const sps_problem_desc* probs, co
             }
             cudaGetLastError();
         }
+        if (b->team > 1) {
+            // a cluster breaks up for good at its first smaller instance: all large ones come
+            // before, so which are solved by a team does not depend on when a cluster got there
+            std::stable_partition(b->order.begin(), b->order.end(),
+                                  [&](int32_t k) { return b->inst[k].nnz >= b->team_nnz; });
+            SPB_CK(cudaMemcpyAsync(b->d_order, b->order.data(), 4 * (size_t)count, cudaMemcpyHostToDevice, b->st));
+        }
         SPB_CK(cudaEventRecord(b->e1, b->st));
         SPB_CK(cudaStreamSynchronize(b->st));
         float ms = 0;

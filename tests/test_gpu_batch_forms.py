@@ -93,3 +93,33 @@ def test_teams_do_not_wait_for_one_another():
             assert b.stats.team == 8
             return min(ms[1:])
     assert best(16) < 1.6 * best(12)
+
+
+def test_every_large_instance_gets_its_team():
+    """Instances of many columns but few nonzeros lie among the large ones in the order of work; a
+    cluster that met one broke up, and the large ones after it were solved by a team or by one
+    block as it happened.  Each has the bits that it has in a batch of large ones alone."""
+    import scipy.sparse as sp
+
+    def box(m, n, per_row, seed):
+        rng = np.random.default_rng(seed)
+        A = sp.csr_matrix((rng.standard_normal(m * per_row),
+                           np.concatenate([rng.choice(n, per_row, replace=False) for _ in range(m)]),
+                           np.arange(0, m * per_row + 1, per_row)), shape=(m, n))
+        return sps.Problem(c=rng.standard_normal(n), A_ub=A, b_ub=A @ np.full(n, 0.25) + rng.uniform(0.1, 1.0, m),
+                           A_eq=sp.csr_matrix((0, n)), b_eq=np.zeros(0), lb=np.zeros(n), ub=np.ones(n),
+                           integer_mask=np.zeros(n, bool))
+    first = [box(300, 600, 20, k) for k in range(40)]                      # work 6900, 6000 nonzeros
+    sparse = [box(40, 4000, 10, 100 + k) for k in range(60)]               # work 4440, 400 nonzeros
+    last = [box(60, 150, 20, 200 + k) for k in range(120)]                 # work 1410, 1200 nonzeros
+    opts = dict(tol=1e-9, max_iters=640, escalate="off", batch_group=4, batch_team=8, batch_team_nnz=1000)
+    with sps.PDHGBatch(first + last, **opts) as b:
+        alone = b.solve()
+        lanes = b.stats.lanes_per_row
+    with sps.PDHGBatch(first + sparse + last, **opts) as b:
+        mixed = b.solve()
+        assert b.stats.team == 8
+        if b.stats.lanes_per_row != lanes:
+            pytest.skip("the two batches timed another schedule")
+    for r, q in zip(alone, mixed[:40] + mixed[100:]):
+        assert np.array_equal(r.x, q.x) and np.array_equal(r.y, q.y) and r.iterations == q.iterations

@@ -73,6 +73,21 @@ def test_same_bits_in_every_batch(m, n, per_row):
             assert np.array_equal(x[0], X[s]) and np.array_equal(y[0], Y[s])
 
 
+@pytest.mark.parametrize("m,n,per_row", [(400, 400, 20), (700, 90, 6), (50, 130, 100)])
+def test_outputs_are_as_exact_as_fp32(m, n, per_row):
+    """Root mean square error of the points against FP64 at most 7e-7: a value is six rounded sums of
+    FP32 (2^-24 each, 1.5e-7 together) of terms that carry the layer's before; a sum whose terms
+    are cut to its own last place, 128 of them, is off by more than a part in 10^6."""
+    L = 3
+    with WarmStartGNN(_graph(m, n, per_row), layers=L, seed=7, max_batch=1, lp_features=False) as net:
+        params = net.params()
+        fvs, fcs, *_ = _inputs(net, 1)
+        X, Y, _ = net.predict_features(fvs, fcs)
+        x, y, _ = gnn_ref.predict(params, gnn_ref.Layout(64, L, 4, 4), net._ptr, net._idx, net._val, fvs[0], fcs[0])
+    assert np.linalg.norm(X[0] - x) <= 7e-7 * np.linalg.norm(x)
+    assert np.linalg.norm(Y[0] - y) <= 7e-7 * np.linalg.norm(y)
+
+
 def test_many_rows_and_long_columns_keep_pace():
     """40 000 rows of 20 edges on 500 columns (1600 edges each) against the transpose, the same
     edges and nodes: 2 times its time (with the few rows' form 10 times)."""
